@@ -42,7 +42,8 @@ struct QPlan {
     int pull_max;            /* most neighbour candidates scored per patch */
     int tile;                /* query patches per CTA (single-image launches) */
     int row0, rows;          /* patch rows of a single-image launch */
-    const float4 *b1;        /* b shifted by one pixel: b1[i] = b[i + 1] */
+    const float *brow;       /* row store of the table image (k_row_store) */
+    int nline;               /* its lines per image row */
     const int *allowed;      /* b patches that may be matched (allowed[p] == allowed_index), or NULL */
     int allowed_index;
     const float4 *adesc;     /* descriptor mode: query descriptor store (ds4 float4 per patch), or NULL */
@@ -70,169 +71,226 @@ __device__ __forceinline__ void count_work(unsigned long long *counters, unsigne
     if ((threadIdx.x & 31) == 0) { atomicAdd(counters, (unsigned long long) c); atomicAdd(counters + 1, (unsigned long long) r); }
 }
 
-constexpr int TWD = 32;                   /* query patches per CTA row segment when none is chosen */
-/* Threads per SM the register caps of the lean choose and the one-candidate pull leave room for.
-   Both compile to 56 registers under these caps; tighter caps (20 x 64 or 24 x 64 threads per
-   SM: 48 or 40 registers, no spills) measured 1-3 % slower at 1080p. */
-constexpr int CHOOSE_LEAN_LANES = 12 * 64;
-constexpr int PULL_ONE_LANES = 16 * 64;
-constexpr int TWD_DESC = 64;              /* query patches per CTA in descriptor mode */
+/* Threads per SM the register caps leave room for: the kernels wait on gathers from L2, so more
+   resident warps pay until the row buffers spill.  Measured at 1080p, 128 patches per CTA, ms at
+   8 / 12 / 16 / 18 x 64 threads per SM: lean choose 0.236 / 0.185 / 0.166 / 0.165, one-candidate
+   pull 0.299 / 0.231 / 0.201 / 0.199, the default schedule's four general pulls 3.23 / 2.99 / 3.04 /
+   3.36 (2.97 at 14) and chooses 1.02 / 0.94 / 0.88 / 0.96 (0.89 at 14). */
+constexpr int CHOOSE_LANES = 14 * 64, CHOOSE_LEAN_LANES = 20 * 64, PULL_LANES = 14 * 64, PULL_ONE_LANES = 18 * 64;
+constexpr int min_ctas(int lanes, int tp) { return lanes / tp < 32 ? lanes / tp : 32; }
 
-/* Stages the 8 pixel rows under a CTA's row segment of TW query patches in shared memory
-   (TW + 7 pixels per row) as packed RGB, 3 floats per pixel: a lane reading channel c of its 8
-   pixels touches word 3 * pixel + c, so each warp-wide 4-byte load hits 32 distinct banks in one
-   wavefront, and a row costs 24 wavefronts instead of the 32 of 16-byte RGBA loads. */
-template<int TW>
-__device__ __forceinline__ void stage_a(float4 *atile, const float4 *__restrict__ a, int aw, int ah, int x0, int y) {
-    constexpr int ATW = TW + 7;
-    float *at = reinterpret_cast<float *>(atile);
-    for (int i = threadIdx.x; i < 8 * ATW; i += TW) {
-        int r = i / ATW, c = i - r * ATW;
-        int gx = x0 + c, gy = y + r;
-        const float4 v = (gx < aw && gy < ah) ? __ldg(a + (size_t) gy * aw + gx) : make_float4(0.f, 0.f, 0.f, 0.f);
-        at[3 * i] = v.x;
-        at[3 * i + 1] = v.y;
-        at[3 * i + 2] = v.z;
+/* A CTA covers TP query patches: warps of 8 x 4 patches (8 columns, 4 rows; lane l is the patch
+   at column l / 4, row l % 4), side by side and stacked to the tile below.  A square-ish tile
+   keeps the candidate rows that neighbouring patches share in the SM's L1, and four lanes that
+   work on one patch find the patches of their four rounds in the same image columns. */
+constexpr int WTW = 8, WTH = 4;           /* query patches per warp: columns, rows */
+constexpr int TILE_DEFAULT = 128;         /* query patches per CTA when none is chosen */
+constexpr int TILE_DESC = 64;             /* query patches per CTA in descriptor mode (of one row) */
+__host__ __device__ constexpr int tile_w(int tp) { return tp <= 32 ? 8 : tp <= 128 ? 16 : 32; }
+__host__ __device__ constexpr int tile_h(int tp) { return tp / tile_w(tp); }
+__host__ __device__ constexpr int stage_pitch(int tp) { return 3 * (tile_w(tp) + 7); }
+__host__ __device__ constexpr int stage_rows(int tp) { return tile_h(tp) + 7; }
+
+/* Columns and rows of a CTA's tile in image mode, and in descriptor mode (a row segment). */
+__host__ __device__ constexpr int cta_w(int tp, bool desc) { return desc ? tp : tile_w(tp); }
+__host__ __device__ constexpr int cta_h(int tp, bool desc) { return desc ? 1 : tile_h(tp); }
+
+/* Shared-memory bytes of a staged query tile of TP patches. */
+constexpr size_t atile_bytes(int tp) { return sizeof(float) * stage_pitch(tp) * stage_rows(tp); }
+
+/* Stages the pixels under a CTA's tile as packed rows, 3 floats per pixel, negated: the scorer
+   adds them to the candidate's pixels (b - a and a - b square to the same bits). */
+template<int TP>
+__device__ __forceinline__ void stage_a(float *at, const float *__restrict__ a, int aw, int ah, int x0, int y0) {
+    constexpr int PITCH = stage_pitch(TP);
+    const int left = 3 * (aw - x0);
+    for (int i = threadIdx.x; i < PITCH * stage_rows(TP); i += TP) {
+        const int r = i / PITCH, c = i - r * PITCH;
+        const int gy = y0 + r;
+        at[i] = (gy < ah && c < left) ? -__ldg(a + ((size_t) gy * aw + x0) * 3 + c) : 0.f;
     }
 }
 
-/* Shared-memory bytes of a staged query tile of TW patches. */
-constexpr size_t atile_bytes(int TW) { return sizeof(float) * 3 * 8 * (TW + 7); }
-
-/* Query row dy of the patch at tile column tx. */
-template<int TW>
-__device__ __forceinline__ void load_arow(const float4 *atile, int dy, int tx, float4 (&av)[8]) {
-    const float *at = reinterpret_cast<const float *>(atile) + 3 * (dy * (TW + 7) + tx);
-#pragma unroll
-    for (int p = 0; p < 8; p++) av[p] = make_float4(at[3 * p], at[3 * p + 1], at[3 * p + 2], 0.f);
+typedef unsigned long long f32x2;         /* two floats in a register pair (add / mul .f32x2) */
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
-/* One 32-byte read-only load: pixels p[0], p[1]. */
-__device__ __forceinline__ void ld_px2(const float4 *p, float4 &u, float4 &v) {
+/* One 32-byte read-only load. */
+__device__ __forceinline__ void ld8(const float *p, float (&v)[8]) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w), "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
         : "l"(p));
 }
 
-/* The 8 pixels (x..x+7, y) of b with four 32-byte loads: pixel index i = y*bw + x is read from b
-   when even and from the shifted copy b1 (b1[i-1] = b[i]) when odd, so every load starts on a
-   32-byte boundary (both arrays are 256-byte aligned). */
-__device__ __forceinline__ void load_brow(const QPlan &q, const float4 *__restrict__ B, int x, int y, float4 (&bv)[8]) {
-    const size_t i = (size_t) y * q.bw + x;
-    const float4 *src = (i & 1) ? q.b1 + (i - 1) : B + i;
-#pragma unroll
-    for (int j = 0; j < 4; j++) ld_px2(src + 2 * j, bv[2 * j], bv[2 * j + 1]);
+/* Lane j of a quad holds the quad's partial sums of patch s in acc[s] (its SSE lane j); returns,
+   to lane s, patch s's total in the reference's order ((l0 + l1) + l2) + l3: a 4 x 4 transpose in
+   two exchange steps. */
+__device__ __forceinline__ float quad_total(const float (&acc)[4]) {
+    const unsigned FULL = 0xffffffffu;
+    const bool b0 = threadIdx.x & 1, b1 = threadIdx.x & 2;
+    const float r0 = __shfl_xor_sync(FULL, b0 ? acc[0] : acc[1], 1), r1 = __shfl_xor_sync(FULL, b0 ? acc[2] : acc[3], 1);
+    const float t0 = b0 ? acc[1] : acc[0], t1 = b0 ? acc[3] : acc[2];
+    const float k0 = b1 ? t1 : t0, k1 = b1 ? r1 : r0;
+    const float g0 = __shfl_xor_sync(FULL, b1 ? t0 : t1, 2), g1 = __shfl_xor_sync(FULL, b1 ? r0 : r1, 2);
+    const float lo0 = b1 ? g0 : k0, lo1 = b1 ? g1 : k1, h0 = b1 ? k0 : g0, h1 = b1 ? k1 : g1;
+    return __fadd_rn(__fadd_rn(__fadd_rn(lo0, lo1), b0 ? h1 : h0), b0 ? h0 : h1);
 }
 
-/* Adds one patch row to the four SSE-lane sums of patch_dist_exact (patchtable.h:349-356): the
-   interleaved RGB float e = 3p + c goes to lane e & 3, in increasing e per lane. */
-__device__ __forceinline__ void row_lanes(const float4 (&av)[8], const float4 (&bv)[8], float (&l)[4]) {
+/* patch_dist_exact (patchtable.h:330-373) of one candidate per lane, 32 of them per call: the
+   whole warp takes part, lanes without a candidate pass valid = false.
+
+   The reference keeps four SSE lane sums, the interleaved RGB float e of a patch row going to sum
+   e & 3 in increasing e; a quad of lanes scores one patch, lane j holding sum j, so every sum is
+   accumulated in exactly that order.  Each quad scores its four lanes' patches together, row by
+   row.  A candidate row is one aligned 128-byte line of the table image's row store (k_row_store):
+   lane j reads its 32 bytes with one load and picks its six floats by the column's parity.  The four
+   patches of a quad lie in the same columns on consecutive rows: a staged query row is read from
+   shared memory once for all of them (11 rows instead of 32).
+
+   Bound: the L1 data pipe (128 bytes per clock: 256 wavefronts for 32 candidates' lines, 66 for the
+   query rows, 24 for the exchanges) at 82 % of its peak in the general pull, issue slots at 61 %.
+   The gather this replaced -- each lane its own candidate's 8 pixels, four 32-byte loads from 32
+   different lines, 24 shared loads per row -- spent one wavefront on every lane's load and ran at
+   89 % of the same pipe: at 1080p the lean choose took 0.265 ms (now 0.165), the one-candidate pull
+   0.257 (0.199), the default schedule's pulls 4.01 (2.97).
+
+   With EXIT a candidate is abandoned (+inf returned) once its partial total reaches `bound`, tested
+   after rows 2, 4 and 6 (the total can only grow, so nothing that would be accepted is lost). */
+template<int TP, bool EXIT>
+__device__ __forceinline__ float score32(const QPlan &q, const float *al, int cand, bool valid, float bound, unsigned &rows) {
+    constexpr int PITCH = stage_pitch(TP);
+    const unsigned FULL = 0xffffffffu;
+    unsigned live = __ballot_sync(FULL, valid);
+    if (!live) return finf();
+    const int lane = threadIdx.x & 31, qb = lane & ~3, j = lane & 3;
+    unsigned v = 0;                       /* line << 1 | odd column; lanes without a candidate read line 0 */
+    if (valid) {
+        const unsigned x = (unsigned) pt_x(cand);
+        v = (((unsigned) pt_y(cand) * (unsigned) q.nline + (x >> 1)) << 1) | (x & 1);
+    }
+    const float *p[4];
+    bool off[4];                          /* the lane's floats start at 1 instead of 0 of its 8 */
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
-        const float t0 = __fsub_rn(av[p].x, bv[p].x), t1 = __fsub_rn(av[p].y, bv[p].y), t2 = __fsub_rn(av[p].z, bv[p].z);
-        const float qd[3] = {__fmul_rn(t0, t0), __fmul_rn(t1, t1), __fmul_rn(t2, t2)};
+    for (int s = 0; s < 4; s++) {
+        const unsigned vs = __shfl_sync(FULL, v, qb | s);
+        const int i0 = 3 * (int) (vs & 1) + j;
+        p[s] = q.brow + (size_t) (vs >> 1) * 32 + (i0 & 3) * 8;
+        off[s] = i0 >= 4;
+    }
+    const size_t pitch = (size_t) q.nline * 32;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    f32x2 aw[4][3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const int e = (3 * p + c) & 3;
-            l[e] = __fadd_rn(l[e], qd[c]);
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int n = 0; n < 3; n++) aw[r][n] = pack2(al[r * PITCH + 8 * n], al[r * PITCH + 8 * n + 4]);
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+#pragma unroll
+        for (int n = 0; n < 3; n++) aw[(r + 3) & 3][n] = pack2(al[(r + 3) * PITCH + 8 * n], al[(r + 3) * PITCH + 8 * n + 4]);
+        float u[4][8];
+#pragma unroll
+        for (int s = 0; s < 4; s++) { ld8(p[s], u[s]); p[s] += pitch; }
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            float w[6];
+#pragma unroll
+            for (int n = 0; n < 6; n++) w[n] = off[s] ? u[s][n + 1] : u[s][n];
+#pragma unroll
+            for (int n = 0; n < 3; n++) {
+                const f32x2 t = add2(pack2(w[2 * n], w[2 * n + 1]), aw[(r + s) & 3][n]);
+                float lo, hi;
+                unpack2(mul2(t, t), lo, hi);
+                acc[s] = __fadd_rn(__fadd_rn(acc[s], lo), hi);
+            }
+        }
+        if (EXIT && (r == 1 || r == 3 || r == 5)) {
+            const bool own = (live >> lane) & 1;
+            if (own) rows += 2;
+            const float part = quad_total(acc);
+            live = __ballot_sync(FULL, own && !(part >= bound));
+            if (!live) return finf();
+#pragma unroll
+            for (int s = 0; s < 4; s++)
+                if (!((live >> (qb | s)) & 1)) p[s] = q.brow;      /* dead: all read one line */
         }
     }
+    const float tot = quad_total(acc);
+    const bool own = (live >> lane) & 1;
+    if (own) rows += EXIT ? 2 : 8;
+    return own ? tot : finf();
 }
 
-__device__ __forceinline__ float lane_total(const float (&l)[4]) {
-    return __fadd_rn(__fadd_rn(__fadd_rn(l[0], l[1]), l[2]), l[3]);
-}
-
-/* patch_dist_exact with the query patch in shared memory; abandons the sum once a row's partial
-   total reaches `bound` (+inf returned). */
-template<int TW>
-__device__ __forceinline__ float ssd_tile(const float4 *atile, int tx, const QPlan &q, const float4 *__restrict__ B,
-                                          int bx, int by, float bound, unsigned &rows) {
-    float l[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-    for (int dy = 0; dy < 8; dy++) {
-        rows++;
-        float4 av[8], bv[8];
-        load_brow(q, B, bx, by + dy, bv);
-        load_arow<TW>(atile, dy, tx, av);
-        row_lanes(av, bv, l);
-        if (dy < 7 && lane_total(l) >= bound) return finf();
-    }
-    return lane_total(l);
-}
-
-/* Up to G candidates' sums advanced together row by row, so each query row is read from shared
-   memory once per group; candidate g takes part when bit g of `valid` is set.  Each sum keeps the
-   reference's lane order and stops once its partial total reaches `bound`.  out[g] = the full sum,
-   or +inf when stopped or not taking part. */
-template<int TW, int G>
-__device__ __forceinline__ void ssd_group(const float4 *atile, int tx, const QPlan &q, const float4 *__restrict__ B,
-                                          const int (&cand)[G], unsigned valid, float bound, float (&out)[G],
-                                          unsigned &rows) {
-    float l[G][4];
-    bool live[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) { l[g][0] = l[g][1] = l[g][2] = l[g][3] = 0.f; live[g] = (valid >> g) & 1; }
-#pragma unroll 1
-    for (int dy = 0; dy < 8; dy++) {
-        bool any = false;
-#pragma unroll
-        for (int g = 0; g < G; g++) any |= live[g];
-        if (!any) break;
-        float4 av[8];
-        load_arow<TW>(atile, dy, tx, av);
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            if (!live[g]) continue;
-            rows++;
-            float4 bv[8];
-            load_brow(q, B, pt_x(cand[g]), pt_y(cand[g]) + dy, bv);
-            row_lanes(av, bv, l[g]);
-            if (dy < 7 && lane_total(l[g]) >= bound) live[g] = false;
-        }
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++) out[g] = live[g] ? lane_total(l[g]) : finf();
-}
-
-/* The query patch a distance is taken from: its RGB rows staged in shared memory (image mode) or
-   its descriptor in registers (descriptor mode, DESC instantiations). */
+/* The query patch a distance is taken from: its staged rows (image mode: the address of the lane's
+   first float) or its descriptor in registers (descriptor mode). */
 struct AQuery {
-    const float4 *atile;
-    int tx;
+    const float *al;
     float4 v[4];
 };
 
-/* One candidate's distance: patch_dist_exact (image mode, abandoned at `bound`) or
+/* One candidate's distance per lane: patch_dist_exact for the whole warp at once (image mode), or
    patch_dist_approx of the descriptors (descriptor mode, always complete: a complete sum at or
    above the bound is rejected by the caller exactly as an abandoned one). */
-template<int TW, bool DESC>
-__device__ __forceinline__ float dist1(const AQuery &aq, const QPlan &q, const float4 *__restrict__ B, int bx, int by,
-                                       float bound, unsigned &rows) {
+template<int TP, bool DESC, bool EXIT>
+__device__ __forceinline__ float dist32(const AQuery &aq, const QPlan &q, int cand, bool valid, float bound, unsigned &rows) {
     if constexpr (DESC) {
+        if (!valid) return finf();
         rows++;
-        return pt_desc_dist(aq.v, q.bdesc + ((size_t) by * q.bew + bx) * q.ds4, q.nd);
+        return pt_desc_dist(aq.v, q.bdesc + ((size_t) pt_y(cand) * q.bew + pt_x(cand)) * q.ds4, q.nd);
     } else {
-        return ssd_tile<TW>(aq.atile, aq.tx, q, B, bx, by, bound, rows);
+        return score32<TP, EXIT>(q, aq.al, cand, valid, bound, rows);
     }
 }
 
-template<int TW, int G, bool DESC>
-__device__ __forceinline__ void dist_group(const AQuery &aq, const QPlan &q, const float4 *__restrict__ B,
-                                           const int (&cand)[G], unsigned valid, float bound, float (&out)[G],
-                                           unsigned &rows) {
-    if constexpr (DESC) {
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-            out[g] = finf();
-            if ((valid >> g) & 1) {
-                rows++;
-                out[g] = pt_desc_dist(aq.v, q.bdesc + ((size_t) pt_y(cand[g]) * q.bew + pt_x(cand[g])) * q.ds4, q.nd);
-            }
-        }
+/* This lane's patch of the tile with top-left patch (x0, y0), and its query. */
+template<int TP, bool DESC>
+__device__ __forceinline__ void tile_lane(const QPlan &q, const float *at, int x0, int y0, int &x, int &y, AQuery &aq) {
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (DESC) {                 /* a row segment: nothing but the row order is shared */
+        x = x0 + threadIdx.x;
+        y = y0;
     } else {
-        ssd_group<TW, G>(aq.atile, aq.tx, q, B, cand, valid, bound, out, rows);
+        constexpr int WX = tile_w(TP) / WTW;
+        const int cx = (wid % WX) * WTW + (lane >> 2), ry = (wid / WX) * WTH;
+        x = x0 + cx;
+        y = y0 + ry + (lane & 3);
+        aq.al = at + ry * stage_pitch(TP) + 3 * cx + (lane & 3);
     }
+}
+
+/* The table entry v as a patch position, -1 when it lies outside b: a table built here only holds
+   patches of b; the range test guards against a corrupt table file or entry array, which must not
+   make a kernel read outside b. */
+__device__ __forceinline__ int table_entry(const QPlan &q, int v) {
+    const int xs = pt_x(v) - 7, ys = pt_y(v) - 7;
+    return (xs >= 0 && ys >= 0 && xs < q.bew && ys < q.beh) ? pt_xy(xs, ys) : -1;
+}
+
+/* Random search (patchtable.h:3874-3903): one of the 8 neighbours of the best match, -1 when it lies
+   outside b or is not allowed.  dx, dy + 1 for r = 0..7 are packed two bits each:
+   {-1,0,1,-1,1,-1,0,1}, {-1,-1,-1,0,0,1,1,1}. */
+__device__ __forceinline__ int random_neighbour(const QPlan &q, int p, int xb, int yb) {
+    const unsigned r = mix32((unsigned) p * 2654435761u + (unsigned) q.pass * 0x9e3779b9u + 0x6a09e667u) & 7u;
+    const int xs = xb + (int) ((37412u >> (2 * r)) & 3u) - 1, ys = yb + (int) ((43328u >> (2 * r)) & 3u) - 1;
+    if (xs < 0 || xs >= q.bew || ys < 0 || ys >= q.beh) return -1;
+    if (q.allowed && __ldg(q.allowed + (size_t) ys * q.bew + xs) != q.allowed_index) return -1;
+    return pt_xy(xs, ys);
 }
 
 /* Proposals of the learned network for one patch (LEARNED instantiation of k_choose_tile). */
@@ -244,347 +302,385 @@ struct LearnedArgs {
     unsigned long long *counters;   /* [confident patches, proposals scored] or NULL */
 };
 
-/* Steps 1-3 for every patch ("choose"): returns the chosen match and its exact distance.  One CTA
-   per 256-patch row segment, with the segment's query rows staged in shared memory.  The LEARNED
-   instantiation replaces, for patches whose proposal confidence reaches the threshold, the table
-   candidate by the network's proposals (scored best-first in groups of three) and, unless
-   configured otherwise, skips k-coherence for them. */
-/* LEAN: the table step only (no further tables, k-coherence, spatial or random search), so the
-   registers those steps need are not reserved. */
-template<int TW, bool LEARNED, bool DESC, bool LEAN = false>
+/* Steps 1-3 for every patch ("choose"): the chosen match and its exact distance.  Each lane walks
+   its own patch's candidates in the reference's order -- table entries, k-coherence neighbours,
+   spatial or random search -- and the warp scores one candidate per lane at a time, so lanes may be
+   at different steps of the walk.  The LEARNED instantiation replaces, for patches whose proposal
+   confidence reaches the threshold, the table candidate by the network's proposals (best first)
+   and, unless configured otherwise, skips k-coherence for them.
+   LEAN: the table step only (no further tables, k-coherence, spatial or random search), one
+   candidate per patch, without the registers of the walk. */
+template<int TP, bool LEARNED, bool LEAN>
 __device__ __forceinline__ void
-choose_seg(const QPlan &c_q, float4 *atile, const float4 *__restrict__ a, const float4 *__restrict__ b,
-           const int *__restrict__ cur_pos, const float *__restrict__ cur_d, const int *__restrict__ tcand,
-           const int2 *__restrict__ kcoh, int do_table, int *ch_pos, float *ch_d, int *kc_done, int use_done,
-           unsigned long long *counters, const LearnedArgs &la, int x0, int y) {
-    if constexpr (!DESC) {
-        stage_a<TW>(atile, a, c_q.aw, c_q.ah, x0, y);
-        __syncthreads();
-    }
-    const int x = x0 + threadIdx.x;
-    const bool live = x < c_q.ew;
+choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
+            const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
+            int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs &la,
+            int x0, int y0, int y1) {
+    const unsigned FULL = 0xffffffffu;
+    stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
+    __syncthreads();
+    AQuery aq;
+    int x, y;
+    tile_lane<TP, false>(c_q, at, x0, y0, x, y, aq);
+    const bool live = x < c_q.ew && y < y1;
+    const int p = live ? y * c_q.ew + x : 0;
     unsigned ne = 0, rows = 0, n_conf = 0, n_prop = 0;
-    if (live) {
-        const int p = y * c_q.ew + x;
-        AQuery aq;
-        aq.atile = atile;
-        aq.tx = threadIdx.x;
-        if constexpr (DESC) pt_desc_load(c_q.adesc + (size_t) p * c_q.ds4, 4 * c_q.ds4, aq.v);
-        /* no state arrays: the initial field, x = b's ew + 1 and DIST_INFINITY (patchtable.h:3538-3547) */
-        int pos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);
-        float dstore = cur_d ? cur_d[p] : (float) PT_DIST_INF;
-        int xb = pt_x(pos), yb = pt_y(pos);
-        float dbest = (float) ((double) dstore * c_q.prop_scale);
-        float dch = dstore;
-        bool confident = false;
-        if (LEARNED) confident = la.conf[p] >= la.threshold;
-        if (LEARNED && confident && do_table && la.cand) {
-            /* the proposals in the network's order, repeats dropped, three at a time */
+    /* no state arrays: the initial field, x = b's ew + 1 and DIST_INFINITY (patchtable.h:3538-3547) */
+    const int pos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);
+    const float dstore = cur_d ? cur_d[p] : (float) PT_DIST_INF;
+    int xb = pt_x(pos), yb = pt_y(pos);
+    float dbest = (float) ((double) dstore * c_q.prop_scale);
+    float dch = dstore;
+    auto entry = [&](int v) { return table_entry(c_q, v); };
+    if constexpr (LEAN) {
+        int cand = -1;
+        if (live && do_table) {
+            cand = entry(tcand[p]);
+            if (cand == pt_xy(xb, yb)) cand = -1;
+        }
+        const float d = dist32<TP, false, false>(aq, c_q, cand, cand >= 0, dbest, rows);
+        if (cand >= 0) {
+            ne++;
+            if (d < dbest) { dch = d; xb = pt_x(cand); yb = pt_y(cand); }
+        }
+        if (live) { ch_pos[p] = pt_xy(xb, yb); ch_d[p] = dch; }
+        count_work(counters, ne, rows);
+        return;
+    }
+    bool confident = false;
+    unsigned keep = 0;                    /* the network's proposals still to score, repeats dropped */
+    if (LEARNED && live) {
+        confident = la.conf[p] >= la.threshold;
+        if (confident && do_table && la.cand) {
             const int4 *cp = reinterpret_cast<const int4 *>(la.cand + (size_t) p * PT_PROP_TOPK);
             const int4 c0 = cp[0], c1 = cp[1];
             const int raw[PT_PROP_TOPK] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            int cand[PT_PROP_TOPK + 1];
-            unsigned keep = 0;
-            const int own = pt_xy(xb, yb);
+            int cand[PT_PROP_TOPK];
 #pragma unroll
             for (int j = 0; j < PT_PROP_TOPK; j++) {
-                const int px = pt_x(raw[j]) - 7, py = pt_y(raw[j]) - 7;
-                const bool in_b = raw[j] >= 0 && px >= 0 && py >= 0 && px < c_q.bew && py < c_q.beh;
-                cand[j] = in_b ? pt_xy(px, py) : -1;
-                bool dup = !in_b || cand[j] == own;
+                cand[j] = raw[j] >= 0 ? entry(raw[j]) : -1;
+                bool dup = cand[j] < 0 || cand[j] == pt_xy(xb, yb);
 #pragma unroll
                 for (int t = 0; t < j; t++) dup |= ((keep >> t) & 1) && cand[t] == cand[j];
                 if (!dup) keep |= 1u << j;
             }
-            cand[PT_PROP_TOPK] = -1;
-            constexpr int G = 3;
-#pragma unroll
-            for (int g0 = 0; g0 < PT_PROP_TOPK; g0 += G) {
-                const unsigned m = (keep >> g0) & ((1u << G) - 1);
-                if (!m) continue;
-                const int cg[G] = {cand[g0], cand[g0 + 1], g0 + 2 <= PT_PROP_TOPK ? cand[g0 + 2] : -1};
-                float d[G];
-                dist_group<TW, G, DESC>(aq, c_q, b, cg, m, dbest, d, rows);
-#pragma unroll
-                for (int g = 0; g < G; g++)
-                    if (((m >> g) & 1) && d[g] < dbest) { dbest = d[g]; dch = d[g]; xb = pt_x(cg[g]); yb = pt_y(cg[g]); }
-            }
             n_prop = __popc(keep);
-            ne += n_prop;
             n_conf = 1;
-        } else if (do_table) {
-            int v = tcand[p];
-            int xs = pt_x(v) - 7, ys = pt_y(v) - 7;
-            /* a table built here only holds patches of b; the range test guards against a corrupt
-               table file or entry array, which must not make the kernel read outside b */
-            const bool in_b = xs >= 0 && ys >= 0 && xs < c_q.bew && ys < c_q.beh;
-            if (in_b && (xs != xb || ys != yb)) {
-                float dc = dist1<TW, DESC>(aq, c_q, b, xs, ys, dbest, rows);
-                ne++;
-                if (dc < dbest) { dbest = dc; dch = dc; xb = xs; yb = ys; }
-            }
-            /* Further tables (patchtable.h:3711-3735): each entry is scored unless it equals the
-               best so far or the previous table's entry. */
-            const size_t np = (size_t) c_q.ew * c_q.eh;
-            for (int k = 0; k < (LEAN ? 0 : c_q.ntc); k++) {
-                const int v1 = c_q.tcand_more[(size_t) k * np + p];
-                const int xs1 = pt_x(v1) - 7, ys1 = pt_y(v1) - 7;
-                const bool in_b1 = xs1 >= 0 && ys1 >= 0 && xs1 < c_q.bew && ys1 < c_q.beh;
-                if (in_b1 && (xs1 != xb || ys1 != yb) && (xs1 != xs || ys1 != ys)) {
-                    float dc = dist1<TW, DESC>(aq, c_q, b, xs1, ys1, dbest, rows);
-                    ne++;
-                    if (dc < dbest) { dbest = dc; dch = dc; xb = xs1; yb = ys1; }
-                }
-                xs = xs1;
-                ys = ys1;
-            }
         }
-        const int kc_src = pt_xy(xb, yb);
-        const bool repeat = use_done && kc_done[p] == kc_src;
-        bool accepted = false;
-        const bool kc_here = !LEARNED || !confident || la.kcoh_confident;
-        if (!LEAN && c_q.do_kcoh && kc_here && !repeat && xb < c_q.bew && yb < c_q.beh) {
-            /* The reference tries the list in order and stops at the first neighbour whose stored
-               distance reaches triangle * best.  Here two neighbours are scored together with the
-               best known before the group as the early-exit bound, then the sequential decisions
-               are replayed: a sum cut short by that looser bound could not have been accepted, and
-               one that completes is exact, so the outcome equals the one-by-one loop. */
-            const int ks = c_q.ks;
-            const int2 *kp = kcoh + ((size_t) (yb / ks) * c_q.bew + (xb / ks)) * c_q.kc;
-            const int kdx = ks > 1 ? xb % ks : 0, kdy = ks > 1 ? yb % ks : 0;
-            constexpr int G = 2;             /* -speed presets list 2 to 20 neighbours; pairs keep registers low */
-            bool done = false;
-            for (int k = 0; k < c_q.kc_try && !done; k += G) {
-                int cg[G];
-                float kdg[G];
-                unsigned m = 0;
-#pragma unroll
-                for (int j = 0; j < G; j++) {
-                    cg[j] = 0;
-                    kdg[j] = 0.f;
-                    if (m == (1u << j) - 1 && k + j < c_q.kc_try) {
-                        const int2 e = kp[k + j];
-                        const float kd = __int_as_float(e.y);
-                        if ((double) kd < c_q.triangle * (double) dbest) {
-                            int xs = pt_x(e.x) + kdx, ys = pt_y(e.x) + kdy;
-                            if (xs >= c_q.bew) xs = c_q.bew - 1;
-                            if (ys >= c_q.beh) ys = c_q.beh - 1;
-                            cg[j] = pt_xy(xs, ys);
-                            kdg[j] = kd;
-                            m |= 1u << j;
+    }
+    const bool table = do_table && !(LEARNED && confident && la.cand);
+    enum { PROPOSALS, TABLES, KCOH, WINDOW, RANDOM, DONE };
+    int ph = live ? (LEARNED ? PROPOSALS : TABLES) : DONE;
+    int it = 0;
+    int xs1 = 0, ys1 = 0;                 /* the previous table's entry */
+    int kc_src = 0, kdx = 0, kdy = 0;
+    bool repeat = false, accepted = false;
+    const int2 *kp = kcoh;
+    int wx = 0, wy = 0, wx0 = 0, wx1 = 0, wy1 = 0, own = 0;
+    const size_t np = (size_t) c_q.ew * c_q.eh;
+    for (;;) {
+        int cand = -1;
+        while (cand < 0 && ph != DONE) {
+            if (LEARNED && ph == PROPOSALS) {
+                if (!keep) { ph = TABLES; continue; }
+                const int j = __ffs(keep) - 1;
+                keep &= keep - 1;
+                cand = entry(la.cand[(size_t) p * PT_PROP_TOPK + j]);
+            } else if (ph == TABLES) {
+                /* the first table's entry, then the further tables' (patchtable.h:3711-3735): each is
+                   scored unless it equals the best so far or the previous table's entry */
+                if (!table || it > c_q.ntc) {
+                    ph = KCOH;
+                    it = 0;
+                    kc_src = pt_xy(xb, yb);
+                    if (c_q.do_kcoh) {
+                        repeat = use_done && kc_done[p] == kc_src;
+                        if ((!LEARNED || !confident || la.kcoh_confident) && !repeat && xb < c_q.bew && yb < c_q.beh) {
+                            const int ks = c_q.ks;
+                            kp = kcoh + ((size_t) (yb / ks) * c_q.bew + (xb / ks)) * c_q.kc;
+                            if (ks > 1) { kdx = xb % ks; kdy = yb % ks; }
+                            continue;
                         }
                     }
+                    it = c_q.kc_try;      /* nothing to try */
+                    continue;
                 }
-                if (m != (1u << G) - 1) done = true;     /* the list ends or stops inside this group */
-                if (!m) break;
-                float d[G];
-                dist_group<TW, G, DESC>(aq, c_q, b, cg, m, dbest, d, rows);
-                ne += __popc(m);
-#pragma unroll
-                for (int j = 0; j < G; j++) {
-                    if (!((m >> j) & 1)) continue;
-                    if ((double) kdg[j] >= c_q.triangle * (double) dbest) { done = true; break; }
-                    if (d[j] < dbest) { dbest = d[j]; dch = d[j]; xb = pt_x(cg[j]); yb = pt_y(cg[j]); accepted = true; }
+                const int v = it == 0 ? tcand[p] : c_q.tcand_more[(size_t) (it - 1) * np + p];
+                const int xs = pt_x(v) - 7, ys = pt_y(v) - 7;
+                const int e = entry(v);
+                if (e >= 0 && e != pt_xy(xb, yb) && (it == 0 || xs != xs1 || ys != ys1)) cand = e;
+                xs1 = xs;
+                ys1 = ys;
+                it++;
+            } else if (ph == KCOH) {
+                /* the reference tries the list in order and stops at the first neighbour whose
+                   stored distance reaches triangle * best */
+                int2 e = make_int2(0, 0);
+                bool go = it < c_q.kc_try;
+                if (go) {
+                    e = kp[it++];
+                    go = (double) __int_as_float(e.y) < c_q.triangle * (double) dbest;
                 }
+                if (go) {
+                    cand = pt_xy(min(pt_x(e.x) + kdx, c_q.bew - 1), min(pt_y(e.x) + kdy, c_q.beh - 1));
+                    continue;
+                }
+                ph = DONE;
+                if (c_q.do_kcoh) kc_done[p] = (repeat || !accepted) ? kc_src : -1;
+                if (xb < c_q.bew && yb < c_q.beh) {
+                    if (c_q.spatial > 0) {
+                        /* Spatial search (patchtable.h:3855-3873): every other patch of the (2s+1)^2
+                           window around the best match, rows then columns. */
+                        const int S = c_q.spatial;
+                        ph = WINDOW;
+                        own = pt_xy(xb, yb);
+                        wy = max(yb - S, 0);
+                        wy1 = min(yb + S + 1, c_q.beh);
+                        wx0 = max(xb - S, 0);
+                        wx1 = min(xb + S + 1, c_q.bew);
+                        wx = wx0;
+                    } else if (c_q.do_rs) {
+                        ph = RANDOM;
+                    }
+                }
+            } else if (ph == WINDOW) {
+                if (wy >= wy1) { ph = DONE; continue; }
+                const int e = pt_xy(wx, wy);
+                if (e != own && (!c_q.allowed || __ldg(c_q.allowed + (size_t) wy * c_q.bew + wx) == c_q.allowed_index)) cand = e;
+                if (++wx >= wx1) { wx = wx0; wy++; }
+            } else {
+                ph = DONE;
+                cand = random_neighbour(c_q, p, xb, yb);
             }
         }
-        if (!LEAN && c_q.do_kcoh) kc_done[p] = (repeat || !accepted) ? kc_src : -1;
-        const bool have = xb < c_q.bew && yb < c_q.beh;
-        if (!LEAN && c_q.spatial > 0 && have) {
-            /* Spatial search (patchtable.h:3855-3873): every other patch of the (2s+1)^2 window
-               around the best match, rows then columns, scored in pairs and replayed in order. */
-            const int S = c_q.spatial, xb0 = xb, yb0 = yb;
-            int symin = yb0 - S, symax = yb0 + S + 1, sxmin = xb0 - S, sxmax = xb0 + S + 1;
-            if (symin < 0) symin = 0; else if (symax > c_q.beh) symax = c_q.beh;
-            if (sxmin < 0) sxmin = 0; else if (sxmax > c_q.bew) sxmax = c_q.bew;
-            if (symax > c_q.beh) symax = c_q.beh;          /* windows wider than b */
-            if (sxmax > c_q.bew) sxmax = c_q.bew;
-            const int swd = sxmax - sxmin, nwin = (symax - symin) * swd;
-            constexpr int G = 2;
-            for (int i0 = 0; i0 < nwin; i0 += G) {
-                int cg[G];
-                unsigned m = 0;
-#pragma unroll
-                for (int j = 0; j < G; j++) {
-                    cg[j] = 0;
-                    const int i = i0 + j;
-                    if (i >= nwin) continue;
-                    const int ys = symin + i / swd, xs = sxmin + i % swd;
-                    if (xs == xb0 && ys == yb0) continue;
-                    if (c_q.allowed && __ldg(c_q.allowed + (size_t) ys * c_q.bew + xs) != c_q.allowed_index) continue;
-                    cg[j] = pt_xy(xs, ys);
-                    m |= 1u << j;
-                }
-                if (!m) continue;
-                float d[G];
-                dist_group<TW, G, DESC>(aq, c_q, b, cg, m, dbest, d, rows);
-                ne += __popc(m);
-#pragma unroll
-                for (int j = 0; j < G; j++)
-                    if (((m >> j) & 1) && d[j] < dbest) { dbest = d[j]; dch = d[j]; xb = pt_x(cg[j]); yb = pt_y(cg[j]); }
+        if (!__any_sync(FULL, cand >= 0)) break;
+        const float d = dist32<TP, false, true>(aq, c_q, cand, cand >= 0, dbest, rows);
+        if (cand >= 0) {
+            ne++;
+            if (d < dbest) {
+                dbest = dch = d;
+                xb = pt_x(cand);
+                yb = pt_y(cand);
+                if (ph == KCOH) accepted = true;
             }
-        } else if (!LEAN && c_q.do_rs && have) {
-            /* Random search (patchtable.h:3874-3903): one of the 8 neighbours of the best match.
-               dx, dy + 1 for r = 0..7 are packed two bits each: {-1,0,1,-1,1,-1,0,1},
-               {-1,-1,-1,0,0,1,1,1}. */
-            const unsigned r = mix32((unsigned) p * 2654435761u + (unsigned) c_q.pass * 0x9e3779b9u + 0x6a09e667u) & 7u;
-            const int xs = xb + (int) ((37412u >> (2 * r)) & 3u) - 1, ys = yb + (int) ((43328u >> (2 * r)) & 3u) - 1;
-            if (xs >= 0 && xs < c_q.bew && ys >= 0 && ys < c_q.beh &&
-                (!c_q.allowed || __ldg(c_q.allowed + (size_t) ys * c_q.bew + xs) == c_q.allowed_index)) {
-                const float dc = dist1<TW, DESC>(aq, c_q, b, xs, ys, dbest, rows);
-                ne++;
-                if (dc < dbest) { dbest = dc; dch = dc; xb = xs; yb = ys; }
+        }
+    }
+    if (live) { ch_pos[p] = pt_xy(xb, yb); ch_d[p] = dch; }
+    count_work(counters, ne, rows);
+    if (LEARNED && la.counters) {
+        unsigned c = __reduce_add_sync(FULL, n_conf), n = __reduce_add_sync(FULL, n_prop);
+        if ((threadIdx.x & 31) == 0) { atomicAdd(la.counters, (unsigned long long) c); atomicAdd(la.counters + 1, (unsigned long long) n); }
+    }
+}
+
+template<int TP, bool LEARNED, bool LEAN = false>
+__global__ void __launch_bounds__(TP, min_ctas(LEAN ? CHOOSE_LEAN_LANES : CHOOSE_LANES, TP))
+k_choose_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
+              const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
+              int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs la) {
+    extern __shared__ float at[];
+    choose_tile<TP, LEARNED, LEAN>(c_q, at, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done,
+                                   counters, la, blockIdx.x * tile_w(TP), blockIdx.y * tile_h(TP) + c_q.row0,
+                                   c_q.row0 + c_q.rows);
+}
+
+/* The choose in descriptor mode: each lane walks its patch's candidates by itself (a candidate is one
+   or two sectors, nothing to share), the k-coherence neighbours two at a time so that the walk waits
+   for memory once per pair.  The lockstep walk of choose_tile measured 0.129 against 0.124 ms here
+   (540 x 960, 8 channels, the four chooses of the default schedule). */
+__global__ void __launch_bounds__(TILE_DESC, 10 * 64 / TILE_DESC)
+k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restrict__ cur_d,
+              const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table, int *ch_pos, float *ch_d,
+              int *kc_done, int use_done, unsigned long long *counters) {
+    const int x = blockIdx.x * TILE_DESC + threadIdx.x, y = blockIdx.y + q.row0;
+    unsigned ne = 0;
+    if (x < q.ew) {
+        const int p = y * q.ew + x;
+        float4 av[4];
+        pt_desc_load(q.adesc + (size_t) p * q.ds4, 4 * q.ds4, av);
+        const int pos = cur_pos ? cur_pos[p] : pt_xy(q.bew + 1, 0);
+        float dch = cur_d ? cur_d[p] : (float) PT_DIST_INF;
+        float dbest = (float) ((double) dch * q.prop_scale);
+        int xb = pt_x(pos), yb = pt_y(pos);
+        auto dist = [&](int c) { return pt_desc_dist(av, q.bdesc + ((size_t) pt_y(c) * q.bew + pt_x(c)) * q.ds4, q.nd); };
+        auto offer = [&](int c, float d) {
+            ne++;
+            if (!(d < dbest)) return false;
+            dbest = dch = d;
+            xb = pt_x(c);
+            yb = pt_y(c);
+            return true;
+        };
+        if (do_table) {
+            int prev = 0;
+            for (int k = 0; k <= q.ntc; k++) {
+                const int v = k == 0 ? tcand[p] : q.tcand_more[(size_t) (k - 1) * q.ew * q.eh + p];
+                const int c = table_entry(q, v);
+                if (c >= 0 && c != pt_xy(xb, yb) && (k == 0 || v != prev)) offer(c, dist(c));
+                prev = v;
+            }
+        }
+        const int src = pt_xy(xb, yb);
+        const bool repeat = use_done && kc_done[p] == src;
+        bool accepted = false;
+        if (q.do_kcoh && !repeat && xb < q.bew && yb < q.beh) {
+            const int ks = q.ks;
+            const int2 *kp = kcoh + ((size_t) (yb / ks) * q.bew + (xb / ks)) * q.kc;
+            const int kdx = ks > 1 ? xb % ks : 0, kdy = ks > 1 ? yb % ks : 0;
+            for (int k = 0; k < q.kc_try; k += 2) {
+                const int2 e0 = kp[k], e1 = k + 1 < q.kc_try ? kp[k + 1] : e0;
+                auto near = [&](const int2 &e) { return (double) __int_as_float(e.y) < q.triangle * (double) dbest; };
+                auto place = [&](const int2 &e) { return pt_xy(min(pt_x(e.x) + kdx, q.bew - 1), min(pt_y(e.x) + kdy, q.beh - 1)); };
+                if (!near(e0)) break;
+                const int c0 = place(e0), c1 = place(e1);
+                const bool two = k + 1 < q.kc_try && near(e1);
+                const float d0 = dist(c0), d1 = two ? dist(c1) : 0.f;
+                accepted |= offer(c0, d0);
+                if (!two || !near(e1)) break;
+                accepted |= offer(c1, d1);
+            }
+        }
+        if (q.do_kcoh) kc_done[p] = (repeat || !accepted) ? src : -1;
+        if (xb < q.bew && yb < q.beh) {
+            if (q.spatial > 0) {
+                const int S = q.spatial, xb0 = xb, yb0 = yb;
+                for (int ys = max(yb0 - S, 0); ys < min(yb0 + S + 1, q.beh); ys++)
+                    for (int xs = max(xb0 - S, 0); xs < min(xb0 + S + 1, q.bew); xs++) {
+                        if (xs == xb0 && ys == yb0) continue;
+                        if (q.allowed && __ldg(q.allowed + (size_t) ys * q.bew + xs) != q.allowed_index) continue;
+                        offer(pt_xy(xs, ys), dist(pt_xy(xs, ys)));
+                    }
+            } else if (q.do_rs) {
+                const int c = random_neighbour(q, p, xb, yb);
+                if (c >= 0) offer(c, dist(c));
             }
         }
         ch_pos[p] = pt_xy(xb, yb);
         ch_d[p] = dch;
     }
-    count_work(counters, ne, rows);
-    if (LEARNED && la.counters) {
-        unsigned c = __reduce_add_sync(0xffffffffu, n_conf), q = __reduce_add_sync(0xffffffffu, n_prop);
-        if ((threadIdx.x & 31) == 0) { atomicAdd(la.counters, (unsigned long long) c); atomicAdd(la.counters + 1, (unsigned long long) q); }
-    }
-}
-
-/* At least 10 x 64 threads' worth of CTAs per SM: the register budget this leaves keeps the gather
-   latency hidden without the spills of tighter caps (measured at 1080p, 64 patches per CTA:
-   choose 0.70 ms unrestricted, 0.611 at 10 x 64, 0.619 at 12 x 64, 0.625 at 16 x 64). */
-template<int TW, bool LEARNED, bool DESC, bool LEAN = false>
-__global__ void __launch_bounds__(TW, (LEAN ? CHOOSE_LEAN_LANES : 10 * 64) / TW)
-k_choose_tile(const QPlan c_q, const float4 *__restrict__ a, const float4 *__restrict__ b, const int *__restrict__ cur_pos,
-              const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
-              int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs la) {
-    extern __shared__ float4 atile[];
-    choose_seg<TW, LEARNED, DESC, LEAN>(c_q, atile, a, b, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done,
-                                        use_done, counters, la, blockIdx.x * TW, blockIdx.y + c_q.row0);
+    count_work(counters, ne, ne);
 }
 
 /* Step 4 as a pull: the best of the stored match and every neighbour's chosen offset applied to
    this patch.  The patch's own choice comes first; the distinct neighbour candidates follow in
    increasing order of the distance their neighbour achieved with them (the likeliest good ones
-   first, so the running best -- the early-exit bound -- tightens soonest), three at a time.
+   first, so the running best -- the early-exit bound -- tightens soonest).
    Neighbours sit `step` patches apart; passes with decreasing steps (jump flooding) carry an
    offset across a region in a logarithmic number of passes, where the reference's sequential
    sweep carries it along a whole row in one sweep. */
 /* ONE: a single neighbour candidate per patch (pull_max 1).  The candidate is the one the
    general path would sort first -- among distinct candidates keyed by their first occurrence, the
    smallest key, the earliest on ties -- found in one streaming pass, and it is scored alone. */
-template<int TW, int R, bool DESC, bool ONE = false>
+template<int TP, int R, bool DESC, bool ONE>
 __device__ __forceinline__ void
-pull_seg(const QPlan &c_q, float4 *atile, const float4 *__restrict__ a, const float4 *__restrict__ b,
-         const int *__restrict__ cur_pos, const float *__restrict__ cur_d, const int *__restrict__ ch_pos,
-         const float *__restrict__ ch_d, int *nxt_pos, float *nxt_d, unsigned long long *counters, int x0, int y) {
+pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
+          const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos,
+          float *nxt_d, unsigned long long *counters, int x0, int y0, int y1) {
+    const unsigned FULL = 0xffffffffu;
     if constexpr (!DESC) {
-        stage_a<TW>(atile, a, c_q.aw, c_q.ah, x0, y);
+        stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
         __syncthreads();
     }
-    const int x = x0 + threadIdx.x;
-    const bool live = x < c_q.ew;
+    AQuery aq;
+    int x, y;
+    tile_lane<TP, DESC>(c_q, at, x0, y0, x, y, aq);
+    const bool live = x < c_q.ew && y < y1;
+    const int p = live ? y * c_q.ew + x : 0;
+    if constexpr (DESC) pt_desc_load(c_q.adesc + (size_t) p * c_q.ds4, 4 * c_q.ds4, aq.v);
     unsigned ne = 0, rows = 0;
-    if (live) {
-        const int p = y * c_q.ew + x;
-        AQuery aq;
-        aq.atile = atile;
-        aq.tx = threadIdx.x;
-        if constexpr (DESC) pt_desc_load(c_q.adesc + (size_t) p * c_q.ds4, 4 * c_q.ds4, aq.v);
-        int bpos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);      /* null: the initial field */
-        float bd = cur_d ? cur_d[p] : (float) PT_DIST_INF;
-        {
-            int cp = ch_pos[p];
-            if (pt_x(cp) < c_q.bew && pt_y(cp) < c_q.beh && cp != bpos && ch_d[p] < bd) { bd = ch_d[p]; bpos = cp; }
-        }
-        constexpr int MAXC = (2 * R + 1) * (2 * R + 1) - 1;
-        const int S = c_q.step;
-        int nc = 0;
-        if constexpr (ONE) {
-            /* the distinct candidates seen so far, newest first (fixed register slots) */
-            int seen[MAXC];
-#pragma unroll
-            for (int t = 0; t < MAXC; t++) seen[t] = -1;
-            int best = -1;
-            float bestk = finf();
-#pragma unroll
-            for (int dy = -R; dy <= R; dy++) {
-#pragma unroll
-                for (int dx = -R; dx <= R; dx++) {
-                    if (dx == 0 && dy == 0) continue;
-                    const int ny = y + S * dy, nx = x + S * dx;
-                    if (ny < 0 || ny >= c_q.eh || nx < 0 || nx >= c_q.ew) continue;
-                    const int q = ny * c_q.ew + nx;
-                    const int cp = ch_pos[q];
-                    const int xs = pt_x(cp) - S * dx, ys = pt_y(cp) - S * dy;
-                    if (xs < 0 || ys < 0 || xs >= c_q.bew || ys >= c_q.beh) continue;
-                    if (c_q.allowed && __ldg(c_q.allowed + (size_t) ys * c_q.bew + xs) != c_q.allowed_index) continue;
-                    const int c = pt_xy(xs, ys);
-                    bool dup = c == bpos;
-#pragma unroll
-                    for (int t = 0; t < MAXC; t++) dup |= seen[t] == c;
-                    if (dup) continue;
-#pragma unroll
-                    for (int t = MAXC - 1; t > 0; t--) seen[t] = seen[t - 1];
-                    seen[0] = c;
-                    const float k = ch_d[q];
-                    if (k < bestk) { bestk = k; best = c; }   /* the general sort's insertion rule */
-                    nc++;
-                }
-            }
-            nc = best >= 0 ? 1 : 0;
-            if (nc) {
-                const float d = dist1<TW, DESC>(aq, c_q, b, pt_x(best), pt_y(best), bd, rows);
-                if (d < bd) { bd = d; bpos = best; }
-            }
-        } else {
-        /* distinct neighbour candidates sorted by the neighbour's own distance (ties keep the
-           neighbour order), kept in registers: every slot index is known at compile time */
-        int cand[MAXC];
-        float key[MAXC];
-#pragma unroll
-        for (int t = 0; t < MAXC; t++) { cand[t] = -1; key[t] = finf(); }
+    int bpos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);      /* null: the initial field */
+    float bd = cur_d ? cur_d[p] : (float) PT_DIST_INF;
+    {
+        const int cp = ch_pos[p];
+        const float cd = ch_d[p];
+        if (pt_x(cp) < c_q.bew && pt_y(cp) < c_q.beh && cp != bpos && cd < bd) { bd = cd; bpos = cp; }
+    }
+    constexpr int MAXC = (2 * R + 1) * (2 * R + 1) - 1;
+    const int S = c_q.step;
+    int nc = 0;
+    /* calls fn(candidate, the neighbour's own distance) for every neighbour's offset inside b */
+    auto neighbours = [&](auto &&fn) {
 #pragma unroll
         for (int dy = -R; dy <= R; dy++) {
 #pragma unroll
             for (int dx = -R; dx <= R; dx++) {
                 if (dx == 0 && dy == 0) continue;
                 const int ny = y + S * dy, nx = x + S * dx;
-                if (ny < 0 || ny >= c_q.eh || nx < 0 || nx >= c_q.ew) continue;
-                const int q = ny * c_q.ew + nx;
-                const int cp = ch_pos[q];
+                if (!live || ny < 0 || ny >= c_q.eh || nx < 0 || nx >= c_q.ew) continue;
+                const int n = ny * c_q.ew + nx;
+                const int cp = ch_pos[n];
                 const int xs = pt_x(cp) - S * dx, ys = pt_y(cp) - S * dy;
                 if (xs < 0 || ys < 0 || xs >= c_q.bew || ys >= c_q.beh) continue;
                 if (c_q.allowed && __ldg(c_q.allowed + (size_t) ys * c_q.bew + xs) != c_q.allowed_index) continue;
-                int c = pt_xy(xs, ys);
-                bool dup = c == bpos;
+                fn(pt_xy(xs, ys), ch_d + n);
+            }
+        }
+    };
+    if constexpr (ONE) {
+        /* the distinct candidates seen so far, newest first (fixed register slots) */
+        int seen[MAXC];
 #pragma unroll
-                for (int t = 0; t < MAXC; t++) dup |= cand[t] == c;
-                if (dup) continue;
-                float k = ch_d[q];
+        for (int t = 0; t < MAXC; t++) seen[t] = -1;
+        int best = -1;
+        float bestk = finf();
+        neighbours([&](int c, const float *kp) {
+            bool dup = c == bpos;
 #pragma unroll
-                for (int t = 0; t < MAXC; t++) {
-                    if (k < key[t]) {
-                        const float tk = key[t]; key[t] = k; k = tk;
-                        const int tc = cand[t]; cand[t] = c; c = tc;
-                    }
+            for (int t = 0; t < MAXC; t++) dup |= seen[t] == c;
+            if (dup) return;
+#pragma unroll
+            for (int t = MAXC - 1; t > 0; t--) seen[t] = seen[t - 1];
+            seen[0] = c;
+            const float k = *kp;
+            if (k < bestk) { bestk = k; best = c; }   /* the general sort's insertion rule */
+        });
+        const float d = dist32<TP, DESC, true>(aq, c_q, best, best >= 0, bd, rows);
+        if (best >= 0) {
+            ne = 1;
+            if (d < bd) { bd = d; bpos = best; }
+        }
+    } else {
+        /* distinct neighbour candidates sorted by the neighbour's own distance (ties keep the
+           neighbour order), kept in registers: every slot index is known at compile time */
+        int cand[MAXC];
+        float key[MAXC];
+#pragma unroll
+        for (int t = 0; t < MAXC; t++) { cand[t] = -1; key[t] = finf(); }
+        neighbours([&](int c, const float *kp) {
+            bool dup = c == bpos;
+#pragma unroll
+            for (int t = 0; t < MAXC; t++) dup |= cand[t] == c;
+            if (dup) return;
+            float k = *kp;
+#pragma unroll
+            for (int t = 0; t < MAXC; t++) {
+                if (k < key[t]) {
+                    const float tk = key[t]; key[t] = k; k = tk;
+                    const int tc = cand[t]; cand[t] = c; c = tc;
                 }
-                nc++;
             }
-        }
+            nc++;
+        });
         if (nc > c_q.pull_max) nc = c_q.pull_max;   /* the best-first prefix of the list */
-        constexpr int G = 3;
+        ne = nc;
+        if constexpr (DESC) {
+            float d[MAXC];                          /* every candidate's loads in flight at once */
 #pragma unroll
-        for (int g0 = 0; g0 < MAXC; g0 += G) {
-            if (g0 < nc) {
-                const int cg[G] = {cand[g0], g0 + 1 < MAXC ? cand[g0 + 1] : -1, g0 + 2 < MAXC ? cand[g0 + 2] : -1};
-                const int left = nc - g0;
-                const unsigned m = left >= G ? (1u << G) - 1 : (1u << left) - 1;
-                float d[G];
-                dist_group<TW, G, DESC>(aq, c_q, b, cg, m, bd, d, rows);
+            for (int t = 0; t < MAXC; t++) d[t] = dist32<TP, DESC, false>(aq, c_q, cand[t], t < nc, bd, rows);
 #pragma unroll
-                for (int g = 0; g < G; g++)
-                    if (((m >> g) & 1) && d[g] < bd) { bd = d[g]; bpos = cg[g]; }
+            for (int t = 0; t < MAXC; t++)
+                if (t < nc && d[t] < bd) { bd = d[t]; bpos = cand[t]; }
+        } else {
+            for (int t0 = 0; __any_sync(FULL, t0 < nc); t0++) {
+                const int c = cand[0];
+                const float d = dist32<TP, DESC, true>(aq, c_q, c, t0 < nc, bd, rows);
+                if (t0 < nc && d < bd) { bd = d; bpos = c; }
+#pragma unroll
+                for (int t = 0; t + 1 < MAXC; t++) cand[t] = cand[t + 1];
             }
         }
-        }
-        ne += nc;
+    }
+    if (live) {
         if (c_q.ann) {                          /* k_output fused: x, y, dist of the final field */
             double *o = c_q.ann + 3 * (size_t) p;
             o[0] = pt_x(bpos);
@@ -598,22 +694,19 @@ pull_seg(const QPlan &c_q, float4 *atile, const float4 *__restrict__ a, const fl
     count_work(counters, ne, rows);
 }
 
-/* At most 14 x 64 threads' worth of CTAs per SM (73 registers, 10 bytes of spills): the pull is
-   latency-bound, and the extra resident warps hide the gathers (measured at 1080p with one
-   candidate per patch: 0.341 -> 0.286 ms; at 16 x 64 the spills grow to 200 bytes and it slows). */
-template<int TW, int R, bool DESC, bool ONE = false>
-__global__ void __launch_bounds__(TW, (ONE ? PULL_ONE_LANES : 14 * 64) / TW)
-k_pull_tile(const QPlan c_q, const float4 *__restrict__ a, const float4 *__restrict__ b, const int *__restrict__ cur_pos,
+template<int TP, int R, bool DESC, bool ONE = false>
+__global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES, TP))
+k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
             const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
             int *nxt_pos, float *nxt_d, unsigned long long *counters) {
-    extern __shared__ float4 atile[];
-    pull_seg<TW, R, DESC, ONE>(c_q, atile, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters, blockIdx.x * TW,
-                               blockIdx.y + c_q.row0);
+    extern __shared__ float at[];
+    pull_tile<TP, R, DESC, ONE>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
+                                blockIdx.x * cta_w(TP, DESC), blockIdx.y * cta_h(TP, DESC) + c_q.row0, c_q.row0 + c_q.rows);
 }
 
-/* ---- batched queries: many images, one launch per phase over a flattened segment list ---- */
+/* ---- batched queries: many images, one launch per phase over a flattened tile list ---- */
 
-/* Index of the image that owns flattened segment s (segs[i] = first segment of image i). */
+/* Index of the image that owns flattened tile s (segs[i] = first tile of image i). */
 __device__ __forceinline__ int owner(const PtBatchImage *__restrict__ imgs, int n, long long s, int twi) {
     int lo = 0, hi = n - 1;
     while (lo < hi) {
@@ -623,13 +716,13 @@ __device__ __forceinline__ int owner(const PtBatchImage *__restrict__ imgs, int 
     return lo;
 }
 
-/* Runs body(s) for the row segments this CTA takes from the launch's work counter (zeroed before
-   the launch): segments go out in order, one at a time, to whichever CTA is free, so uneven
-   segment costs cannot leave some CTAs with a longer share.  A CTA claims its next segment when it
+/* Runs body(s) for the tiles this CTA takes from the launch's work counter (zeroed before
+   the launch): tiles go out in order, one at a time, to whichever CTA is free, so uneven
+   tile costs cannot leave some CTAs with a longer share.  A CTA claims its next tile when it
    starts the current one and reads the claim only after it, so the counter's round trip overlaps
    the work. */
 template<class Body>
-__device__ __forceinline__ void for_each_segment(unsigned long long *work, long long nseg, Body &&body) {
+__device__ __forceinline__ void for_each_tile(unsigned long long *work, long long nseg, Body &&body) {
     __shared__ long long s_next;
     if (threadIdx.x == 0) s_next = (long long) atomicAdd(work, 1ull);
     __syncthreads();
@@ -645,68 +738,76 @@ __device__ __forceinline__ void for_each_segment(unsigned long long *work, long 
     }
 }
 
-/* Persistent choose over every row segment of every image, handed out by a work counter. */
-template<int TW, bool LEAN = false>
-__global__ void __launch_bounds__(TW, (LEAN ? CHOOSE_LEAN_LANES : 10 * 64) / TW)
+/* Persistent choose over every tile of every image, handed out by a work counter. */
+template<int TP, bool LEAN = false>
+__global__ void __launch_bounds__(TP, min_ctas(LEAN ? CHOOSE_LEAN_LANES : CHOOSE_LANES, TP))
 k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
-               const float4 *__restrict__ a, const float4 *__restrict__ b, const int *__restrict__ cur_pos,
+               const float *__restrict__ a, const int *__restrict__ cur_pos,
                const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
                int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters,
                unsigned long long *work) {
-    extern __shared__ float4 atile[];
+    extern __shared__ float at[];
     LearnedArgs none;
     none.cand = nullptr; none.conf = nullptr; none.threshold = 0.f; none.kcoh_confident = 0; none.counters = nullptr;
-    for_each_segment(work, nseg, [&](long long s) {
+    for_each_tile(work, nseg, [&](long long s) {
         const int i = owner(imgs, n, s, twi);
         const PtBatchImage &g = imgs[i];
-        const long long ls = s - g.seg_off[twi];
-        const int spr = (g.ew + TW - 1) / TW;
-        const int y = (int) (ls / spr), x0 = (int) (ls % spr) * TW;
+        const int ls = (int) (s - g.seg_off[twi]);
+        const int spr = (g.ew + tile_w(TP) - 1) / tile_w(TP);
         QPlan q = base;
         q.aw = g.w; q.ah = g.h; q.ew = g.ew; q.eh = g.eh;
         const long long o = g.patch_off;
-        choose_seg<TW, false, false, LEAN>(q, atile, a + g.pix_off, b, cur_pos ? cur_pos + o : nullptr,
-                                           cur_d ? cur_d + o : nullptr, tcand + o, kcoh, do_table, ch_pos + o, ch_d + o,
-                                           kc_done + o, use_done, counters, none, x0, y);
+        choose_tile<TP, false, LEAN>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
+                                            cur_d ? cur_d + o : nullptr, tcand + o, kcoh, do_table, ch_pos + o, ch_d + o,
+                                            kc_done + o, use_done, counters, none, (ls % spr) * tile_w(TP),
+                                            (ls / spr) * tile_h(TP), g.eh);
     });
 }
 
-template<int TW, int R, bool ONE = false>
-__global__ void __launch_bounds__(TW, (ONE ? PULL_ONE_LANES : 14 * 64) / TW)
+template<int TP, int R, bool ONE = false>
+__global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES, TP))
 k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
-             const float4 *__restrict__ a, const float4 *__restrict__ b, const int *__restrict__ cur_pos,
+             const float *__restrict__ a, const int *__restrict__ cur_pos,
              const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
              int *nxt_pos, float *nxt_d, unsigned long long *counters, unsigned long long *work) {
-    extern __shared__ float4 atile[];
-    for_each_segment(work, nseg, [&](long long s) {
+    extern __shared__ float at[];
+    for_each_tile(work, nseg, [&](long long s) {
         const int i = owner(imgs, n, s, twi);
         const PtBatchImage &g = imgs[i];
-        const long long ls = s - g.seg_off[twi];
-        const int spr = (g.ew + TW - 1) / TW;
-        const int y = (int) (ls / spr), x0 = (int) (ls % spr) * TW;
+        const int ls = (int) (s - g.seg_off[twi]);
+        const int spr = (g.ew + tile_w(TP) - 1) / tile_w(TP);
         QPlan q = base;
         q.aw = g.w; q.ah = g.h; q.ew = g.ew; q.eh = g.eh;
         const long long o = g.patch_off;
         if (base.ann) q.ann = base.ann + 3 * o;        /* last pass: this image's NNF records */
-        pull_seg<TW, R, false, ONE>(q, atile, a + g.pix_off, b, cur_pos ? cur_pos + o : nullptr,
-                                    cur_d ? cur_d + o : nullptr, ch_pos + o, ch_d + o, nxt_pos + o, nxt_d + o, counters, x0, y);
+        pull_tile<TP, R, false, ONE>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
+                                     cur_d ? cur_d + o : nullptr, ch_pos + o, ch_d + o, nxt_pos + o, nxt_d + o, counters,
+                                     (ls % spr) * tile_w(TP), (ls / spr) * tile_h(TP), g.eh);
     });
 }
 
-/* patch_dist_exact of a patch of a (RGBA rows in global memory) and a patch of b, in the
-   reference's lane order, without an early exit. */
-__device__ __forceinline__ float ssd_global(const QPlan &q, const float4 *__restrict__ a, int ax, int ay,
-                                           const float4 *__restrict__ B, int bx, int by) {
-    float l[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-    for (int dy = 0; dy < 8; dy++) {
-        float4 av[8], bv[8];
-        load_brow(q, B, bx, by + dy, bv);
-#pragma unroll
-        for (int p = 0; p < 8; p++) av[p] = __ldg(a + (size_t) (ay + dy) * q.aw + ax + p);
-        row_lanes(av, bv, l);
+/* The row store of a table image: for every image row and every even pixel 2c, the 32 floats
+   (10 pixels and 2 floats of the next) from that pixel on, as one 128-byte line with the floats of
+   equal index mod 4 together: float i of the run is at 8 * (i & 3) + i / 4.  A patch row at column
+   x starts at float 3 * (x & 1) of line x / 2, so its float e = j + 4 n of SSE lane j lies in the
+   8-float group (i0 & 3) at i0 / 4 + n with i0 = 3 * (x & 1) + j: one 32-byte load per lane, the
+   four lanes of a quad reading one whole line, and one select per float.  64 bytes per pixel (the
+   two RGBA copies that single-lane gathers needed took 32).  A line per third pixel takes 43 bytes
+   but two selects per float: 1080p query at one pass 0.500 against 0.462 ms, default schedule 4.40
+   against 4.02; a line per pixel (128 bytes, no select) gains 2 % more. */
+__global__ void k_row_store(const float4 *__restrict__ b, int bw, int bh, int nline, float *out) {
+    const long long t = blockIdx.x * (long long) NT + threadIdx.x;
+    if (t >= (long long) bh * nline * 32) return;
+    const long long line = t >> 5;
+    const int y = (int) (line / nline), c = (int) (line - (long long) y * nline);
+    const int g = (int) (t & 31) >> 3, m = (int) t & 7, i = 4 * m + g;
+    const int x = 2 * c + i / 3, ch = i % 3;
+    float v = 0.f;
+    if (x < bw) {
+        const float4 px = __ldg(b + (size_t) y * bw + x);
+        v = ch == 0 ? px.x : ch == 1 ? px.y : px.z;
     }
-    return lane_total(l);
+    out[t] = v;
 }
 
 /* Initial field from the previous frame's NNF (patchtable.h:3548-3585): its matches (clamped to
@@ -714,32 +815,45 @@ __device__ __forceinline__ float ssd_global(const QPlan &q, const float4 *__rest
    scale_sv[p] (when given) or temporal_scale, or the previous distance times temporal_scale.
    orig[p] keeps what the end of the lookup restores for a patch that kept this match and this
    distance (patchtable.h:4178-4193): the scaled distance divided by temporal_scale. */
-__global__ void k_init_temporal(const QPlan q, const double *__restrict__ prev, const float *__restrict__ scale_sv,
-                                int recalc, int sanitize, double temporal_scale, const float4 *__restrict__ a,
-                                const float4 *__restrict__ B, int *cur_pos, float *cur_d, double *orig, int *bad) {
-    const int p = blockIdx.x * NT + threadIdx.x;
-    if (p >= q.ew * q.eh) return;
-    const int x = p % q.ew, y = p / q.ew;
-    int xs = (int) prev[3 * (size_t) p], ys = (int) prev[3 * (size_t) p + 1];
-    if (xs < 0 || ys < 0 || xs >= q.bew || ys >= q.beh) {
-        if (!sanitize) atomicExch(bad, 1);
-        xs = min(max(xs, 0), q.bew - 1);
-        ys = min(max(ys, 0), q.beh - 1);
-    }
-    double scaled;
-    if (recalc) {
-        float dcur;
-        if (q.adesc) {
-            float4 v[4];
-            pt_desc_load(q.adesc + (size_t) p * q.ds4, 4 * q.ds4, v);
-            dcur = pt_desc_dist(v, q.bdesc + ((size_t) ys * q.bew + xs) * q.ds4, q.nd);
-        } else {
-            dcur = ssd_global(q, a, x, y, B, xs, ys);
+template<bool DESC>
+__global__ void __launch_bounds__(TILE_DEFAULT)
+k_init_temporal(const QPlan q, const double *__restrict__ prev, const float *__restrict__ scale_sv, int recalc,
+                int sanitize, double temporal_scale, const float *__restrict__ a, int *cur_pos, float *cur_d, double *orig,
+                int *bad) {
+    constexpr int TP = TILE_DEFAULT;
+    __shared__ float at[atile_bytes(TP) / sizeof(float)];
+    const int x0 = blockIdx.x * cta_w(TP, DESC), y0 = blockIdx.y * cta_h(TP, DESC);
+    if constexpr (!DESC) {
+        if (recalc) {
+            stage_a<TP>(at, a, q.aw, q.ah, x0, y0);
+            __syncthreads();
         }
-        scaled = (double) dcur * (scale_sv ? (double) scale_sv[p] : temporal_scale);
-    } else {
+    }
+    AQuery aq;
+    int x, y;
+    tile_lane<TP, DESC>(q, at, x0, y0, x, y, aq);
+    const bool live = x < q.ew && y < q.eh;
+    const int p = live ? y * q.ew + x : 0;
+    int xs = 0, ys = 0;
+    if (live) {
+        xs = (int) prev[3 * (size_t) p];
+        ys = (int) prev[3 * (size_t) p + 1];
+        if (xs < 0 || ys < 0 || xs >= q.bew || ys >= q.beh) {
+            if (!sanitize) atomicExch(bad, 1);
+            xs = min(max(xs, 0), q.bew - 1);
+            ys = min(max(ys, 0), q.beh - 1);
+        }
+    }
+    double scaled = 0.0;
+    if (recalc) {
+        if constexpr (DESC) pt_desc_load(q.adesc + (size_t) p * q.ds4, 4 * q.ds4, aq.v);
+        unsigned rows = 0;
+        const float dcur = dist32<TP, DESC, false>(aq, q, pt_xy(xs, ys), live, finf(), rows);
+        if (live) scaled = (double) dcur * (scale_sv ? (double) scale_sv[p] : temporal_scale);
+    } else if (live) {
         scaled = prev[3 * (size_t) p + 2] * temporal_scale;
     }
+    if (!live) return;
     cur_pos[p] = pt_xy(xs, ys);
     cur_d[p] = (float) scaled;
     orig[p] = scaled / temporal_scale;
@@ -747,23 +861,29 @@ __global__ void k_init_temporal(const QPlan q, const double *__restrict__ prev, 
 
 /* init_random (patchtable.h:3522-3537): a random match per patch with its distance; the match
    comes from a hash of the patch index instead of two rand() calls. */
-__global__ void k_init_random(const QPlan q, const float4 *__restrict__ a, const float4 *__restrict__ B, int *cur_pos,
-                              float *cur_d) {
-    const int p = blockIdx.x * NT + threadIdx.x;
-    if (p >= q.ew * q.eh) return;
-    const int x = p % q.ew, y = p / q.ew;
+template<bool DESC>
+__global__ void __launch_bounds__(TILE_DEFAULT)
+k_init_random(const QPlan q, const float *__restrict__ a, int *cur_pos, float *cur_d) {
+    constexpr int TP = TILE_DEFAULT;
+    __shared__ float at[atile_bytes(TP) / sizeof(float)];
+    const int x0 = blockIdx.x * cta_w(TP, DESC), y0 = blockIdx.y * cta_h(TP, DESC);
+    if constexpr (!DESC) {
+        stage_a<TP>(at, a, q.aw, q.ah, x0, y0);
+        __syncthreads();
+    }
+    AQuery aq;
+    int x, y;
+    tile_lane<TP, DESC>(q, at, x0, y0, x, y, aq);
+    const bool live = x < q.ew && y < q.eh;
+    const int p = live ? y * q.ew + x : 0;
     unsigned hsh = mix32((unsigned) p * 0x9e3779b1u + 0x85ebca6bu);
     const int xs = (int) (hsh % (unsigned) q.bew);
     hsh = mix32(hsh ^ 0x27d4eb2fu);
     const int ys = (int) (hsh % (unsigned) q.beh);
-    float d;
-    if (q.adesc) {
-        float4 v[4];
-        pt_desc_load(q.adesc + (size_t) p * q.ds4, 4 * q.ds4, v);
-        d = pt_desc_dist(v, q.bdesc + ((size_t) ys * q.bew + xs) * q.ds4, q.nd);
-    } else {
-        d = ssd_global(q, a, x, y, B, xs, ys);
-    }
+    if constexpr (DESC) pt_desc_load(q.adesc + (size_t) p * q.ds4, 4 * q.ds4, aq.v);
+    unsigned rows = 0;
+    const float d = dist32<TP, DESC, false>(aq, q, pt_xy(xs, ys), live, finf(), rows);
+    if (!live) return;
     cur_pos[p] = pt_xy(xs, ys);
     cur_d[p] = d;
 }
@@ -822,6 +942,11 @@ bool one_pull(const QPlan &q) { return g_lean_kernels.load(std::memory_order_rel
 
 extern "C" int pt_set_lean_kernels(int on) { return g_lean_kernels.exchange(on ? 1 : 0); }
 
+static dim3 tile_grid(const QPlan &q, int tp) {
+    const int w = cta_w(tp, q.adesc != nullptr), h = cta_h(tp, q.adesc != nullptr);
+    return dim3((q.ew + w - 1) / w, (q.rows + h - 1) / h);
+}
+
 static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     memset(&q, 0, sizeof(q));
     q.aw = s.aw; q.ah = s.ah; q.ew = s.aw - 7; q.eh = s.ah - 7;
@@ -835,14 +960,15 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     q.do_kcoh = s.kcoherence > 0;
     q.step = s.step < 1 ? 1 : s.step;
     q.pull_max = s.pull_max > 0 ? s.pull_max : 1 << 30;
-    q.tile = s.tile > 0 ? s.tile : TWD;
+    q.tile = s.tile > 0 ? s.tile : TILE_DEFAULT;
     q.row0 = s.rows > 0 ? s.row0 : 0;
     q.rows = s.rows > 0 ? s.rows : q.eh;
     if (s.rows > 0 && (q.row0 < 0 || q.row0 + q.rows > q.eh))
         return pt_fail(PT_BAD_ARG, "query rows [%d, %d) outside 0..%d", q.row0, q.row0 + q.rows, q.eh);
     if (q.tile != 32 && q.tile != 64 && q.tile != 128 && q.tile != 256)
         return pt_fail(PT_BAD_ARG, "gpu_tile %d: query patches per CTA must be 32, 64, 128 or 256", s.tile);
-    q.b1 = s.b1;
+    q.brow = s.brow;
+    q.nline = pt_row_lines(s.bw);
     q.allowed = s.allowed;
     q.allowed_index = s.allowed_index;
     q.adesc = reinterpret_cast<const float4 *>(s.adesc);
@@ -858,10 +984,21 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     if (q.adesc) {
         if (!q.bdesc || (s.ds != 8 && s.ds != 16) || q.nd < 3 || q.nd > s.ds)
             return pt_fail(PT_BAD_ARG, "descriptor query: store of %d floats for %d dimensions", s.ds, q.nd);
-    } else if (!q.b1) {
-        return pt_fail(PT_BAD_ARG, "query without the shifted copy of the table image");
+    } else if (!q.brow) {
+        return pt_fail(PT_BAD_ARG, "query without the row store of the table image");
     }
     if (q.radius > 2) return pt_fail(PT_UNSUPPORTED, "propagation radius %d > 2 on the GPU path", q.radius);
+    return PT_OK;
+}
+
+int pt_row_lines(int bw) { return (bw - 7 + 1) / 2; }       /* lines of patch columns 0 .. bw - 8 */
+
+size_t pt_row_store_floats(int bw, int bh) { return (size_t) pt_row_lines(bw) * bh * 32; }
+
+pt_status pt_launch_row_store(const float4 *b, int bw, int bh, float *out, cudaStream_t st) {
+    const long long n = (long long) pt_row_store_floats(bw, bh);
+    k_row_store<<<(unsigned) ((n + NT - 1) / NT), NT, 0, st>>>(b, bw, bh, pt_row_lines(bw), out);
+    PT_LAUNCHED();
     return PT_OK;
 }
 
@@ -871,7 +1008,7 @@ pt_status pt_launch_init(int n, int pos, float d, int *cur_pos, float *cur_d, cu
     return PT_OK;
 }
 
-pt_status pt_launch_choose(const QuerySetup &s, int n, const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+pt_status pt_launch_choose(const QuerySetup &s, int n, const float *a, const int *cur_pos, const float *cur_d,
                            const int *tcand, const int2 *kcoh, int do_table, int *ch_pos,
                            float *ch_d, int *kc_done, int use_done, unsigned long long *evals, cudaStream_t st) {
     QPlan q;
@@ -880,18 +1017,17 @@ pt_status pt_launch_choose(const QuerySetup &s, int n, const float4 *a, const fl
     LearnedArgs none;
     memset(&none, 0, sizeof(none));
     if (q.adesc) {                       /* descriptor mode: one tile width, nothing staged */
-        constexpr int T = TWD_DESC;
-        dim3 grid((q.ew + T - 1) / T, q.rows);
-        k_choose_tile<T, false, true><<<grid, T, 0, st>>>(q, a, b, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d,
-                                                          kc_done, use_done, evals, none);
+        constexpr int T = TILE_DESC;
+        const dim3 grid = tile_grid(q, T);
+        k_choose_desc<<<grid, T, 0, st>>>(q, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals);
         PT_LAUNCHED();
         return PT_OK;
     }
-#define PT_CHOOSE_T(T) { dim3 grid((q.ew + T - 1) / T, q.rows); \
-        if (lean) k_choose_tile<T, false, false, true><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, b, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); \
-        else k_choose_tile<T, false, false><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, b, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); }
+#define PT_CHOOSE_T(T) { const dim3 grid = tile_grid(q, T); \
+        if (lean) k_choose_tile<T, false, true><<<grid, T, atile_bytes(T), st>>>( \
+            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); \
+        else k_choose_tile<T, false><<<grid, T, atile_bytes(T), st>>>( \
+            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); }
     const bool lean = lean_choose(q);
     switch (q.tile) {
         case 32: PT_CHOOSE_T(32) break;
@@ -904,7 +1040,7 @@ pt_status pt_launch_choose(const QuerySetup &s, int n, const float4 *a, const fl
     return PT_OK;
 }
 
-pt_status pt_launch_choose_learned(const QuerySetup &s, const float4 *a, const float4 *b, const int *cur_pos,
+pt_status pt_launch_choose_learned(const QuerySetup &s, const float *a, const int *cur_pos,
                                    const float *cur_d, const int *tcand, const int2 *kcoh, int do_table, int *ch_pos,
                                    float *ch_d, int *kc_done, int use_done, const int *lcand, const float *lconf,
                                    float threshold, int kcoh_confident, unsigned long long *evals,
@@ -919,8 +1055,8 @@ pt_status pt_launch_choose_learned(const QuerySetup &s, const float4 *a, const f
     la.threshold = threshold;
     la.kcoh_confident = kcoh_confident;
     la.counters = lcounters;
-#define PT_CHOOSE_L(T) { dim3 grid((q.ew + T - 1) / T, q.rows); \
-        k_choose_tile<T, true, false><<<grid, T, atile_bytes(T), st>>>(q, a, b, cur_pos, cur_d, tcand, kcoh, \
+#define PT_CHOOSE_L(T) { const dim3 grid = tile_grid(q, T); \
+        k_choose_tile<T, true><<<grid, T, atile_bytes(T), st>>>(q, a, cur_pos, cur_d, tcand, kcoh, \
                                                                                    do_table, ch_pos, ch_d, kc_done, use_done, \
                                                                                    evals, la); }
     switch (q.tile) {
@@ -934,7 +1070,7 @@ pt_status pt_launch_choose_learned(const QuerySetup &s, const float4 *a, const f
     return PT_OK;
 }
 
-pt_status pt_launch_pull(const QuerySetup &s, int n, const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *cur_pos, const float *cur_d,
                          const int *ch_pos, const float *ch_d, int *nxt_pos, float *nxt_d,
                          unsigned long long *evals, cudaStream_t st) {
     QPlan q;
@@ -942,18 +1078,18 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float4 *a, const floa
     (void) n;
     const bool r1 = q.radius <= 1;
     if (q.adesc) {
-        constexpr int T = TWD_DESC;
-        dim3 grid((q.ew + T - 1) / T, q.rows);
-        if (r1) k_pull_tile<T, 1, true><<<grid, T, 0, st>>>(q, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
-        else k_pull_tile<T, 2, true><<<grid, T, 0, st>>>(q, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+        constexpr int T = TILE_DESC;
+        const dim3 grid = tile_grid(q, T);
+        if (r1) k_pull_tile<T, 1, true><<<grid, T, 0, st>>>(q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+        else k_pull_tile<T, 2, true><<<grid, T, 0, st>>>(q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
         PT_LAUNCHED();
         return PT_OK;
     }
-#define PT_PULL_T(T, RR) { dim3 grid((q.ew + T - 1) / T, q.rows); \
+#define PT_PULL_T(T, RR) { const dim3 grid = tile_grid(q, T); \
         if (one) k_pull_tile<T, RR, false, true><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
         else k_pull_tile<T, RR, false><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); }
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); }
     const bool one = one_pull(q);
     switch (q.tile) {
         case 32: if (r1) PT_PULL_T(32, 1) else PT_PULL_T(32, 2) break;
@@ -1003,8 +1139,13 @@ int persistent_grid(K kernel, int threads, size_t smem, long long work) {
 
 int pt_batch_tw(int twi) { return (twi >= 0 && twi < PT_BATCH_NTW) ? BATCH_TW[twi] : 0; }
 
+long long pt_batch_tiles(int twi, int ew, int eh) {
+    const int tp = pt_batch_tw(twi);
+    return (long long) ((ew + tile_w(tp) - 1) / tile_w(tp)) * ((eh + tile_h(tp) - 1) / tile_h(tp));
+}
+
 pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
-                                 const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+                                 const float *a, const int *cur_pos, const float *cur_d,
                                  const int *tcand, const int2 *kcoh, int do_table, int *ch_pos, float *ch_d, int *kc_done,
                                  int use_done, unsigned long long *evals, unsigned long long *work, cudaStream_t st) {
     QPlan q;
@@ -1013,10 +1154,10 @@ pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, 
     PT_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), st));
 #define PT_CHOOSE_B(T) { const size_t sm = atile_bytes(T); \
         if (lean) { const int g = persistent_grid(k_choose_batch<T, true>, T, sm, nseg); \
-            k_choose_batch<T, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, b, cur_pos, cur_d, tcand, kcoh, do_table, \
+            k_choose_batch<T, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, tcand, kcoh, do_table, \
                                                       ch_pos, ch_d, kc_done, use_done, evals, work); } \
         else { const int g = persistent_grid(k_choose_batch<T>, T, sm, nseg); \
-            k_choose_batch<T><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, b, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, \
+            k_choose_batch<T><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, \
                                                 ch_d, kc_done, use_done, evals, work); } }
     const bool lean = lean_choose(q);
     switch (BATCH_TW[twi]) {
@@ -1031,7 +1172,7 @@ pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, 
 }
 
 pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
-                               const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d, const int *ch_pos,
+                               const float *a, const int *cur_pos, const float *cur_d, const int *ch_pos,
                                const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *evals,
                                unsigned long long *work, cudaStream_t st) {
     QPlan q;
@@ -1040,10 +1181,10 @@ pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, in
     PT_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), st));
 #define PT_PULL_B(T, RR) { const size_t sm = atile_bytes(T); \
         if (one) { const int g = persistent_grid(k_pull_batch<T, RR, true>, T, sm, nseg); \
-            k_pull_batch<T, RR, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, \
+            k_pull_batch<T, RR, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, \
                                                         nxt_d, evals, work); } \
         else { const int g = persistent_grid(k_pull_batch<T, RR>, T, sm, nseg); \
-            k_pull_batch<T, RR><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, b, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, \
+            k_pull_batch<T, RR><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, \
                                                   evals, work); } }
     const bool one = one_pull(q);
     const bool r1 = q.radius <= 1;
@@ -1059,13 +1200,17 @@ pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, in
 }
 
 pt_status pt_launch_init_temporal(const QuerySetup &s, const double *prev, const float *scale_sv, int recalc, int sanitize,
-                                  double temporal_scale, const float4 *a, const float4 *b, int *cur_pos, float *cur_d,
+                                  double temporal_scale, const float *a, int *cur_pos, float *cur_d,
                                   double *orig, int *bad, cudaStream_t st) {
     QPlan q;
     PT_TRY(make_qplan(s, q));
-    const int n = q.ew * q.eh;
-    k_init_temporal<<<(n + NT - 1) / NT, NT, 0, st>>>(q, prev, scale_sv, recalc, sanitize, temporal_scale, a, b, cur_pos, cur_d,
-                                                     orig, bad);
+    const dim3 grid = tile_grid(q, TILE_DEFAULT);
+    if (q.adesc)
+        k_init_temporal<true><<<grid, TILE_DEFAULT, 0, st>>>(q, prev, scale_sv, recalc, sanitize, temporal_scale, a, cur_pos,
+                                                             cur_d, orig, bad);
+    else
+        k_init_temporal<false><<<grid, TILE_DEFAULT, 0, st>>>(q, prev, scale_sv, recalc, sanitize, temporal_scale, a, cur_pos,
+                                                              cur_d, orig, bad);
     PT_LAUNCHED();
     return PT_OK;
 }
@@ -1077,12 +1222,13 @@ pt_status pt_launch_output_temporal(int n, const int *pos, const float *d, const
     return PT_OK;
 }
 
-pt_status pt_launch_init_random(const QuerySetup &s, const float4 *a, const float4 *b, int *cur_pos, float *cur_d,
+pt_status pt_launch_init_random(const QuerySetup &s, const float *a, int *cur_pos, float *cur_d,
                                 cudaStream_t st) {
     QPlan q;
     PT_TRY(make_qplan(s, q));
-    const int n = q.ew * q.eh;
-    k_init_random<<<(n + NT - 1) / NT, NT, 0, st>>>(q, a, b, cur_pos, cur_d);
+    const dim3 grid = tile_grid(q, TILE_DEFAULT);
+    if (q.adesc) k_init_random<true><<<grid, TILE_DEFAULT, 0, st>>>(q, a, cur_pos, cur_d);
+    else k_init_random<false><<<grid, TILE_DEFAULT, 0, st>>>(q, a, cur_pos, cur_d);
     PT_LAUNCHED();
     return PT_OK;
 }

@@ -1,14 +1,14 @@
 /* Batched queries: many query images of any sizes against one table, in one pass of launches.
 
    The reference matches one image per lookup() call (patchtable/patchtable.h:4448).  A batch
-   concatenates its images -- RGB pixels, RGBA copies, table entries, query state and the float64
+   concatenates its images -- RGB pixels, table entries, query state and the float64
    NNF -- and runs every phase of the query once for all of them: one descriptor launch over the
    flattened list of 64 x 8 descriptor tiles that also looks each patch's cell up in the table,
-   and per propagation pass one choose and one pull launch over the flattened list of row segments
+   and per propagation pass one choose and one pull launch over the flattened list of patch tiles
    (the first pass starts from the initial field, the last pull writes the NNF).  The choose /
    pull / descriptor launches are persistent (as many CTAs as fit on the GPU); a work counter per
-   launch hands the segments out one at a time to whichever CTA is free, and each CTA finds the
-   image that owns its segment by binary search over per-image prefix counts.  Every patch is computed exactly as the
+   launch hands the tiles out one at a time to whichever CTA is free, and each CTA finds the
+   image that owns its tile by binary search over per-image prefix counts.  Every patch is computed exactly as the
    single-image query computes it, so each image's NNF equals its own pt_table_lookup_device
    result.
 
@@ -30,7 +30,7 @@ struct pt_batch {
     DevBuf<PtBatchImage> d_imgs;
     long long npix = 0, P = 0, ntiles = 0, nseg[PT_BATCH_NTW] = {0, 0, 0, 0};
     int twi = PT_BATCH_NTW - 1;           /* 256 query patches per CTA until tuned */
-    DevBuf<float4> rgba;
+    DevBuf<float> rgb;                    /* copy of a query buffer that shares memory with the NNF */
     DevBuf<int> tcand, pos[2], chpos, kcdone;
     DevBuf<float> dd[2], chd;
     DevBuf<unsigned long long> work;      /* work counters of the persistent launches */
@@ -52,11 +52,16 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     PtTableView v;
     PT_TRY(pt_table_view(B->t, &v));
     const pt_params &p = v.p;
-    const int ds = v.ds;
-    (void) ds;
+    /* the distance kernels read the images themselves: a buffer that shares memory with the NNF is copied */
+    const size_t rgb_bytes = sizeof(float) * 3 * (size_t) B->npix;
+    if (pt_overlap(d_rgb, rgb_bytes, d_ann, sizeof(double) * 3 * (size_t) B->P)) {
+        PT_CUDA(B->rgb.reserve(3 * (size_t) B->npix));
+        PT_CUDA(cudaMemcpyAsync(B->rgb.p, d_rgb, rgb_bytes, cudaMemcpyDeviceToDevice, st));
+        d_rgb = B->rgb.p;
+    }
     /* descriptors are needed only for the table step: one fused pass writes the table entries */
     PT_TRY(pt_launch_descriptor_cells_batch(p.ndims, p.nchroma, B->d_imgs.p, B->n, B->ntiles, d_rgb, pt_color_mode(p),
-                                            B->rgba.p, v.bins, v.to_bin, v.table, B->tcand.p, B->work.p, st));
+                                            nullptr, v.bins, v.to_bin, v.table, B->tcand.p, B->work.p, st));
     QuerySetup qs;
     qs.aw = 0; qs.ah = 0; qs.bw = v.w; qs.bh = v.h;
     qs.prop_scale = 1.0 / (1 + p.coherence_spatial);
@@ -67,7 +72,7 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     qs.spatial = p.spatial;
     qs.do_rs = p.do_rs;
     qs.radius = std::min(2, p.query_step + p.prop_dist);
-    qs.b1 = v.b_rgba1;
+    qs.brow = v.b_row;
     qs.pull_max = p.gpu_pull_max;
     qs.allowed = v.allowed;
     qs.allowed_index = p.allowed_index;
@@ -85,14 +90,14 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
         qi.pass = i;
         if (!pt_pass_kcoh(p, i, passes)) qi.kcoherence = 0;
         const int use_done = i > 0 && pt_pass_kcoh(p, i - 1, passes);
-        PT_TRY(pt_launch_choose_batch(qi, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, B->rgba.p, v.b_rgba,
+        PT_TRY(pt_launch_choose_batch(qi, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
                                       i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->tcand.p, v.kcoh,
                                       do_table, B->chpos.p, B->chd.p, B->kcdone.p, use_done, nullptr, B->work.p + 1, st));
         if (p.do_prop) {
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
             if (i == passes - 1 && direct_out) qp.ann = d_ann;
-            PT_TRY(pt_launch_pull_batch(qp, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, B->rgba.p, v.b_rgba,
+            PT_TRY(pt_launch_pull_batch(qp, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
                                         i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->chpos.p, B->chd.p,
                                         B->pos[1 - cur].p, B->dd[1 - cur].p, nullptr, B->work.p + 2, st));
             cur = 1 - cur;
@@ -133,8 +138,7 @@ pt_status pt_batch_create(pt_table *t, int n, const int *h, const int *w, pt_bat
         g.tile_off = tiles;
         for (int k = 0; k < PT_BATCH_NTW; k++) {
             g.seg_off[k] = seg[k];
-            const int tw = pt_batch_tw(k);
-            seg[k] += (long long) g.eh * ((g.ew + tw - 1) / tw);
+            seg[k] += pt_batch_tiles(k, g.ew, g.eh);
         }
         pix += (long long) h[i] * w[i];
         pat += (long long) g.eh * g.ew;
@@ -149,7 +153,7 @@ pt_status pt_batch_create(pt_table *t, int n, const int *h, const int *w, pt_bat
     B->ntiles = tiles;
     for (int k = 0; k < PT_BATCH_NTW; k++) B->nseg[k] = seg[k];
     auto fail = [&](pt_status s) { delete B; return s; };
-    if (B->d_imgs.reserve(n) || B->rgba.reserve(pix) || B->tcand.reserve(pat) ||
+    if (B->d_imgs.reserve(n) || B->tcand.reserve(pat) ||
         B->pos[0].reserve(pat) || B->pos[1].reserve(pat) || B->dd[0].reserve(pat) || B->dd[1].reserve(pat) ||
         B->chpos.reserve(pat) || B->chd.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
         return fail(pt_fail(PT_OOM, "batch buffers for %lld pixels / %lld patches", pix, pat));

@@ -28,6 +28,12 @@ PT_HD int pt_xy(int x, int y) { return x | (y << 16); }
 PT_HD int pt_x(int v) { return v & 65535; }
 PT_HD int pt_y(int v) { return v >> 16; }
 
+/* Whether two memory ranges share a byte. */
+inline bool pt_overlap(const void *a, size_t na, const void *b, size_t nb) {
+    const uintptr_t x = (uintptr_t) a, y = (uintptr_t) b;
+    return x < y + nb && y < x + na;
+}
+
 /* Records an error message for pt_last_error() and returns the status. */
 pt_status pt_fail(pt_status s, const char *fmt, ...);
 /* Counts device kernel launches issued by the library (pt_kernel_launch_count). */

@@ -120,9 +120,9 @@ struct QuerySetup {
     int kc_try = 0;          /* k-coherence neighbours tried per patch (0 = all kcoherence) */
     int step = 1;            /* neighbour spacing of a pull pass */
     int pull_max = 0;        /* most neighbour candidates a pull scores per patch (0 = all) */
-    int tile = 0;            /* query patches per CTA in choose / pull: 32, 64, 128, 256 (0 = 32) */
+    int tile = 0;            /* query patches per CTA in choose / pull: 32, 64, 128, 256 (0 = 64) */
     int row0 = 0, rows = 0;  /* patch rows [row0, row0 + rows) of a single-image launch (rows 0 = all) */
-    const float4 *b1 = nullptr;   /* the table image shifted by one pixel, b1[i] = b[i + 1] */
+    const float *brow = nullptr;  /* row store of the table image (pt_launch_row_store) */
     const int *allowed = nullptr; /* b patches a match may use (allowed[p] == allowed_index), or NULL */
     int allowed_index = 0;
     /* Descriptor mode (is_descriptor): distances are patch_dist_approx between the query's and the
@@ -172,19 +172,24 @@ inline int pt_pass_step(int i, int n, int jump) {
     for (int k = 0; k < i && s > 1; k++) s /= 2;
     return s;
 }
+/* The row store the distance kernels read the table image from: its lines per image row, its
+   floats, and the kernel that writes it from the RGBA image. */
+int pt_row_lines(int bw);
+size_t pt_row_store_floats(int bw, int bh);
+pt_status pt_launch_row_store(const float4 *b, int bw, int bh, float *out, cudaStream_t st);
 pt_status pt_launch_init(int n, int pos, float d, int *cur_pos, float *cur_d, cudaStream_t st);
-pt_status pt_launch_choose(const QuerySetup &s, int n, const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+pt_status pt_launch_choose(const QuerySetup &s, int n, const float *a, const int *cur_pos, const float *cur_d,
                            const int *tcand, const int2 *kcoh, int do_table, int *ch_pos,
                            float *ch_d, int *kc_done, int use_done, unsigned long long *evals, cudaStream_t st);
 /* choose with the learned network's proposals (k_proposal.cu) for patches with lconf >= threshold;
    lcand (n x PT_PROP_TOPK table entries) may be NULL on passes without proposals; lcounters
    (may be NULL) accumulates {confident patches, proposals scored}. */
-pt_status pt_launch_choose_learned(const QuerySetup &s, const float4 *a, const float4 *b, const int *cur_pos,
+pt_status pt_launch_choose_learned(const QuerySetup &s, const float *a, const int *cur_pos,
                                    const float *cur_d, const int *tcand, const int2 *kcoh, int do_table, int *ch_pos,
                                    float *ch_d, int *kc_done, int use_done, const int *lcand, const float *lconf,
                                    float threshold, int kcoh_confident, unsigned long long *evals,
                                    unsigned long long *lcounters, cudaStream_t st);
-pt_status pt_launch_pull(const QuerySetup &s, int n, const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *cur_pos, const float *cur_d,
                          const int *ch_pos, const float *ch_d, int *nxt_pos, float *nxt_d,
                          unsigned long long *evals, cudaStream_t st);
 /* Packed positions and float distances of a float64 NNF whose distances are float values. */
@@ -194,17 +199,17 @@ pt_status pt_launch_output(int n, const int *pos, const float *d, double *ann, c
    unscaled distance (patchtable.h:3548-3585, 4178-4193); *bad becomes 1 when a previous match lies
    outside the table image and sanitize is off. */
 /* init_random: a hashed random match and its distance per patch. */
-pt_status pt_launch_init_random(const QuerySetup &s, const float4 *a, const float4 *b, int *cur_pos, float *cur_d,
+pt_status pt_launch_init_random(const QuerySetup &s, const float *a, int *cur_pos, float *cur_d,
                                 cudaStream_t st);
 pt_status pt_launch_init_temporal(const QuerySetup &s, const double *prev, const float *scale_sv, int recalc, int sanitize,
-                                  double temporal_scale, const float4 *a, const float4 *b, int *cur_pos, float *cur_d,
+                                  double temporal_scale, const float *a, int *cur_pos, float *cur_d,
                                   double *orig, int *bad, cudaStream_t st);
 pt_status pt_launch_output_temporal(int n, const int *pos, const float *d, const int *pos0, const float *d0,
                                     const double *orig, double *ann, cudaStream_t st);
 
 /* Batched queries (pt_batch.cu): the images of a batch are concatenated -- pixels, patches and
-   query state -- and every phase is one persistent launch over the flattened list of row
-   segments, handed out one at a time through a work counter (`work`, zeroed by the launcher).  seg_off[t] is the image's first segment when a CTA covers PT_BATCH_TW(t) patches. */
+   query state -- and every phase is one persistent launch over the flattened list of
+   patch tiles, handed out one at a time through a work counter (`work`, zeroed by the launcher).  seg_off[t] is the image's first tile when a CTA covers pt_batch_tw(t) patches. */
 #define PT_BATCH_NTW 4
 struct PtBatchImage {
     int h, w, eh, ew;
@@ -213,12 +218,14 @@ struct PtBatchImage {
     long long tile_off;                  /* first 64 x 8 descriptor tile */
 };
 int pt_batch_tw(int twi);
+/* CTA tiles of an image of ew x eh patches at that width. */
+long long pt_batch_tiles(int twi, int ew, int eh);
 pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
-                                 const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d,
+                                 const float *a, const int *cur_pos, const float *cur_d,
                                  const int *tcand, const int2 *kcoh, int do_table, int *ch_pos, float *ch_d, int *kc_done,
                                  int use_done, unsigned long long *evals, unsigned long long *work, cudaStream_t st);
 pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
-                               const float4 *a, const float4 *b, const int *cur_pos, const float *cur_d, const int *ch_pos,
+                               const float *a, const int *cur_pos, const float *cur_d, const int *ch_pos,
                                const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *evals,
                                unsigned long long *work, cudaStream_t st);
 /* The batch's descriptor pass fused with the table step: tcand[p] = table[cell(p)] for every
@@ -231,8 +238,7 @@ pt_status pt_launch_descriptor_cells_batch(int ndims, int nchroma, const PtBatch
 struct PtTableView {
     pt_params p;
     int h, w, ds;
-    const float4 *b_rgba;
-    const float4 *b_rgba1;               /* b_rgba shifted by one pixel (32-byte aligned row loads) */
+    const float *b_row;                  /* row store of the table image */
     const int *table;
     const int *to_bin;
     const int2 *kcoh;

@@ -11,7 +11,7 @@
    Limits and behaviour:
      * query images of at most PT_NOALLOC_MAX_PIXELS (262144) pixels, e.g. 512 x 512, and tables
        with ndims <= 8; larger requests fail with PT_BAD_ARG / PT_UNSUPPORTED;
-     * the array costs 20 MiB of device memory on every GPU that loads the library, held until
+     * the array costs 19 MiB of device memory on every GPU that loads the library, held until
        the process exits;
      * all calls share the array: calls that overlap on the GPU (different streams, threads or
        tables at the same time) race on it and must be serialised by the caller;
@@ -30,9 +30,9 @@
 namespace {
 
 constexpr size_t kMaxPixels = PT_NOALLOC_MAX_PIXELS;
-/* per pixel: RGBA copy (16 B) + descriptor record (32 B) + table candidate (4 B)
-   + four position buffers (16 B) + three distance buffers (12 B) */
-constexpr size_t kBytesPerPixel = 16 + 32 + 4 + 16 + 12;
+/* per pixel: descriptor record (32 B) + table candidate (4 B) + four position buffers (16 B)
+   + three distance buffers (12 B) + copy of a query image that shares memory with the NNF (12 B) */
+constexpr size_t kBytesPerPixel = 32 + 4 + 16 + 12 + 12;
 constexpr size_t kScratchBytes = kMaxPixels * kBytesPerPixel;
 
 static __device__ __align__(256) unsigned char pt_noalloc_scratch[kScratchBytes];
@@ -76,7 +76,6 @@ extern "C" pt_status pt_table_lookup_device_noalloc(pt_table *t, const float *d_
     const pt_params &p = v.p;
     const size_t N = kMaxPixels;
     unsigned char *s = (unsigned char *) base;
-    float4 *rgba = (float4 *) s;            s += N * 16;
     float *desc = (float *) s;              s += N * 32;
     int *tcand = (int *) s;                 s += N * 4;
     int *pos0 = (int *) s;                  s += N * 4;
@@ -85,13 +84,19 @@ extern "C" pt_status pt_table_lookup_device_noalloc(pt_table *t, const float *d_
     int *kcdone = (int *) s;                s += N * 4;
     float *d0 = (float *) s;                s += N * 4;
     float *d1 = (float *) s;                s += N * 4;
-    float *chd = (float *) s;
+    float *chd = (float *) s;               s += N * 4;
+    float *rgb = (float *) s;
     int *pos[2] = {pos0, pos1};
     float *dd[2] = {d0, d1};
 
     long long P = (long long) (h - 7) * (w - 7);
     int n = (int) P;
-    PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, d_a, h, w, pt_color_mode(p), rgba, desc, 8, st));
+    const size_t rgb_bytes = sizeof(float) * 3 * (size_t) h * w;
+    if (pt_overlap(d_a, rgb_bytes, d_ann, sizeof(double) * 3 * (size_t) P)) {
+        PT_CUDA(cudaMemcpyAsync(rgb, d_a, rgb_bytes, cudaMemcpyDeviceToDevice, st));
+        d_a = rgb;
+    }
+    PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, d_a, h, w, pt_color_mode(p), nullptr, desc, 8, st));
     PT_TRY(pt_launch_table_candidates(v.bins, desc, 8, P, v.to_bin, v.table, tcand, st));
     QuerySetup qs;
     qs.aw = w; qs.ah = h; qs.bw = v.w; qs.bh = v.h;
@@ -104,7 +109,7 @@ extern "C" pt_status pt_table_lookup_device_noalloc(pt_table *t, const float *d_
     qs.do_rs = p.do_rs;
     qs.radius = p.query_step + p.prop_dist;
     if (qs.radius > 2) qs.radius = 2;
-    qs.b1 = v.b_rgba1;
+    qs.brow = v.b_row;
     qs.pull_max = p.gpu_pull_max;
     qs.tile = p.gpu_tile;
     qs.allowed = v.allowed;
@@ -120,12 +125,12 @@ extern "C" pt_status pt_table_lookup_device_noalloc(pt_table *t, const float *d_
         qi.pass = i;
         if (!pt_pass_kcoh(p, i, passes)) qi.kcoherence = 0;
         const int use_done = i > 0 && pt_pass_kcoh(p, i - 1, passes);
-        PT_TRY(pt_launch_choose(qi, n, rgba, v.b_rgba, pos[cur], dd[cur], tcand, v.kcoh, do_table, chpos, chd,
+        PT_TRY(pt_launch_choose(qi, n, d_a, pos[cur], dd[cur], tcand, v.kcoh, do_table, chpos, chd,
                                 kcdone, use_done, nullptr, st));
         if (p.do_prop) {
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
-            PT_TRY(pt_launch_pull(qp, n, rgba, v.b_rgba, pos[cur], dd[cur], chpos, chd, pos[1 - cur], dd[1 - cur],
+            PT_TRY(pt_launch_pull(qp, n, d_a, pos[cur], dd[cur], chpos, chd, pos[1 - cur], dd[1 - cur],
                                   nullptr, st));
             cur = 1 - cur;
         } else {

@@ -113,7 +113,7 @@ struct pt_table {
     bool own_stream = false;
     cudaStream_t st2 = nullptr;       /* the build's second stream (range and partition) */
     DevBuf<float4> b_rgba;
-    DevBuf<float4> b_rgba1;           /* b_rgba shifted by one pixel, b_rgba1[i] = b_rgba[i + 1] */
+    DevBuf<float> b_row;              /* row store of b the query's distances read (pt_launch_row_store) */
     DevBuf<float> b_desc;
     DevBuf<int> allowed;
     std::vector<int> nslices;
@@ -138,7 +138,6 @@ struct pt_table {
     DevBuf<int> q_tcand_more;
     /* query scratch, reused across lookups (like lookup_buffer/lookup_wh, patchtable.h:1507-1509) */
     DevBuf<float> q_rgb;
-    DevBuf<float4> q_rgba;
     DevBuf<float> q_desc;
     DevBuf<int> q_tcand;
     DevBuf<int> q_pos[2], q_chpos, q_kcdone;
@@ -464,12 +463,8 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
                         packed[((size_t) y * t->ew + x) * t->ds + d] = wh0[((size_t) (y + 7) * (w + 7) + (x + 7)) * t->nd + d];
             PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
         }
-        /* The query reads b patch rows with 32-byte loads: from b_rgba at even pixel indices and
-           from this one-pixel-shifted copy at odd ones, so every load is 32-byte aligned. */
-        const size_t npx = (size_t) h * w;
-        PT_CUDA(t->b_rgba1.reserve(npx));
-        PT_CUDA(cudaMemsetAsync(t->b_rgba1.p, 0, sizeof(float4) * npx, t->st));
-        PT_CUDA(cudaMemcpyAsync(t->b_rgba1.p, t->b_rgba.p + 1, sizeof(float4) * (npx - 1), cudaMemcpyDeviceToDevice, t->st));
+        PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
+        PT_TRY(pt_launch_row_store(t->b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     std::vector<int> allowed_h;
@@ -627,7 +622,6 @@ pt_status ensure_query_buffers(pt_table *t, int h, int w) {
     size_t in_floats;
     query_input_dims(t, h, w, ih, iw, in_floats);
     PT_CUDA(t->q_rgb.reserve(std::max((size_t) h * w * 3, in_floats)));
-    PT_CUDA(t->q_rgba.reserve((size_t) h * w));
     PT_CUDA(t->q_desc.reserve((size_t) P * t->ds));
     PT_CUDA(t->q_tcand.reserve(P));
     for (int k = 0; k < 2; k++) { PT_CUDA(t->q_pos[k].reserve(P)); PT_CUDA(t->q_d[k].reserve(P)); }
@@ -677,6 +671,12 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     if (P >= (1ll << 31)) return pt_fail(PT_BAD_ARG, "query image too large");
     int n = (int) P;
     PT_TRY(ensure_query_buffers(t, h, w));
+    /* the distance kernels read the query image itself: one that shares memory with the NNF is copied */
+    const size_t rgb_bytes = sizeof(float) * (size_t) h * w * 3;
+    if (!t->desc_mode && pt_overlap(a_rgb, rgb_bytes, d_ann, sizeof(double) * 3 * (size_t) P)) {
+        PT_CUDA(cudaMemcpyAsync(t->q_rgb.p, a_rgb, rgb_bytes, cudaMemcpyDeviceToDevice, st));
+        a_rgb = t->q_rgb.p;
+    }
     unsigned long long *ctr = prof ? t->q_counters.p : nullptr;
     if (ctr) PT_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 6, st));
     PT_TRY(mark(t, prof, -1, st));
@@ -687,16 +687,16 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
         query_input_dims(t, h, w, ih, iw, nin);
         PT_TRY(pt_launch_descriptor_input(a_rgb, ih, iw, t->nd, t->in_padded, t->q_desc.p, t->ds, st));
     } else if (t->pca) {
-        PT_TRY(pt_launch_pca(a_rgb, h, w, pt_color_mode(p), t->q_rgba.p, t->pca_mean.p, t->pca_basis.p, t->nd,
+        PT_TRY(pt_launch_pca(a_rgb, h, w, pt_color_mode(p), nullptr, t->pca_mean.p, t->pca_basis.p, t->nd,
                              t->q_desc.p, t->ds, st));
     } else if (learned || !t->subs.empty()) {
-        PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), t->q_rgba.p, t->q_desc.p,
+        PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), nullptr, t->q_desc.p,
                                     t->ds, st));
     }
     /* The plain single-table query needs its descriptors only for the table step: one fused pass. */
     const bool fused = !t->desc_mode && !t->pca && !learned && t->subs.empty();
     if (fused)
-        PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), t->q_rgba.p, t->bins,
+        PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), nullptr, t->bins,
                                           t->to_bin.p, t->table.p, t->q_tcand.p, 0, (h - 7 + 7) / 8, st));
     PT_TRY(mark(t, prof, LookupProfile::DESC, st));
     if (!fused)
@@ -728,7 +728,7 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     qs.spatial = p.spatial;
     qs.do_rs = p.do_rs;
     qs.radius = p.query_step + p.prop_dist;
-    qs.b1 = t->b_rgba1.p;
+    qs.brow = t->b_row.p;
     qs.pull_max = p.gpu_pull_max;
     qs.tile = p.gpu_tile;
     qs.allowed = t->allowed.p;
@@ -751,13 +751,13 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
         PT_CUDA(cudaMemsetAsync(t->q_tbad.p, 0, sizeof(int), st));
     }
     if (p.init_random) {                      /* takes precedence over ann_prev, patchtable.h:3522-3537 */
-        PT_TRY(pt_launch_init_random(qs, t->q_rgba.p, t->b_rgba.p, t->q_pos[0].p, t->q_d[0].p, st));
+        PT_TRY(pt_launch_init_random(qs, a_rgb, t->q_pos[0].p, t->q_d[0].p, st));
     } else if (d_prev) {
         PT_CUDA(t->q_tpos0.reserve(P));
         PT_CUDA(t->q_td0.reserve(P));
         PT_CUDA(t->q_torig.reserve(P));
         PT_TRY(pt_launch_init_temporal(qs, d_prev, d_sv, p.recalc_dist_temporal, p.sanitize_input, temporal_scale,
-                                       t->q_rgba.p, t->b_rgba.p, t->q_pos[0].p, t->q_d[0].p, t->q_torig.p, t->q_tbad.p, st));
+                                       a_rgb, t->q_pos[0].p, t->q_d[0].p, t->q_torig.p, t->q_tbad.p, st));
         PT_CUDA(cudaMemcpyAsync(t->q_tpos0.p, t->q_pos[0].p, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
         PT_CUDA(cudaMemcpyAsync(t->q_td0.p, t->q_d[0].p, sizeof(float) * n, cudaMemcpyDeviceToDevice, st));
     } else if (learned || pt_default_passes(p) == 0) {
@@ -782,14 +782,14 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
         if (!pt_pass_kcoh(p, i, passes)) qi.kcoherence = 0;
         const int use_done = i > 0 && pt_pass_kcoh(p, i - 1, passes);
         if (learned)
-            PT_TRY(pt_launch_choose_learned(qi, t->q_rgba.p, t->b_rgba.p, t->q_pos[cur].p, t->q_d[cur].p, t->q_tcand.p,
+            PT_TRY(pt_launch_choose_learned(qi, a_rgb, t->q_pos[cur].p, t->q_d[cur].p, t->q_tcand.p,
                                             t->kcoh.p, do_table, t->q_chpos.p, t->q_chd.p, t->q_kcdone.p, use_done,
                                             i == 0 ? (ext ? ext->cand : t->q_lcand.p) : nullptr,
                                             ext ? ext->conf : t->q_lconf.p, ext ? ext->threshold : pt_prop_threshold(net),
                                             ext ? ext->kcoh_confident : pt_prop_kcoh_confident(net), ctr,
                                             ctr ? ctr + 4 : nullptr, st));
         else
-            PT_TRY(pt_launch_choose(qi, n, t->q_rgba.p, t->b_rgba.p, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
+            PT_TRY(pt_launch_choose(qi, n, a_rgb, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
                                     fresh && i == 0 ? nullptr : t->q_d[cur].p, t->q_tcand.p, t->kcoh.p, do_table,
                                     t->q_chpos.p, t->q_chd.p, t->q_kcdone.p, use_done, ctr, st));
         PT_TRY(mark(t, prof, LookupProfile::CHOOSE, st));
@@ -797,7 +797,7 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
             if (i == passes - 1 && direct_out) qp.ann = d_ann;
-            PT_TRY(pt_launch_pull(qp, n, t->q_rgba.p, t->b_rgba.p, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
+            PT_TRY(pt_launch_pull(qp, n, a_rgb, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
                                   fresh && i == 0 ? nullptr : t->q_d[cur].p, t->q_chpos.p, t->q_chd.p,
                                   t->q_pos[1 - cur].p, t->q_d[1 - cur].p, ctr ? ctr + 2 : nullptr, st));
             PT_TRY(mark(t, prof, LookupProfile::PULL, st));
@@ -816,8 +816,8 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
 }
 
 /* The host lookup of a one-pass schedule, pipelined over bands of patch rows.  A band needs only
-   its own pixel rows plus 7; its choose also reads the next band's RGBA rows (written by that
-   band's descriptor launch) and its pull the next band's choices.  Four streams carry the phases:
+   its own pixel rows plus 7; its choose also reads the next band's pixel rows (uploaded before
+   that band's descriptor launch) and its pull the next band's choices.  Four streams carry the phases:
    upload of band b -> descriptor and table entries of band b (one fused pass) -> choose of band
    b-1 -> pull of band b-2 -> download of band b-2, each waiting on the events its inputs come
    from; choose and pull start from the initial field without reading state arrays.  Consecutive
@@ -912,7 +912,7 @@ pt_status enqueue_bands(pt_table *t, const BandIO &io, int h, int w, const std::
     qs.spatial = p.spatial;
     qs.do_rs = p.do_rs;
     qs.radius = std::min(2, p.query_step + p.prop_dist);
-    qs.b1 = t->b_rgba1.p;
+    qs.brow = t->b_row.p;
     qs.pull_max = p.gpu_pull_max;
     qs.tile = p.gpu_tile;
     qs.allowed = t->allowed.p;
@@ -939,7 +939,7 @@ pt_status enqueue_bands(pt_table *t, const BandIO &io, int h, int w, const std::
         if (b < nb) {
             const int r0 = edge[b], r1 = edge[b + 1];
             PT_CUDA(cudaStreamWaitEvent(sa, ev_in[b], 0));
-            PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, rgb, h, w, pt_color_mode(p), t->q_rgba.p,
+            PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, rgb, h, w, pt_color_mode(p), nullptr,
                                               t->bins, t->to_bin.p, t->table.p, t->q_tcand.p, r0 / 8, (r1 - r0 + 7) / 8, sa));
             PT_CUDA(cudaEventRecord(ev_a[b], sa));
         }
@@ -950,7 +950,7 @@ pt_status enqueue_bands(pt_table *t, const BandIO &io, int h, int w, const std::
             qc.row0 = r0;
             qc.rows = r1 - r0;
             qc.stream = sb;
-            PT_TRY(pt_launch_choose(qc, (int) P, t->q_rgba.p, t->b_rgba.p, nullptr, nullptr, t->q_tcand.p, t->kcoh.p,
+            PT_TRY(pt_launch_choose(qc, (int) P, rgb, nullptr, nullptr, t->q_tcand.p, t->kcoh.p,
                                     p.do_table_lookup, t->q_chpos.p, t->q_chd.p, t->q_kcdone.p, 0, nullptr, sb));
             PT_CUDA(cudaEventRecord(ev_b[b - 1], sb));
         }
@@ -964,7 +964,7 @@ pt_status enqueue_bands(pt_table *t, const BandIO &io, int h, int w, const std::
             /* the pull writes the band's final field: packed position and float distance, or
                (without host widening) the float64 records */
             if (!widen) qb.ann = t->q_ann.p;
-            PT_TRY(pt_launch_pull(qb, (int) P, t->q_rgba.p, t->b_rgba.p, nullptr, nullptr, t->q_chpos.p, t->q_chd.p,
+            PT_TRY(pt_launch_pull(qb, (int) P, rgb, nullptr, nullptr, t->q_chpos.p, t->q_chd.p,
                                   t->q_pos[1].p, t->q_d[1].p, nullptr, sc));
             const size_t o = (size_t) r0 * ew;
             const size_t n = (size_t) (r1 - r0) * ew;
@@ -1272,10 +1272,8 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
                     packed[((size_t) y * t->ew + x) * t->ds + d] = wh0[((size_t) (y + 7) * (w + 7) + (x + 7)) * nd + d];
         PT_CUDA(t->b_desc.reserve(packed.size()));
         PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
-        const size_t npx = (size_t) h * w;
-        PT_CUDA(t->b_rgba1.reserve(npx));
-        PT_CUDA(cudaMemsetAsync(t->b_rgba1.p, 0, sizeof(float4) * npx, t->st));
-        PT_CUDA(cudaMemcpyAsync(t->b_rgba1.p, t->b_rgba.p + 1, sizeof(float4) * (npx - 1), cudaMemcpyDeviceToDevice, t->st));
+        PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
+        PT_TRY(pt_launch_row_store(t->b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     /* the file has no k-coherence set (the reference's load leaves it empty); it is rebuilt from
@@ -1655,8 +1653,7 @@ pt_status pt_table_view(const pt_table *t, PtTableView *v) {
                                        "pt_table_lookup_device(_temporal) and the profile only");
     v->p = t->p;
     v->h = t->h; v->w = t->w; v->ds = t->ds;
-    v->b_rgba = t->b_rgba.p;
-    v->b_rgba1 = t->b_rgba1.p;
+    v->b_row = t->b_row.p;
     v->table = t->table.p;
     v->to_bin = t->to_bin.p;
     v->kcoh = t->kcoh.p;
