@@ -602,6 +602,11 @@ def device_bytes_in_use() -> int:
     return int(lib().pt_device_bytes_in_use())
 
 
+def release_memory() -> None:
+    """Gives the device and page-locked memory the library keeps for reuse back (see pt_release_memory)."""
+    _check(lib().pt_release_memory())
+
+
 def launch_count() -> int:
     return int(lib().pt_kernel_launch_count())
 

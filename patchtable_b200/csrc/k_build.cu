@@ -415,8 +415,8 @@ pt_status pt_dt_other(int *table, int G, const int *nslices, int dt_algo, cudaSt
         long long maxlines = 0;
         for (int d = 0; d < G; d++) maxlines = std::max(maxlines, s.n / nslices[d]);
         DevBuf<float> dist[2];
-        DevBuf<int> vs;
-        DevBuf<float> zs;
+        DevBuf<int> vs(st);
+        DevBuf<float> zs(st);
         PT_CUDA(dist[0].reserve(s.n));
         PT_CUDA(dist[1].reserve(s.n));
         PT_CUDA(vs.reserve(maxlines * maxn));

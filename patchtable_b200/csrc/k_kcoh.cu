@@ -379,14 +379,14 @@ pt_status pt_kc_lists_masked(int ew, int eh, int fbs, int ks, int reset, const i
     if (Q0 >= (1ll << 31) || N0 >= (1ll << 31) || reset < 1)
         return pt_fail(PT_UNSUPPORTED, "k-coherence index lists");    /* callers use the general path */
     const long long M = std::max(N0, Q0);
-    DevBuf<int> tflag, tinc, qflag, qinc, gflag, ginc, tot;
+    DevBuf<int> tflag(st), tinc(st), qflag(st), qinc(st), gflag(st), ginc(st), tot(st);
     PT_CUDA(tflag.reserve(N0)); PT_CUDA(tinc.reserve(N0));
     PT_CUDA(qflag.reserve(Q0)); PT_CUDA(qinc.reserve(Q0));
     PT_CUDA(gflag.reserve(Q0)); PT_CUDA(ginc.reserve(Q0));
     PT_CUDA(tot.reserve(3));
     size_t tmp_bytes = 0;
     PT_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp_bytes, tflag.p, tinc.p, (int) M, st));
-    DevBuf<unsigned char> tmp;
+    DevBuf<unsigned char> tmp(st);
     PT_CUDA(tmp.reserve(tmp_bytes));
     const unsigned blocks = (unsigned) ((M + 255) / 256);
     k_kc_flags<<<blocks, 256, 0, st>>>(allowed, allowed_index, ew, fbs, ks, ntx, (int) N0, nqx, (int) Q0, tflag.p, qflag.p);
@@ -428,7 +428,7 @@ pt_status pt_kc_lists(int ew, int eh, int fbs, int ks, int reset, int *trows, in
         return pt_fail(PT_UNSUPPORTED, "k-coherence index lists");    /* callers use the general path */
     const bool first = cols[0] != 0;                                   /* query 0 opens a segment of its own */
     const long long nseg = (long long) nqy * (long long) cols.size();
-    DevBuf<int> d_cols;
+    DevBuf<int> d_cols(st);
     PT_CUDA(d_cols.reserve(cols.size()));
     PT_CUDA(cudaMemcpyAsync(d_cols.p, cols.data(), sizeof(int) * cols.size(), cudaMemcpyHostToDevice, st));
     const long long tot = std::max(std::max(N, Q), nseg);
@@ -478,9 +478,9 @@ pt_status pt_kcoherence(const float4 *b_rgba, int bw, const float *bdesc, int ds
         }
         const int W = wide ? Kc / 64 : 1;
         if (Kc > N) return pt_fail(PT_BAD_ARG, "k-coherence: image has too few patches (%d)", N);
-        DevBuf<int> nbr, mm, knn, ovf;
-        DevBuf<unsigned long long> valid;
-        DevBuf<float> ssd;
+        DevBuf<int> nbr(st), mm(st), knn(st), ovf(st);
+        DevBuf<unsigned long long> valid(st);
+        DevBuf<float> ssd(st);
         PT_CUDA(nbr.reserve((size_t) Q * Kc));
         PT_CUDA(mm.reserve(Q));
         PT_CUDA(knn.reserve(Q));
@@ -509,14 +509,14 @@ pt_status pt_kcoherence(const float4 *b_rgba, int bw, const float *bdesc, int ds
         else
             k_kc_ssd<<<(unsigned) ((tot + 255) / 256), 256, 0, st>>>(b_rgba, bw, nbr.p, Kc, Q, qpos, tpos, knn.p, ssd.p);
         PT_LAUNCHED();
-        DevBuf<int2> o0, o1;
-        DevBuf<unsigned char> fn, pre;
+        DevBuf<int2> o0(st), o1(st);
+        DevBuf<unsigned char> fn(st), pre(st);
         PT_CUDA(o0.reserve((size_t) Q * kc));
         PT_CUDA(o1.reserve((size_t) Q * kc));
         PT_CUDA(fn.reserve(nseg));
         PT_CUDA(pre.reserve(nseg));
-        DevBuf<float> wsd;
-        DevBuf<int> wsp, wso;
+        DevBuf<float> wsd(st);
+        DevBuf<int> wsp(st), wso(st);
         if (wide) {
             PT_CUDA(wsd.reserve((size_t) nseg * Kc));
             PT_CUDA(wsp.reserve((size_t) nseg * Kc));
@@ -530,7 +530,7 @@ pt_status pt_kcoherence(const float4 *b_rgba, int bw, const float *bdesc, int ds
         PT_LAUNCHED();
         size_t tb = 0;
         PT_CUDA(cub::DeviceScan::InclusiveScan(nullptr, tb, fn.p, pre.p, ComposeOp(), nseg, st));
-        DevBuf<unsigned char> tmp;
+        DevBuf<unsigned char> tmp(st);
         PT_CUDA(tmp.reserve(tb));
         PT_CUDA(cub::DeviceScan::InclusiveScan(tmp.p, tb, fn.p, pre.p, ComposeOp(), nseg, st));
         pt_count_launches(1);

@@ -645,7 +645,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
     if (nd < 1 || nd > PT_DESC_MAX) return pt_fail(PT_UNSUPPORTED, "knn: %d dims", nd);
     /* range of the train and query points */
     const int NB = 2 * 148;
-    DevBuf<float> pmn, pmx;
+    DevBuf<float> pmn(st), pmx(st);
     PT_CUDA(pmn.reserve(NB * PT_DESC_MAX));
     PT_CUDA(pmx.reserve(NB * PT_DESC_MAX));
     k_range<<<NB / 2, NT, 0, st>>>(train, N, nd, pmn.p, pmx.p);
@@ -673,9 +673,9 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
     }
     for (int d = 0; d < nd; d++) qz.scale[d] = rmax > 0.f ? (float) ((1u << qz.bits) - 1) / rmax : 0.f;
     /* sort train points and queries along the curve */
-    DevBuf<unsigned long long> codes, codes2;
-    DevBuf<int> idx, perm, qidx, qorder, sidx;
-    DevBuf<float> sp;
+    DevBuf<unsigned long long> codes(st), codes2(st);
+    DevBuf<int> idx(st), perm(st), qidx(st), qorder(st), sidx(st);
+    DevBuf<float> sp(st);
     PT_CUDA(codes.reserve(std::max(N, Q)));
     PT_CUDA(codes2.reserve(std::max(N, Q)));
     PT_CUDA(idx.reserve(std::max(N, Q)));
@@ -686,7 +686,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
     PT_CUDA(sp.reserve((size_t) N * dp));
     size_t tb = 0;
     PT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, codes.p, codes2.p, idx.p, perm.p, std::max(N, Q), 0, 64, st));
-    DevBuf<unsigned char> tmp;
+    DevBuf<unsigned char> tmp(st);
     PT_CUDA(tmp.reserve(tb));
     k_curve<<<(N + 255) / 256, 256, 0, st>>>(qz, train, N, codes.p, idx.p);
     PT_LAUNCHED();
@@ -705,7 +705,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
         /* bucket boxes and the binary tree above them */
         int L = 1;
         while (L < nbk) L <<= 1;
-        DevBuf<float> lo, hi;
+        DevBuf<float> lo(st), hi(st);
         PT_CUDA(lo.reserve((size_t) 2 * L * nd));
         PT_CUDA(hi.reserve((size_t) 2 * L * nd));
         k_leaf_box<<<(L + 255) / 256, 256, 0, st>>>(sp.p, N, nd, L, lo.p, hi.p);
@@ -714,7 +714,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
             k_inner_box<<<(first + 255) / 256, 256, 0, st>>>(first, first, nd, lo.p, hi.p);
             PT_LAUNCHED();
         }
-        DevBuf<float> wd;
+        DevBuf<float> wd(st);
         PT_CUDA(wd.reserve((size_t) Q * K));
         k_knn_wide<<<grid, NT, 0, st>>>(sp.p, perm.p, N, nd, L, lo.p, hi.p, qdesc, qorder.p, Q, K, wd.p, out);
         PT_LAUNCHED();
@@ -732,7 +732,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
         off[l] = total;
         total += (size_t) 2 * nd * tr.stride[l];
     }
-    DevBuf<float> boxes, rows;
+    DevBuf<float> boxes(st), rows(st);
     PT_CUDA(boxes.reserve(total));
     PT_CUDA(rows.reserve((size_t) nbk * 2 * dp));
     tr.bucket = rows.p;

@@ -345,12 +345,12 @@ pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *de
     a.run_dt = run_dt; a.dt_iters = dt_iters; a.fill_zeros = fill_zeros; a.vfill = vfill;
     a.spin_limit = pt_spin_limit();
     /* Scratch: claim keys and two frontiers of at most one element per cell. */
-    DevBuf<unsigned> claim;
-    DevBuf<int> fidx0, fidx1, status;
-    DevBuf<unsigned char> flab0, flab1;
-    DevBuf<unsigned> emask;
-    DevBuf<long long> ctot, seed_n;
-    DevBuf<unsigned> bar;
+    DevBuf<unsigned> claim(st);
+    DevBuf<int> fidx0(st), fidx1(st), status(st);
+    DevBuf<unsigned char> flab0(st), flab1(st);
+    DevBuf<unsigned> emask(st);
+    DevBuf<long long> ctot(st), seed_n(st);
+    DevBuf<unsigned> bar(st);
     if (run_dt) {
         PT_CUDA(claim.reserve(ncells));
         PT_CUDA(fidx0.reserve(ncells)); PT_CUDA(fidx1.reserve(ncells));

@@ -64,11 +64,20 @@ struct PtPartition {
 };
 
 #ifdef __CUDACC__
-/* A device buffer owned by the table; freed with cudaFree. */
+/* pt_memory.cu: device and page-locked memory, pooled. */
+cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch);
+void pt_dev_free(void *p, int dev, cudaStream_t st, bool scratch);
+cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got);
+void pt_pinned_free(void *p, size_t bytes);
+
+/* A device buffer.  DevBuf() may be used on any stream, and its release waits for the device.
+   DevBuf(st) is scratch: used on st only (or on streams joined into it before the release), and
+   released in st's order without waiting; st outlives it. */
 template<class T> struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     DevBuf() {}
+    explicit DevBuf(cudaStream_t s) : st(s), scratch(true) {}
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }
@@ -77,36 +86,45 @@ template<class T> struct DevBuf {
         release();
         const size_t bytes = sizeof(T) * (count ? count : 1);
         if (!pt_alloc_admit(bytes)) return cudaErrorMemoryAllocation;
-        cudaError_t e = cudaMalloc((void **) &p, bytes);
+        cudaGetDevice(&dev);
+        cudaError_t e = pt_dev_alloc((void **) &p, bytes, st, scratch);
         if (e == cudaSuccess) { n = count; held = bytes; }
         else { p = nullptr; pt_alloc_release(bytes); }
         return e;
     }
     void release() {
-        if (p) { cudaFree(p); pt_alloc_release(held); }
+        if (p) { pt_dev_free(p, dev, st, scratch); pt_alloc_release(held); }
         p = nullptr; n = 0; held = 0;
     }
 private:
     size_t held = 0;
+    cudaStream_t st = nullptr;
+    bool scratch = false;
+    int dev = 0;
 };
 
-/* Page-locked host memory owned by a table (download staging); freed with cudaFreeHost. */
+/* Page-locked host memory owned by a table (download staging). */
 template<class T> struct PinnedBuf {
     T *p = nullptr;
     size_t n = 0;
     PinnedBuf() {}
     PinnedBuf(const PinnedBuf &) = delete;
     PinnedBuf &operator=(const PinnedBuf &) = delete;
-    ~PinnedBuf() { if (p) cudaFreeHost(p); }
+    ~PinnedBuf() { release(); }
     cudaError_t reserve(size_t count) {
         if (count <= n && p) return cudaSuccess;
-        if (p) cudaFreeHost(p);
-        p = nullptr; n = 0;
-        cudaError_t e = cudaMallocHost((void **) &p, sizeof(T) * (count ? count : 1));
+        release();
+        cudaError_t e = pt_pinned_alloc((void **) &p, sizeof(T) * (count ? count : 1), &held);
         if (e == cudaSuccess) n = count;
         else p = nullptr;
         return e;
     }
+    void release() {
+        if (p) pt_pinned_free(p, held);
+        p = nullptr; n = 0; held = 0;
+    }
+private:
+    size_t held = 0;
 };
 #endif
 

@@ -48,6 +48,7 @@ struct PtPartScratch {
     DevBuf<float> pmin, pmax, keys, sorted, picked;
     DevBuf<int> cnt, idx;
     DevBuf<unsigned char> tmp;
+    explicit PtPartScratch(cudaStream_t st) : pmin(st), pmax(st), keys(st), sorted(st), picked(st), cnt(st), idx(st), tmp(st) {}
 };
 #else
 struct PtPartScratch;

@@ -1,0 +1,153 @@
+/* Device and page-locked host memory of the library.
+
+   Builds take about sixty device buffers and give most of them back, and a cudaMalloc or cudaFree
+   costs 0.1 ms and up (with the mapping of large blocks, 18 of the 31 ms of a 240 x 320 build; a
+   cudaFree also waits for the whole device).  Buffers therefore come from one CUDA memory pool per
+   device.  Scratch buffers (DevBuf given a stream) are freed in that stream's order; all others may
+   have been used on any stream, so their release waits for the device first, as cudaFree did.
+   Reuse across streams that would make one stream wait for another is switched off: the steps of a
+   build run beside each other.
+
+   What the pool keeps for reuse is bounded: at most PT_POOL_KEEP bytes per device stay reserved
+   once they are free, everything is given back when an allocation fails (which is then tried
+   again) and by pt_release_memory().  Page-locked blocks are kept the same way, at most
+   PT_PINNED_KEEP bytes per process.  Both are safe with any number of threads and streams. */
+#include <cuda_runtime.h>
+
+#include <mutex>
+#include <vector>
+
+#include "patchtable_b200.h"
+#include "pt_internal.h"
+
+namespace {
+
+constexpr unsigned long long PT_POOL_KEEP = 4ull << 30;
+constexpr size_t PT_PINNED_KEEP = 256u << 20;
+constexpr int MAX_DEVICES = 64;
+
+struct DevicePool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t st = nullptr;            /* order of the buffers that belong to no stream */
+};
+DevicePool g_pool[MAX_DEVICES];
+
+struct Pinned { void *p; size_t bytes; };
+std::mutex g_pinned_mu;
+std::vector<Pinned> g_pinned;             /* free page-locked blocks */
+size_t g_pinned_bytes = 0;
+
+/* The current device's pool, created on first use. */
+cudaError_t device_pool(DevicePool **out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
+    DevicePool &d = g_pool[dev];
+    std::lock_guard<std::mutex> lock(d.mu);
+    if (!d.pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+        unsigned long long keep = PT_POOL_KEEP;
+        int off = 0;
+        cudaStream_t st = nullptr;
+        if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess ||
+            (e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off)) != cudaSuccess ||
+            (e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        d.st = st;
+        d.pool = pool;
+    }
+    *out = &d;
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch) {
+    DevicePool *d = nullptr;
+    cudaError_t e = device_pool(&d);
+    if (e != cudaSuccess) return e;
+    if (!scratch) st = d->st;
+    e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(d->pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    /* a buffer of no stream must be usable on every stream when this returns */
+    if (e == cudaSuccess && !scratch) e = cudaStreamSynchronize(st);
+    return e;
+}
+
+void pt_dev_free(void *p, int dev, cudaStream_t st, bool scratch) {
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    if (!scratch) {
+        cudaDeviceSynchronize();
+        st = g_pool[dev].st;
+    }
+    cudaFreeAsync(p, st);
+    if (cur != dev) cudaSetDevice(cur);
+}
+
+cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got) {
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        int best = -1;
+        for (int i = 0; i < (int) g_pinned.size(); i++)
+            if (g_pinned[i].bytes >= bytes && g_pinned[i].bytes <= 2 * bytes &&
+                (best < 0 || g_pinned[i].bytes < g_pinned[best].bytes))
+                best = i;
+        if (best >= 0) {
+            *p = g_pinned[best].p;
+            *got = g_pinned[best].bytes;
+            g_pinned_bytes -= *got;
+            g_pinned.erase(g_pinned.begin() + best);
+            return cudaSuccess;
+        }
+    }
+    *got = bytes;
+    return cudaMallocHost(p, bytes);
+}
+
+void pt_pinned_free(void *p, size_t bytes) {
+    cudaDeviceSynchronize();              /* no copy of a failed call may still use it */
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        if (g_pinned_bytes + bytes <= PT_PINNED_KEEP) {
+            g_pinned.push_back({p, bytes});
+            g_pinned_bytes += bytes;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+extern "C" pt_status pt_release_memory(void) {
+    for (DevicePool &d : g_pool) {
+        std::lock_guard<std::mutex> lock(d.mu);
+        if (d.pool) {
+            cudaStreamSynchronize(d.st);
+            PT_CUDA(cudaMemPoolTrimTo(d.pool, 0));
+        }
+    }
+    std::vector<Pinned> held;
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        held.swap(g_pinned);
+        g_pinned_bytes = 0;
+    }
+    for (const Pinned &b : held) cudaFreeHost(b.p);
+    return PT_OK;
+}

@@ -311,7 +311,7 @@ pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
         /* The lists are generated on the device (no host loops or copies): regular grids without
            a mask, the same grids compacted to the allowed points with one. */
         const long long P = (long long) eh * ew;
-        DevBuf<int> d_trows, d_tpos, d_qrows, d_qpos, d_qcell, d_seg;
+        DevBuf<int> d_trows(t->st), d_tpos(t->st), d_qrows(t->st), d_qpos(t->st), d_qcell(t->st), d_seg(t->st);
         PT_CUDA(d_trows.reserve(P)); PT_CUDA(d_tpos.reserve(P));
         PT_CUDA(d_qrows.reserve(P)); PT_CUDA(d_qpos.reserve(P)); PT_CUDA(d_qcell.reserve(P)); PT_CUDA(d_seg.reserve(P + 1));
         int N = 0, Q = 0, nseg = 0;
@@ -326,7 +326,7 @@ pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
             PT_CUDA(t->kcoh.reserve((size_t) P * p.kcoherence));
             PT_CUDA(cudaMemsetAsync(t->kcoh.p, 0, sizeof(int2) * (size_t) P * p.kcoherence, t->st));
             if (Q == 0) return PT_OK;
-            DevBuf<float> train, qdesc;
+            DevBuf<float> train(t->st), qdesc(t->st);
             PT_CUDA(train.reserve((size_t) N * t->nd)); PT_CUDA(qdesc.reserve((size_t) Q * t->nd));
             PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_trows.p, N, train.p, t->st));
             PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_qrows.p, Q, qdesc.p, t->st));
@@ -359,8 +359,8 @@ pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
     PT_CUDA(t->kcoh.reserve((size_t) eh * ew * p.kcoherence));
     PT_CUDA(cudaMemsetAsync(t->kcoh.p, 0, sizeof(int2) * (size_t) eh * ew * p.kcoherence, t->st));
     if (Q == 0) return PT_OK;
-    DevBuf<int> d_trows, d_tpos, d_qrows, d_qpos, d_qcell, d_seg;
-    DevBuf<float> train, qdesc;
+    DevBuf<int> d_trows(t->st), d_tpos(t->st), d_qrows(t->st), d_qpos(t->st), d_qcell(t->st), d_seg(t->st);
+    DevBuf<float> train(t->st), qdesc(t->st);
     PT_CUDA(d_trows.reserve(N)); PT_CUDA(d_tpos.reserve(N));
     PT_CUDA(d_qrows.reserve(Q)); PT_CUDA(d_qpos.reserve(Q)); PT_CUDA(d_qcell.reserve(Q)); PT_CUDA(d_seg.reserve(nseg));
     PT_CUDA(train.reserve((size_t) N * t->nd)); PT_CUDA(qdesc.reserve((size_t) Q * t->nd));
@@ -424,7 +424,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     };
 
     if (t->desc_mode) {
-        DevBuf<float> in;
+        DevBuf<float> in(t->st);
         const size_t nin = (size_t) h * w * channels;
         PT_CUDA(in.reserve(nin));
         PT_CUDA(cudaMemcpyAsync(in.p, b, sizeof(float) * nin, cudaMemcpyHostToDevice, t->st));
@@ -433,7 +433,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         PT_CUDA(cudaStreamSynchronize(t->st));
     } else {
     /* Descriptor of b (get_padded_descriptor, patchtable.h:2492-2546) and the RGBA copy kept as b0. */
-        DevBuf<float> rgb;
+        DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve((size_t) h * w * 3));
         PT_CUDA(cudaMemcpyAsync(rgb.p, b, sizeof(float) * (size_t) h * w * 3, cudaMemcpyHostToDevice, t->st));
         PT_CUDA(t->b_rgba.reserve((size_t) h * w));
@@ -516,7 +516,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         if (e != cudaSuccess) { shuffler.join(); return pt_fail(PT_CUDA_ERR, "stream: %s", cudaGetErrorString(e)); }
     }
     double part_ms = 0.0;
-    PtPartScratch part_scratch;       /* freed when the build returns, after the search has ended */
+    PtPartScratch part_scratch(t->st2);       /* freed when the build returns, after the search has ended */
     std::string part_err;
     pt_status part_st = PT_OK;
     std::thread partitioner([&] {
@@ -561,7 +561,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     t->build_ms[PT_BUILD_SHUFFLE] = shuffle_ms;
     if (order_xy.empty()) return pt_fail(PT_BAD_ARG, "no allowed patches");
     {
-        DevBuf<int> d_rank, d_order;
+        DevBuf<int> d_rank(t->st), d_order(t->st);
         PT_CUDA(d_rank.reserve(P));
         PT_CUDA(d_order.reserve(order_xy.size()));
         PT_CUDA(cudaMemcpyAsync(d_rank.p, rank.data(), sizeof(int) * P, cudaMemcpyHostToDevice, t->st));
@@ -1260,7 +1260,7 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
     t->own_stream = true;
     const long long P = (long long) t->eh * t->ew;
     {
-        DevBuf<float> rgb;
+        DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve(b0.size()));
         PT_CUDA(cudaMemcpyAsync(rgb.p, b0.data(), sizeof(float) * b0.size(), cudaMemcpyHostToDevice, t->st));
         PT_CUDA(t->b_rgba.reserve((size_t) h * w));
