@@ -12,7 +12,7 @@
    the launch always ends and the host reports the status.
 
    Phases (one grid barrier after each):
-     fill      every cell TABLE_UNUSED, every claim key empty;
+     fill      every cell empty;
      populate  each allowed patch's cell takes the smallest shuffle rank that reaches it (the first
                visitor of the reference's random_shuffle order wins);
      resolve   ranks become packed positions; each CTA counts the seeded cells of its contiguous
@@ -20,11 +20,17 @@
      seed      the seeded cells, in increasing cell order, become the first frontier (label 0):
                each CTA writes its range at the prefix of the counts before it;
      levels    the reference's breadth-first fill, level-synchronously: every frontier element
-               claims the unused neighbours its label allows with atomicMin on (element, edge) and
-               keeps a bit mask of those edges; each CTA checks, for its contiguous range of
-               elements, which of the masked claims they won (a second mask); winners fill their
-               cells and append (cell, label) to the next frontier at the scanned offsets, i.e. in
-               (element, edge) order, which is the order of the reference's next frontier list.
+               claims the empty neighbours its label allows with an atomicMin on (element, edge),
+               and the bits of the claims it holds are kept in its edge mask: an element toggles the
+               bits it claims, and the bit of the holder it takes a cell from, so that after the
+               phase the masks hold the winners (toggles commute).  Each CTA counts the bits of its
+               contiguous range of elements; winners fill their cells and append (cell, label) to
+               the next frontier at the scanned offsets, i.e. in (element, edge) order, which is the
+               order of the reference's next frontier list.
+   A filled cell holds its packed position (below 2^30), an empty one 0xffffffff, and a claimed one
+   the claim's key, 2^30 + (element, edge), which its winner overwrites: the claims need no array of
+   their own while every key fits (FUSED), and a neighbour's one read says whether it is empty and
+   whether an earlier element already holds it.
    The filled table is therefore bit-identical to the reference's.  Data written by other CTAs in
    an earlier phase is read with L2-only loads (ld.global.cg), never from a CTA's own L1. */
 #include <cuda_runtime.h>
@@ -40,7 +46,10 @@
 namespace {
 
 constexpr int NT = 256;
-constexpr long long KEY_ELEMENTS = 1ll << 27;   /* claim key = element << 5 | edge */
+constexpr int STAGE = 2048;                     /* new cells staged in shared memory at a time */
+constexpr unsigned EMPTY = 0xffffffffu;
+constexpr unsigned KEY_BASE = 1u << 30;         /* smallest claim key: packed positions lie below */
+constexpr long long KEY_ELEMENTS = 1ll << 27;   /* separate claims: key = element << 5 | edge */
 
 struct CellBuild {
     int G;
@@ -49,16 +58,20 @@ struct CellBuild {
     int nslices[PT_DESC_MAX];
     const float *desc;
     int ds;
-    long long P;
-    const int *rank;             /* shuffle rank of each patch, -1 when not allowed */
+    int ew;
+    long long np;                /* entries of order_xy */
     const int *to_bin;
-    const int *order_xy;         /* packed position of each rank */
-    int *table;
+    const int *order_xy;         /* packed position of each shuffle rank */
+    unsigned *table;
     long long ncells;
-    unsigned *claim;
+    unsigned *claim;             /* the table itself (FUSED), or one key per cell */
+    unsigned key_base;
+    int ebits;                   /* edge bits of a key */
+    unsigned div_mul[PT_DESC_MAX];   /* division by nslices: floor(x / n) = umulhi(x, mul) >> shift for x < 2^31 */
+    int div_shift[PT_DESC_MAX];
     int *fidx[2];
     unsigned char *flab[2];
-    unsigned *emask;             /* per frontier element: edges to unused neighbours, then the edges it won */
+    unsigned *emask[2];          /* per frontier element: the edges whose claims it holds */
     long long *ctot;             /* per-CTA totals */
     unsigned *bar;               /* [0] arrivals, [1] generation */
     int *status;                 /* [0] pt_status of the launch, [1] levels, [2] phase that failed */
@@ -134,8 +147,6 @@ __device__ __forceinline__ void cta_prefix(Shared &sh, const CellBuild &a, long 
 /* Edge e of label lab (patchtable.h:2101-2120): label 0 -> (i, -1), (i, +1) for every dimension i;
    label 2i + 1 + (dir + 1) / 2 -> (i, dir), then (j, -1), (j, +1) for every j > i.  The label the
    filled cell receives is that of the edge's own (dimension, direction). */
-__device__ __forceinline__ int edge_count(int G, int lab) { return lab == 0 ? 2 * G : 1 + 2 * (G - 1 - (lab - 1) / 2); }
-
 __device__ __forceinline__ void edge_of(int lab, int e, int &dim, int &dir) {
     if (lab == 0) { dim = e >> 1; dir = (e & 1) ? 1 : -1; return; }
     const int i = (lab - 1) >> 1;
@@ -144,48 +155,95 @@ __device__ __forceinline__ void edge_of(int lab, int e, int &dim, int &dir) {
     dir = ((e - 1) & 1) ? 1 : -1;
 }
 
-/* Neighbour of cell g along (dim, dir) when it lies inside the grid and is still unused; -1 otherwise. */
-__device__ __forceinline__ long long open_neighbour(const CellBuild &a, long long g, int dim, int dir) {
-    const long long gp = g + dir * a.stride[dim];
-    if (gp < 0 || gp >= a.ncells) return -1;
-    const long long dp = (g / a.stride[dim]) % a.nslices[dim] + dir;
-    if (dp < 0 || dp >= a.nslices[dim]) return -1;
-    if (__ldcg(a.table + gp) != PT_UNUSED) return -1;
-    return gp;
+/* x / nslices[d] for x < 2^31. */
+__device__ __forceinline__ unsigned div_slices(const CellBuild &a, int d, unsigned x) {
+    return a.div_mul[d] ? __umulhi(x, a.div_mul[d]) >> a.div_shift[d] : x;
 }
 
+/* The claims of frontier element i (cell g, label lab): all its neighbours are read before the first
+   claim, so an element waits for memory twice, not once per edge. */
+template<int MAXG>
+__device__ __forceinline__ void claim_neighbours(const CellBuild &a, unsigned *emask, unsigned i, unsigned g, int lab) {
+    const int li = lab == 0 ? -1 : (lab - 1) >> 1, lp = (lab - 1) & 1;
+    unsigned v[2 * MAXG];
+    unsigned r = g;
+#pragma unroll
+    for (int d = MAXG - 1; d >= 0; d--) {
+        v[2 * d] = v[2 * d + 1] = 0;
+        if (d < a.G) {
+            const unsigned q = div_slices(a, d, r), dig = r - q * (unsigned) a.nslices[d], st = (unsigned) a.stride[d];
+            r = q;
+            if (dig > 0 && (d > li || (d == li && !lp))) v[2 * d] = __ldcg(a.table + (g - st));
+            if (dig + 1 < (unsigned) a.nslices[d] && (d > li || (d == li && lp))) v[2 * d + 1] = __ldcg(a.table + (g + st));
+        }
+    }
+    const unsigned key0 = a.key_base + (i << a.ebits);
+    unsigned old[2 * MAXG];
+#pragma unroll
+    for (int k = 0; k < 2 * MAXG; k++) {
+        const int d = k >> 1;
+        const unsigned e = lab == 0 ? k : d == li ? 0 : 2 * (d - li) - 1 + (k & 1);
+        old[k] = 0;
+        if (v[k] >= KEY_BASE && (a.claim != a.table || key0 + e < v[k]))
+            old[k] = atomicMin(a.claim + ((k & 1) ? g + (unsigned) a.stride[d] : g - (unsigned) a.stride[d]), key0 + e);
+    }
+    unsigned won = 0;
+#pragma unroll
+    for (int k = 0; k < 2 * MAXG; k++) {
+        const int d = k >> 1;
+        const unsigned e = lab == 0 ? k : d == li ? 0 : 2 * (d - li) - 1 + (k & 1);
+        if (old[k] > key0 + e) {
+            won |= 1u << e;
+            if (old[k] != EMPTY) {
+                const unsigned o = old[k] - a.key_base;
+                atomicXor(emask + (o >> a.ebits), 1u << (o & ((1u << a.ebits) - 1)));
+            }
+        }
+    }
+    if (won) atomicXor(emask + i, won);
+}
+
+/* Bound: the latency of the levels' random accesses (98 M elements over 20 levels in a 1920x1080
+   table).  6.4 ms there, of which claims 2.9, counts 0.16, emission 2.8 and the rest 0.5 ms; 14.8 ms
+   (6.5, 4.2, 3.2, 0.9) with claims in an array of their own, one dependent read per edge with 64-bit
+   divisions, a count phase that read every claim again and lists written a thread's run at a time.
+   Claims unrolled over 8 dimensions instead of 6 take 3.2 ms; 6 CTAs per SM instead of 4, 3.5. */
+template<int MAXG>
 __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
     __shared__ Shared sh;
+    __shared__ int st_cell[STAGE];
+    __shared__ unsigned st_val[STAGE];
+    __shared__ unsigned char st_lab[STAGE];
     const long long nthr = (long long) gridDim.x * NT;
     const long long tid = (long long) blockIdx.x * NT + threadIdx.x;
 
     /* fill */
     for (long long i = tid; i < a.ncells; i += nthr) {
-        a.table[i] = PT_UNUSED;
-        if (a.run_dt) a.claim[i] = 0xffffffffu;
+        a.table[i] = EMPTY;
+        if (a.run_dt && a.claim != a.table) a.claim[i] = EMPTY;
     }
     if (!grid_barrier(a, 0)) return;
 
     /* populate: first visitor in shuffled order wins (patchtable.h:3142-3154) */
-    for (long long p = tid; p < a.P; p += nthr) {
-        const int r = __ldg(a.rank + p);
-        if (r < 0) continue;
+    for (long long r = tid; r < a.np; r += nthr) {
+        const int xy = __ldg(a.order_xy + r);
+        const long long p = (long long) (pt_y(xy) - 7) * a.ew + (pt_x(xy) - 7);
         const float *v = a.desc + p * a.ds;
         long long cell = 0;
         for (int d = 0; d < a.G; d++)
             cell += (long long) pt_get_bin(a.min_val[d], a.range[d], a.to_bin + d * PT_NMAP, __ldg(v + d)) * a.stride[d];
-        atomicMin(a.table + cell, r);
+        atomicMin(a.table + cell, (unsigned) r);
     }
     if (!grid_barrier(a, 1)) return;
 
     /* resolve: ranks -> packed positions; seeded cells of this CTA's range */
-    const long long chunk = (a.ncells + gridDim.x - 1) / gridDim.x;
+    const long long chunk = ((a.ncells + gridDim.x - 1) / gridDim.x + 3) & ~3ll;
     const long long c0 = min(a.ncells, (long long) blockIdx.x * chunk), c1 = min(a.ncells, c0 + chunk);
     {
         long long local = 0;
         for (long long j = c0 + threadIdx.x; j < c1; j += NT) {
-            const int v = __ldcg(a.table + j);
-            if (v != PT_UNUSED) { a.table[j] = __ldg(a.order_xy + v); local++; }
+            const unsigned v = __ldcg(a.table + j);
+            if (v != EMPTY) { a.table[j] = (unsigned) __ldg(a.order_xy + v); local++; }
         }
         const long long s = cta_sum(sh, local);
         if (threadIdx.x == 0) a.ctot[blockIdx.x] = s;
@@ -199,13 +257,26 @@ __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
     if (a.run_dt) {
         /* seed: the first frontier in increasing cell order, label 0 (patchtable.h:2087-2093) */
         long long o = before;
-        for (long long j0 = c0; j0 < c1; j0 += NT) {
-            const long long j = j0 + threadIdx.x;
-            const int f = (j < c1 && __ldcg(a.table + j) != PT_UNUSED) ? 1 : 0;
+        for (long long j0 = c0; j0 < c1; j0 += 4 * NT) {
+            const long long j = j0 + 4 * threadIdx.x;
+            unsigned f = 0;
+            if (j < c1) {
+                const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(a.table + j));
+                f = (v.x != EMPTY ? 1u : 0u) | (v.y != EMPTY ? 2u : 0u) | (v.z != EMPTY ? 4u : 0u) | (v.w != EMPTY ? 8u : 0u);
+                if (j + 4 > c1) f &= (1u << (c1 - j)) - 1;
+            }
             int off, tot;
             __syncthreads();
-            Scan(sh.scan).ExclusiveSum(f, off, tot);
-            if (f) { a.fidx[0][o + off] = (int) j; a.flab[0][o + off] = 0; }
+            Scan(sh.scan).ExclusiveSum(__popc(f), off, tot);
+            long long w = o + off;
+            while (f) {
+                const int k = __ffs(f) - 1;
+                f &= f - 1;
+                a.fidx[0][w] = (int) (j + k);
+                a.flab[0][w] = 0;
+                a.emask[0][w] = 0;
+                w++;
+            }
             o += tot;
         }
         if (!grid_barrier(a, 3)) return;
@@ -213,50 +284,26 @@ __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
         for (int iter = 0;; iter++) {
             if (a.dt_iters > 0 && iter > a.dt_iters) break;
             if (n == 0) break;
-            if (n >= KEY_ELEMENTS) {
+            if (a.claim != a.table && n >= KEY_ELEMENTS) {
                 if (blockIdx.x == 0 && threadIdx.x == 0 && atomicCAS(a.status, 0, (int) PT_UNSUPPORTED) == 0) a.status[2] = 4;
                 return;
             }
             const int *fi = a.fidx[cur];
             const unsigned char *fl = a.flab[cur];
-            /* claim: the smallest (element, edge) key wins each unused neighbour (:2131-2156); the
-               element remembers which of its edges led to an unused neighbour */
-            for (long long i = tid; i < n; i += nthr) {
-                const long long g = __ldcg(fi + i);
-                const int lab = __ldcg(fl + i), ne = edge_count(a.G, lab);
-                unsigned open = 0;
-                for (int e = 0; e < ne; e++) {
-                    int dim, dir;
-                    edge_of(lab, e, dim, dir);
-                    const long long gp = open_neighbour(a, g, dim, dir);
-                    if (gp >= 0) {
-                        atomicMin(a.claim + gp, ((unsigned) i << 5) | (unsigned) e);
-                        open |= 1u << e;
-                    }
-                }
-                a.emask[i] = open;
-            }
+            unsigned *em = a.emask[cur];
+            /* claim: the smallest (element, edge) key wins each empty neighbour (:2131-2156) */
+            for (long long i = tid; i < n; i += nthr)
+                claim_neighbours<MAXG>(a, em, (unsigned) i, (unsigned) __ldcg(fi + i), __ldcg(fl + i));
             if (!grid_barrier(a, 5)) return;
-            /* count the claims each element of this CTA's range won (only its open edges) */
-            const long long ech = (n + gridDim.x - 1) / gridDim.x;
+            /* count the claims won in this CTA's range of elements */
+            const long long ech = ((n + gridDim.x - 1) / gridDim.x + 3) & ~3ll;
             const long long e0 = min(n, (long long) blockIdx.x * ech), e1 = min(n, e0 + ech);
             {
                 long long local = 0;
-                for (long long i = e0 + threadIdx.x; i < e1; i += NT) {
-                    unsigned open = __ldcg(a.emask + i), won = 0;
-                    if (open) {
-                        const long long g = __ldcg(fi + i);
-                        const int lab = __ldcg(fl + i);
-                        while (open) {
-                            const int e = __ffs(open) - 1;
-                            open &= open - 1;
-                            int dim, dir;
-                            edge_of(lab, e, dim, dir);
-                            if (__ldcg(a.claim + g + dir * a.stride[dim]) == (((unsigned) i << 5) | (unsigned) e)) won |= 1u << e;
-                        }
-                    }
-                    a.emask[i] = won;
-                    local += __popc(won);
+                for (long long i = e0 + 4 * threadIdx.x; i < e1; i += 4 * NT) {
+                    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(em + i));
+                    local += __popc(w.x) + (i + 1 < e1 ? __popc(w.y) : 0) + (i + 2 < e1 ? __popc(w.z) : 0) +
+                             (i + 3 < e1 ? __popc(w.w) : 0);
                 }
                 const long long s = cta_sum(sh, local);
                 if (threadIdx.x == 0) a.ctot[blockIdx.x] = s;
@@ -264,32 +311,64 @@ __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
             if (!grid_barrier(a, 6)) return;
             long long base, next;
             cta_prefix(sh, a, base, next);
-            /* emit: winners fill their cells and append to the next frontier in (element, edge) order */
+            /* emit: winners fill their cells and append to the next frontier in (element, edge)
+               order, four consecutive elements per thread */
             int *nfi = a.fidx[1 - cur];
             unsigned char *nfl = a.flab[1 - cur];
+            unsigned *nem = a.emask[1 - cur];
             long long o2 = base;
-            for (long long t0 = e0; t0 < e1; t0 += NT) {
-                const long long i = t0 + threadIdx.x;
-                unsigned won = i < e1 ? __ldcg(a.emask + i) : 0u;
+            for (long long t0 = e0; t0 < e1; t0 += 4 * NT) {
+                const long long i = t0 + 4 * threadIdx.x;
+                unsigned won[4] = {0, 0, 0, 0};
+                int g[4] = {0, 0, 0, 0}, lab[4] = {0, 0, 0, 0};
+                unsigned val[4] = {0, 0, 0, 0};
+                if (i < e1) {
+                    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(em + i));
+                    const int4 gi = __ldcg(reinterpret_cast<const int4 *>(fi + i));
+                    const uchar4 li = __ldcg(reinterpret_cast<const uchar4 *>(fl + i));
+                    won[0] = w.x; won[1] = w.y; won[2] = w.z; won[3] = w.w;
+                    g[0] = gi.x; g[1] = gi.y; g[2] = gi.z; g[3] = gi.w;
+                    lab[0] = li.x; lab[1] = li.y; lab[2] = li.z; lab[3] = li.w;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (i + k >= e1) won[k] = 0;
+                        if (won[k]) val[k] = __ldcg(a.table + g[k]);
+                    }
+                }
                 int off, tot;
                 __syncthreads();
-                Scan(sh.scan).ExclusiveSum(__popc(won), off, tot);
-                if (won) {
-                    const long long g = __ldcg(fi + i);
-                    const int lab = __ldcg(fl + i);
-                    const int val = __ldcg(a.table + g);
-                    long long w = o2 + off;
-                    while (won) {
-                        const int e = __ffs(won) - 1;
-                        won &= won - 1;
-                        int dim, dir;
-                        edge_of(lab, e, dim, dir);
-                        const long long gp = g + dir * a.stride[dim];
-                        a.table[gp] = val;
-                        nfi[w] = (int) gp;
-                        nfl[w] = (unsigned char) (2 * dim + 1 + (dir + 1) / 2);
-                        w++;
+                Scan(sh.scan).ExclusiveSum(__popc(won[0]) + __popc(won[1]) + __popc(won[2]) + __popc(won[3]), off, tot);
+                /* the tile's new cells in order, through shared memory, so that the lists are written
+                   in whole lines */
+                for (int r0 = 0; r0 < tot; r0 += STAGE) {
+                    int w = off - r0;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        unsigned m = won[k];
+                        while (m) {
+                            const int e = __ffs(m) - 1;
+                            m &= m - 1;
+                            if (w >= 0 && w < STAGE) {
+                                int dim, dir;
+                                edge_of(lab[k], e, dim, dir);
+                                st_cell[w] = g[k] + dir * (int) a.stride[dim];
+                                st_val[w] = val[k];
+                                st_lab[w] = (unsigned char) (2 * dim + 1 + (dir + 1) / 2);
+                            }
+                            w++;
+                        }
                     }
+                    __syncthreads();
+                    const int cnt = min(STAGE, tot - r0);
+                    for (int j = threadIdx.x; j < cnt; j += NT) {
+                        const long long o = o2 + r0 + j;
+                        const int gp = st_cell[j];
+                        a.table[gp] = st_val[j];
+                        nfi[o] = gp;
+                        nfl[o] = st_lab[j];
+                        nem[o] = 0;
+                    }
+                    __syncthreads();
                 }
                 o2 += tot;
             }
@@ -299,10 +378,10 @@ __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
             if (!grid_barrier(a, 7)) return;
         }
     }
-    if (a.fill_zeros) {                      /* fill_zeros, patchtable.h:2063-2079 */
-        for (long long i = tid; i < a.ncells; i += nthr)
-            if (__ldcg(a.table + i) == PT_UNUSED) a.table[i] = a.vfill;
-    }
+    /* cells no patch reached: fill_zeros' value (patchtable.h:2063-2079) or TABLE_UNUSED */
+    const unsigned rest = a.fill_zeros ? (unsigned) a.vfill : (unsigned) PT_UNUSED;
+    for (long long i = tid; i < a.ncells; i += nthr)
+        if (__ldcg(a.table + i) == EMPTY) a.table[i] = rest;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.status[1] = levels;
 }
 
@@ -317,7 +396,7 @@ extern "C" int64_t pt_set_spin_limit(int64_t polls) {
     return g_spin_limit.exchange(polls);
 }
 
-pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *desc, int ds, long long P, const int *rank,
+pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *desc, int ds, int ew, long long np,
                          const int *to_bin, const int *order_xy, int *table, long long ncells, int run_dt, int dt_iters,
                          int fill_zeros, int vfill, long long *seeded, int *levels, cudaStream_t st) {
     if (ncells >= (1ll << 31)) return pt_fail(PT_UNSUPPORTED, "tables above 2^31 cells are not supported");
@@ -327,7 +406,9 @@ pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *de
     PT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return pt_fail(PT_UNSUPPORTED, "the table build needs cooperative launches");
     PT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_table_build, NT, 0));
+    const void *kernel = bins.G <= 6 ? (const void *) k_table_build<6>
+                         : bins.G <= 8 ? (const void *) k_table_build<8> : (const void *) k_table_build<PT_DESC_MAX>;
+    PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, NT, 0));
     if (per < 1) return pt_fail(PT_CUDA_ERR, "the table build kernel cannot be resident");
     const int grid = nsm * per;
 
@@ -340,22 +421,36 @@ pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *de
         a.stride[d] = bins.stride[d];
         a.nslices[d] = nslices[d];
     }
-    a.desc = desc; a.ds = ds; a.P = P; a.rank = rank; a.to_bin = to_bin; a.order_xy = order_xy;
-    a.table = table; a.ncells = ncells;
+    a.desc = desc; a.ds = ds; a.ew = ew; a.np = np; a.to_bin = to_bin; a.order_xy = order_xy;
+    a.table = reinterpret_cast<unsigned *>(table); a.ncells = ncells;
+    for (int d = 0; d < bins.G; d++) {
+        /* ceil(2^(31 + l) / n) with 2^(l-1) < n <= 2^l: exact for dividends below 2^31 */
+        int l = 1;
+        while ((1ll << l) < nslices[d]) l++;
+        a.div_mul[d] = nslices[d] > 1 ? (unsigned) (((1ull << (31 + l)) + nslices[d] - 1) / nslices[d]) : 0;
+        a.div_shift[d] = l - 1;
+    }
+    /* claim keys share the table's words while 2^30 + (element, edge) stays below 2^32 for every
+       possible element; otherwise they get an array of their own */
+    a.ebits = bins.G <= 8 ? 4 : 5;
+    const bool fused = ncells <= (long long) ((EMPTY - KEY_BASE) >> a.ebits);
+    a.key_base = fused ? KEY_BASE : 0;
+    if (!fused) a.ebits = 5;
     a.run_dt = run_dt; a.dt_iters = dt_iters; a.fill_zeros = fill_zeros; a.vfill = vfill;
     a.spin_limit = pt_spin_limit();
-    /* Scratch: claim keys and two frontiers of at most one element per cell. */
+    /* Scratch: two frontiers of at most one element per cell, and the claim keys that do not share the
+       table's words. */
     DevBuf<unsigned> claim(st);
     DevBuf<int> fidx0(st), fidx1(st), status(st);
     DevBuf<unsigned char> flab0(st), flab1(st);
-    DevBuf<unsigned> emask(st);
+    DevBuf<unsigned> emask0(st), emask1(st);
     DevBuf<long long> ctot(st), seed_n(st);
     DevBuf<unsigned> bar(st);
     if (run_dt) {
-        PT_CUDA(claim.reserve(ncells));
-        PT_CUDA(fidx0.reserve(ncells)); PT_CUDA(fidx1.reserve(ncells));
-        PT_CUDA(flab0.reserve(ncells)); PT_CUDA(flab1.reserve(ncells));
-        PT_CUDA(emask.reserve(ncells));
+        if (!fused) PT_CUDA(claim.reserve(ncells));
+        PT_CUDA(fidx0.reserve(ncells + 4)); PT_CUDA(fidx1.reserve(ncells + 4));
+        PT_CUDA(flab0.reserve(ncells + 4)); PT_CUDA(flab1.reserve(ncells + 4));
+        PT_CUDA(emask0.reserve(ncells + 4)); PT_CUDA(emask1.reserve(ncells + 4));
     }
     PT_CUDA(ctot.reserve(grid));
     PT_CUDA(seed_n.reserve(1));
@@ -363,16 +458,16 @@ pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *de
     PT_CUDA(status.reserve(4));
     PT_CUDA(cudaMemsetAsync(bar.p, 0, 2 * sizeof(unsigned), st));
     PT_CUDA(cudaMemsetAsync(status.p, 0, 4 * sizeof(int), st));
-    a.claim = claim.p;
+    a.claim = fused ? a.table : claim.p;
     a.fidx[0] = fidx0.p; a.fidx[1] = fidx1.p;
     a.flab[0] = flab0.p; a.flab[1] = flab1.p;
-    a.emask = emask.p;
+    a.emask[0] = emask0.p; a.emask[1] = emask1.p;
     a.ctot = ctot.p;
     a.bar = bar.p;
     a.status = status.p;
     a.seeded = seed_n.p;
     void *args[] = {&a};
-    PT_CUDA(cudaLaunchCooperativeKernel((const void *) k_table_build, grid, NT, args, 0, st));
+    PT_CUDA(cudaLaunchCooperativeKernel(kernel, grid, NT, args, 0, st));
     PT_LAUNCHED();
     int hs[4] = {0, 0, 0, 0};
     long long hn = 0;

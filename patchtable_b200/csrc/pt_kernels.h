@@ -77,11 +77,11 @@ pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, i
                                      const PtBins &bins, const int *to_bin, const int *table, int *tcand, int trow0,
                                      int trows, cudaStream_t st);
 /* k_table_build.cu: the table's cells in one cooperative launch -- fill with TABLE_UNUSED, populate in
-   shuffle-rank order (rank[p] < 0: patch not allowed; order_xy[rank] = packed position), the
+   shuffle-rank order (order_xy[rank] = packed position of the np allowed patches, ew per row), the
    propagation DT when run_dt (at most dt_iters levels when > 0), and fill_zeros with vfill when
    asked.  *seeded receives table_add_count, *levels the DT levels run.  Grid-barrier waits give up
    after pt_spin_limit() polls and the call returns PT_TIMEOUT. */
-pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *desc, int ds, long long P, const int *rank,
+pt_status pt_build_cells(const PtBins &bins, const int *nslices, const float *desc, int ds, int ew, long long np,
                          const int *to_bin, const int *order_xy, int *table, long long ncells, int run_dt, int dt_iters,
                          int fill_zeros, int vfill, long long *seeded, int *levels, cudaStream_t st);
 /* dt_algo 4 downsample, 5 hybrid (prop1 + downsample + unmask), 6 euclidean on a table whose

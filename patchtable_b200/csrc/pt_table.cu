@@ -487,7 +487,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     };
     /* Populate in std::random_shuffle order (patchtable.h:3142-3154): the permutation is drawn
        from the C library rand(), consuming it exactly as the reference does. */
-    std::vector<int> order_xy, rank(P, -1);
+    std::vector<int> order_xy;
     double shuffle_ms = 0.0;
     std::thread shuffler([&] {
         const double t0 = now_s();
@@ -500,10 +500,6 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
                 size_t j = (size_t) (rand() % (int) (i + 1));
                 if (i != j) std::swap(order_xy[i], order_xy[j]);
             }
-        for (size_t i = 0; i < order_xy.size(); i++) {
-            int v = order_xy[i];
-            rank[(size_t) (pt_y(v) - 7) * t->ew + (pt_x(v) - 7)] = (int) i;
-        }
         shuffle_ms = 1000.0 * (now_s() - t0);
     });
     /* set_min_max + set_nslices (patchtable.h:1758-1810, 2567-2582), then the partition */
@@ -561,12 +557,10 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     t->build_ms[PT_BUILD_SHUFFLE] = shuffle_ms;
     if (order_xy.empty()) return pt_fail(PT_BAD_ARG, "no allowed patches");
     {
-        DevBuf<int> d_rank(t->st), d_order(t->st);
-        PT_CUDA(d_rank.reserve(P));
+        DevBuf<int> d_order(t->st);
         PT_CUDA(d_order.reserve(order_xy.size()));
-        PT_CUDA(cudaMemcpyAsync(d_rank.p, rank.data(), sizeof(int) * P, cudaMemcpyHostToDevice, t->st));
         PT_CUDA(cudaMemcpyAsync(d_order.p, order_xy.data(), sizeof(int) * order_xy.size(), cudaMemcpyHostToDevice, t->st));
-        PT_CUDA(t->table.reserve(t->ncells));
+        PT_CUDA(t->table.reserve(t->ncells + 4));       /* the build reads four cells at a time */
         /* Distance transform (patchtable.h:3254-3298): prop is the level-synchronous fill inside
            the cooperative build launch; the others run on its resolved table. */
         const bool prop = p.run_dt && p.dt_algo == 1;
@@ -576,9 +570,9 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         if (!allowed_h.empty())
             for (long long i = 0; i < P; i++)
                 if (allowed_h[i] == p.allowed_index) { vfill = pt_xy((int) (i % t->ew) + 7, (int) (i / t->ew) + 7); break; }
-        PT_TRY(pt_build_cells(t->bins, t->nslices.data(), t->b_desc.p, t->ds, P, d_rank.p, t->to_bin.p, d_order.p,
-                              t->table.p, t->ncells, prop, p.dt_iters, fill_zeros, vfill, &t->add_count, &t->dt_levels,
-                              t->st));
+        PT_TRY(pt_build_cells(t->bins, t->nslices.data(), t->b_desc.p, t->ds, t->ew, (long long) order_xy.size(),
+                              t->to_bin.p, d_order.p, t->table.p, t->ncells, prop, p.dt_iters, fill_zeros, vfill,
+                              &t->add_count, &t->dt_levels, t->st));
         if (p.run_dt && p.dt_algo == 2)
             PT_TRY(pt_dt_brute(t->table.p, t->G, t->nslices.data(), t->part_dev.p, t->part_ofs, t->b_desc.p, t->ds, P, t->ew,
                                t->st));
