@@ -41,6 +41,7 @@ struct QPlan {
     int step;                /* neighbour spacing of this pull pass (jump flooding) */
     int pull_max;            /* most neighbour candidates scored per patch */
     int tile;                /* query patches per CTA (single-image launches) */
+    int auto_tile;           /* no width was asked for */
     int row0, rows;          /* patch rows of a single-image launch */
     const float *brow;       /* row store of the table image (k_row_store) */
     int nline;               /* its lines per image row */
@@ -71,12 +72,17 @@ __device__ __forceinline__ void count_work(unsigned long long *counters, unsigne
     if ((threadIdx.x & 31) == 0) { atomicAdd(counters, (unsigned long long) c); atomicAdd(counters + 1, (unsigned long long) r); }
 }
 
-/* Threads per SM the register caps leave room for: the kernels wait on gathers from L2, so more
-   resident warps pay until the row buffers spill.  Measured at 1080p, 128 patches per CTA, ms at
-   8 / 12 / 16 / 18 x 64 threads per SM: lean choose 0.236 / 0.185 / 0.166 / 0.165, one-candidate
-   pull 0.299 / 0.231 / 0.201 / 0.199, the default schedule's four general pulls 3.23 / 2.99 / 3.04 /
-   3.36 (2.97 at 14) and chooses 1.02 / 0.94 / 0.88 / 0.96 (0.89 at 14). */
-constexpr int CHOOSE_LANES = 14 * 64, CHOOSE_LEAN_LANES = 20 * 64, PULL_LANES = 14 * 64, PULL_ONE_LANES = 18 * 64;
+/* Threads per SM the register caps leave room for, and the rows a choose keeps in flight.  The kernels
+   wait on gathers from L2: more resident warps pay until the row buffers spill.  Measured at 1080p,
+   128 patches per CTA, in ms: lean choose at 16 / 18 / 20 / 22 x 64 threads per SM 0.152 / 0.154 / 0.150 /
+   0.160, one-candidate pull at 14 / 16 / 18 / 20 0.195 / 0.182 / 0.182 / 0.191, the default schedule's
+   four pulls at 10 / 12 / 14 / 16 2.83 / 2.78 / 2.87 / 2.83, its chooses at 8 / 10 / 12 / 14 0.80 / 0.85 /
+   0.88 / 0.85, and 0.785 at 8 with two rows in flight. */
+constexpr int CHOOSE_LANES = 8 * 64, CHOOSE_LEAN_LANES = 20 * 64, PULL_LANES = 12 * 64, PULL_ONE_LANES = 16 * 64;
+constexpr int CHOOSE_D = 2;
+/* Warps that share one 8 x 4 tile's candidate lists in the pull of a small image, and how many tiles
+   per SM still are one (k_pull_tile's launcher). */
+constexpr int SPLIT_W = 4, SPLIT_D = 4, SPLIT_TILES = 4;
 constexpr int min_ctas(int lanes, int tp) { return lanes / tp < 32 ? lanes / tp : 32; }
 
 /* A CTA covers TP query patches: warps of 8 x 4 patches (8 columns, 4 rows; lane l is the patch
@@ -98,20 +104,25 @@ __host__ __device__ constexpr int cta_h(int tp, bool desc) { return desc ? 1 : t
 /* Shared-memory bytes of a staged query tile of TP patches. */
 constexpr size_t atile_bytes(int tp) { return sizeof(float) * stage_pitch(tp) * stage_rows(tp); }
 
-/* Stages the pixels under a CTA's tile as packed rows, 3 floats per pixel, negated: the scorer
-   adds them to the candidate's pixels (b - a and a - b square to the same bits). */
-template<int TP>
+/* Starts copying the pixels under a CTA's tile into shared memory as packed rows, 3 floats per pixel
+   (zeros beyond the image): asynchronous 4-byte copies, any row is only 4-byte aligned.  The tile may
+   be read after stage_wait and a __syncthreads; what does not need it goes in between. */
+template<int TP, int THREADS = TP>
 __device__ __forceinline__ void stage_a(float *at, const float *__restrict__ a, int aw, int ah, int x0, int y0) {
     constexpr int PITCH = stage_pitch(TP);
     const int left = 3 * (aw - x0);
-    for (int i = threadIdx.x; i < PITCH * stage_rows(TP); i += TP) {
+    for (int i = threadIdx.x; i < PITCH * stage_rows(TP); i += THREADS) {
         const int r = i / PITCH, c = i - r * PITCH;
         const int gy = y0 + r;
-        at[i] = (gy < ah && c < left) ? -__ldg(a + ((size_t) gy * aw + x0) * 3 + c) : 0.f;
+        const bool in = gy < ah && c < left;
+        const float *src = a + (in ? ((size_t) gy * aw + x0) * 3 + c : 0);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                     :: "r"((unsigned) __cvta_generic_to_shared(at + i)), "l"(src), "r"(in ? 4 : 0) : "memory");
     }
 }
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-typedef unsigned long long f32x2;         /* two floats in a register pair (add / mul .f32x2) */
+typedef unsigned long long f32x2;         /* two floats in a register pair (.f32x2 arithmetic) */
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
     f32x2 r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -120,9 +131,10 @@ __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
 __device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+/* a - b, as b * -1 + a: one rounding, the subtraction's bits. */
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
     f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    asm("{\n\t.reg .b64 m;\n\tmov.b64 m, 0xbf800000bf800000;\n\tfma.rn.f32x2 %0, %2, m, %1;\n\t}" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
@@ -164,15 +176,17 @@ __device__ __forceinline__ float quad_total(const float (&acc)[4]) {
    shared memory once for all of them (11 rows instead of 32).
 
    Bound: the L1 data pipe (128 bytes per clock: 256 wavefronts for 32 candidates' lines, 66 for the
-   query rows, 24 for the exchanges) at 82 % of its peak in the general pull, issue slots at 61 %.
+   query rows, 24 for the exchanges) at 83 % of its peak in the general pull, issue slots at 60 %.
    The gather this replaced -- each lane its own candidate's 8 pixels, four 32-byte loads from 32
    different lines, 24 shared loads per row -- spent one wavefront on every lane's load and ran at
-   89 % of the same pipe: at 1080p the lean choose took 0.265 ms (now 0.165), the one-candidate pull
-   0.257 (0.199), the default schedule's pulls 4.01 (2.97).
+   89 % of the same pipe: at 1080p the lean choose took 0.265 ms (now 0.150), the one-candidate pull
+   0.257 (0.182), the default schedule's pulls 4.01 (2.78).
+
+   D rows per candidate are in flight at a time: more registers, fewer waits.
 
    With EXIT a candidate is abandoned (+inf returned) once its partial total reaches `bound`, tested
    after rows 2, 4 and 6 (the total can only grow, so nothing that would be accepted is lost). */
-template<int TP, bool EXIT>
+template<int TP, bool EXIT, int D>
 __device__ __forceinline__ float score32(const QPlan &q, const float *al, int cand, bool valid, float bound, unsigned &rows) {
     constexpr int PITCH = stage_pitch(TP);
     const unsigned FULL = 0xffffffffu;
@@ -200,21 +214,28 @@ __device__ __forceinline__ float score32(const QPlan &q, const float *al, int ca
     for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int n = 0; n < 3; n++) aw[r][n] = pack2(al[r * PITCH + 8 * n], al[r * PITCH + 8 * n + 4]);
+    float u[D][4][8];                     /* the next D rows, on their way or arrived */
+#pragma unroll
+    for (int r = 0; r < D - 1; r++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) { ld8(p[s], u[r][s]); p[s] += pitch; }
 #pragma unroll
     for (int r = 0; r < 8; r++) {
 #pragma unroll
         for (int n = 0; n < 3; n++) aw[(r + 3) & 3][n] = pack2(al[(r + 3) * PITCH + 8 * n], al[(r + 3) * PITCH + 8 * n + 4]);
-        float u[4][8];
+        if (r + D - 1 < 8) {
 #pragma unroll
-        for (int s = 0; s < 4; s++) { ld8(p[s], u[s]); p[s] += pitch; }
+            for (int s = 0; s < 4; s++) { ld8(p[s], u[(r + D - 1) % D][s]); p[s] += pitch; }
+        }
 #pragma unroll
         for (int s = 0; s < 4; s++) {
+            const float (&ur)[8] = u[r % D][s];
             float w[6];
 #pragma unroll
-            for (int n = 0; n < 6; n++) w[n] = off[s] ? u[s][n + 1] : u[s][n];
+            for (int n = 0; n < 6; n++) w[n] = off[s] ? ur[n + 1] : ur[n];
 #pragma unroll
             for (int n = 0; n < 3; n++) {
-                const f32x2 t = add2(pack2(w[2 * n], w[2 * n + 1]), aw[(r + s) & 3][n]);
+                const f32x2 t = sub2(pack2(w[2 * n], w[2 * n + 1]), aw[(r + s) & 3][n]);
                 float lo, hi;
                 unpack2(mul2(t, t), lo, hi);
                 acc[s] = __fadd_rn(__fadd_rn(acc[s], lo), hi);
@@ -237,6 +258,87 @@ __device__ __forceinline__ float score32(const QPlan &q, const float *al, int ca
     return own ? tot : finf();
 }
 
+/* The first eight candidates of `mask` (bit l: lane l's, v its line << 1 | odd column), one per quad:
+   the k-th goes to quad k, which reads the query rows of its lane's patch.  Returns its lane the total
+   (+inf when abandoned at `bound` after row 4); other lanes get no meaningful value. */
+template<int TP, bool EXIT>
+__device__ __forceinline__ float score8(const QPlan &q, const float *al, unsigned mask, unsigned v, float bound) {
+    constexpr int PITCH = stage_pitch(TP);
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, k = lane >> 2, j = lane & 3;
+    unsigned m = mask;
+#pragma unroll
+    for (int i = 0; i < 7; i++)
+        if (k > i) m &= m - 1;
+    const bool on = m != 0;
+    const int src = on ? __ffs(m) - 1 : __ffs(mask) - 1;
+    const unsigned vs = __shfl_sync(FULL, v, src);
+    const int i0 = 3 * (int) (vs & 1) + j;
+    const bool off = i0 >= 4;
+    const float *p = q.brow + (size_t) (vs >> 1) * 32 + (i0 & 3) * 8;
+    const size_t pitch = (size_t) q.nline * 32;
+    /* the address of patch src's first query float for SSE lane j, from this lane's own */
+    const float *as = al + (src & 3) * PITCH + 3 * ((src >> 2) - k);
+    float acc = 0.f, part = 0.f;
+#pragma unroll
+    for (int r0 = 0; r0 < 8; r0 += 4) {
+        float u[4][8];
+#pragma unroll
+        for (int r = 0; r < 4; r++) { ld8(p, u[r]); p += pitch; }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const float *ar = as + (r0 + r) * PITCH;
+#pragma unroll
+            for (int n = 0; n < 3; n++) {
+                const f32x2 w = pack2(off ? u[r][2 * n + 1] : u[r][2 * n], off ? u[r][2 * n + 2] : u[r][2 * n + 1]);
+                const f32x2 t = sub2(w, pack2(ar[8 * n], ar[8 * n + 4]));
+                float lo, hi;
+                unpack2(mul2(t, t), lo, hi);
+                acc = __fadd_rn(__fadd_rn(acc, lo), hi);
+            }
+        }
+        const int qb = lane & ~3;
+        const float l0 = __shfl_sync(FULL, acc, qb), l1 = __shfl_sync(FULL, acc, qb | 1), l2 = __shfl_sync(FULL, acc, qb | 2),
+                    l3 = __shfl_sync(FULL, acc, qb | 3);
+        part = __fadd_rn(__fadd_rn(__fadd_rn(l0, l1), l2), l3);
+        if (EXIT && r0 == 0) {
+            const float b = __shfl_sync(FULL, bound, src);
+            if (!__any_sync(FULL, on && !(part >= b))) { part = finf(); break; }
+        }
+    }
+    return __shfl_sync(FULL, part, 4 * (__popc(mask & ((1u << lane) - 1)) & 7));
+}
+
+/* One candidate's distance per lane, all 32 lanes of the warp together: in one round of 32, or, when
+   at most 16 lanes have one (the ends of candidate lists, the later passes' few new neighbours), in
+   rounds of eight, a candidate per quad: 280 instructions and 160 wavefronts each instead of 1,010 and
+   346.  At 1080p the default schedule's pulls take 2.90 ms with the line at 16, 2.93 at 8 or 24 and
+   3.03 with rounds of 32 only. */
+template<int TP, bool EXIT, int D>
+__device__ __forceinline__ float score_warp(const QPlan &q, const float *al, int cand, bool valid, float bound, unsigned &rows) {
+    const unsigned FULL = 0xffffffffu;
+    unsigned mask = __ballot_sync(FULL, valid);
+    if (!mask) return finf();
+    if (__popc(mask) > 16) return score32<TP, EXIT, D>(q, al, cand, valid, bound, rows);
+    const int lane = threadIdx.x & 31;
+    unsigned v = 0;
+    if (valid) {
+        const unsigned x = (unsigned) pt_x(cand);
+        v = (((unsigned) pt_y(cand) * (unsigned) q.nline + (x >> 1)) << 1) | (x & 1);
+        rows += 8;
+    }
+    float d = finf();
+    while (mask) {
+        const float e = score8<TP, EXIT>(q, al, mask, v, bound);
+        unsigned rest = mask;
+#pragma unroll
+        for (int i = 0; i < 8; i++) rest &= rest - 1;
+        if (((mask & ~rest) >> lane) & 1) d = e;
+        mask = rest;
+    }
+    return d;
+}
+
 /* The query patch a distance is taken from: its staged rows (image mode: the address of the lane's
    first float) or its descriptor in registers (descriptor mode). */
 struct AQuery {
@@ -247,21 +349,21 @@ struct AQuery {
 /* One candidate's distance per lane: patch_dist_exact for the whole warp at once (image mode), or
    patch_dist_approx of the descriptors (descriptor mode, always complete: a complete sum at or
    above the bound is rejected by the caller exactly as an abandoned one). */
-template<int TP, bool DESC, bool EXIT>
+template<int TP, bool DESC, bool EXIT, int D = 1>
 __device__ __forceinline__ float dist32(const AQuery &aq, const QPlan &q, int cand, bool valid, float bound, unsigned &rows) {
     if constexpr (DESC) {
         if (!valid) return finf();
         rows++;
         return pt_desc_dist(aq.v, q.bdesc + ((size_t) pt_y(cand) * q.bew + pt_x(cand)) * q.ds4, q.nd);
     } else {
-        return score32<TP, EXIT>(q, aq.al, cand, valid, bound, rows);
+        return score_warp<TP, EXIT, D>(q, aq.al, cand, valid, bound, rows);
     }
 }
 
 /* This lane's patch of the tile with top-left patch (x0, y0), and its query. */
-template<int TP, bool DESC>
+template<int TP, bool DESC, int WPT = 1>
 __device__ __forceinline__ void tile_lane(const QPlan &q, const float *at, int x0, int y0, int &x, int &y, AQuery &aq) {
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wid = WPT > 1 ? 0 : threadIdx.x >> 5, lane = threadIdx.x & 31;
     if constexpr (DESC) {                 /* a row segment: nothing but the row order is shared */
         x = x0 + threadIdx.x;
         y = y0;
@@ -317,8 +419,6 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
             int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs &la,
             int x0, int y0, int y1) {
     const unsigned FULL = 0xffffffffu;
-    stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
-    __syncthreads();
     AQuery aq;
     int x, y;
     tile_lane<TP, false>(c_q, at, x0, y0, x, y, aq);
@@ -332,12 +432,15 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
     float dbest = (float) ((double) dstore * c_q.prop_scale);
     float dch = dstore;
     auto entry = [&](int v) { return table_entry(c_q, v); };
+    stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
     if constexpr (LEAN) {
         int cand = -1;
         if (live && do_table) {
             cand = entry(tcand[p]);
             if (cand == pt_xy(xb, yb)) cand = -1;
         }
+        stage_wait();
+        __syncthreads();
         const float d = dist32<TP, false, false>(aq, c_q, cand, cand >= 0, dbest, rows);
         if (cand >= 0) {
             ne++;
@@ -378,7 +481,7 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
     const int2 *kp = kcoh;
     int wx = 0, wy = 0, wx0 = 0, wx1 = 0, wy1 = 0, own = 0;
     const size_t np = (size_t) c_q.ew * c_q.eh;
-    for (;;) {
+    for (bool staged = false;;) {
         int cand = -1;
         while (cand < 0 && ph != DONE) {
             if (LEARNED && ph == PROPOSALS) {
@@ -453,8 +556,14 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
                 cand = random_neighbour(c_q, p, xb, yb);
             }
         }
+        if (!staged) {
+            /* later passes find nothing new for most patches: a tile without a candidate ends here */
+            stage_wait();
+            if (!__syncthreads_or(cand >= 0)) break;
+            staged = true;
+        }
         if (!__any_sync(FULL, cand >= 0)) break;
-        const float d = dist32<TP, false, true>(aq, c_q, cand, cand >= 0, dbest, rows);
+        const float d = dist32<TP, false, true, CHOOSE_D>(aq, c_q, cand, cand >= 0, dbest, rows);
         if (cand >= 0) {
             ne++;
             if (d < dbest) {
@@ -571,19 +680,22 @@ k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__res
 /* ONE: a single neighbour candidate per patch (pull_max 1).  The candidate is the one the
    general path would sort first -- among distinct candidates keyed by their first occurrence, the
    smallest key, the earliest on ties -- found in one streaming pass, and it is scored alone. */
-template<int TP, int R, bool DESC, bool ONE>
+template<int TP, int R, bool DESC, bool ONE, int D = 1, int WPT = 1>
 __device__ __forceinline__ void
 pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
           const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos,
           float *nxt_d, unsigned long long *counters, int x0, int y0, int y1) {
     const unsigned FULL = 0xffffffffu;
-    if constexpr (!DESC) {
-        stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
-        __syncthreads();
-    }
+    if constexpr (!DESC) stage_a<TP, TP * WPT>(at, a, c_q.aw, c_q.ah, x0, y0);
+    auto staged = [&]() {
+        if constexpr (!DESC) {
+            stage_wait();
+            __syncthreads();
+        }
+    };
     AQuery aq;
     int x, y;
-    tile_lane<TP, DESC>(c_q, at, x0, y0, x, y, aq);
+    tile_lane<TP, DESC, WPT>(c_q, at, x0, y0, x, y, aq);
     const bool live = x < c_q.ew && y < y1;
     const int p = live ? y * c_q.ew + x : 0;
     if constexpr (DESC) pt_desc_load(c_q.adesc + (size_t) p * c_q.ds4, 4 * c_q.ds4, aq.v);
@@ -634,7 +746,8 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
             const float k = *kp;
             if (k < bestk) { bestk = k; best = c; }   /* the general sort's insertion rule */
         });
-        const float d = dist32<TP, DESC, true>(aq, c_q, best, best >= 0, bd, rows);
+        staged();
+        const float d = dist32<TP, DESC, true, D>(aq, c_q, best, best >= 0, bd, rows);
         if (best >= 0) {
             ne = 1;
             if (d < bd) { bd = d; bpos = best; }
@@ -663,6 +776,7 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
         });
         if (nc > c_q.pull_max) nc = c_q.pull_max;   /* the best-first prefix of the list */
         ne = nc;
+        staged();
         if constexpr (DESC) {
             float d[MAXC];                          /* every candidate's loads in flight at once */
 #pragma unroll
@@ -671,12 +785,38 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
             for (int t = 0; t < MAXC; t++)
                 if (t < nc && d[t] < bd) { bd = d[t]; bpos = cand[t]; }
         } else {
-            for (int t0 = 0; __any_sync(FULL, t0 < nc); t0++) {
-                const int c = cand[0];
-                const float d = dist32<TP, DESC, true>(aq, c_q, c, t0 < nc, bd, rows);
-                if (t0 < nc && d < bd) { bd = d; bpos = c; }
+            /* with WPT warps on the tile, warp w scores candidates w, w + WPT, ... of the list */
+            const int w = WPT > 1 ? threadIdx.x >> 5 : 0;
+            int from = -1;
+            auto next = [&]() {
 #pragma unroll
                 for (int t = 0; t + 1 < MAXC; t++) cand[t] = cand[t + 1];
+            };
+            for (int t = 0; t < w; t++) next();
+            for (int t0 = w; __any_sync(FULL, t0 < nc); t0 += WPT) {
+                const int c = cand[0];
+                const float d = dist32<TP, DESC, true, D>(aq, c_q, c, t0 < nc, bd, rows);
+                if (t0 < nc && d < bd) { bd = d; bpos = c; from = t0; }
+#pragma unroll
+                for (int t = 0; t < WPT; t++) next();
+            }
+            if constexpr (WPT > 1) {
+                /* the smallest distance, the earliest in the list on ties: what one warp going through
+                   the whole list keeps */
+                __shared__ float s_d[WPT][32];
+                __shared__ int s_pos[WPT][32], s_from[WPT][32];
+                const int lane = threadIdx.x & 31;
+                s_d[w][lane] = bd;
+                s_pos[w][lane] = bpos;
+                s_from[w][lane] = from;
+                __syncthreads();
+                if (w > 0) { count_work(counters, 0, rows); return; }
+#pragma unroll
+                for (int v = 1; v < WPT; v++) {
+                    const int f = s_from[v][lane];
+                    const float d = s_d[v][lane];
+                    if (f >= 0 && (d < bd || (d == bd && from >= 0 && f < from))) { bd = d; bpos = s_pos[v][lane]; from = f; }
+                }
             }
         }
     }
@@ -694,13 +834,13 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
     count_work(counters, ne, rows);
 }
 
-template<int TP, int R, bool DESC, bool ONE = false>
-__global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES, TP))
+template<int TP, int R, bool DESC, bool ONE = false, int D = 1, int WPT = 1>
+__global__ void __launch_bounds__(TP * WPT, min_ctas(WPT > 1 ? 2 * TP * WPT : ONE ? PULL_ONE_LANES : PULL_LANES, TP * WPT))
 k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
             const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
             int *nxt_pos, float *nxt_d, unsigned long long *counters) {
     extern __shared__ float at[];
-    pull_tile<TP, R, DESC, ONE>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
+    pull_tile<TP, R, DESC, ONE, D, WPT>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
                                 blockIdx.x * cta_w(TP, DESC), blockIdx.y * cta_h(TP, DESC) + c_q.row0, c_q.row0 + c_q.rows);
 }
 
@@ -826,6 +966,7 @@ k_init_temporal(const QPlan q, const double *__restrict__ prev, const float *__r
     if constexpr (!DESC) {
         if (recalc) {
             stage_a<TP>(at, a, q.aw, q.ah, x0, y0);
+            stage_wait();
             __syncthreads();
         }
     }
@@ -869,6 +1010,7 @@ k_init_random(const QPlan q, const float *__restrict__ a, int *cur_pos, float *c
     const int x0 = blockIdx.x * cta_w(TP, DESC), y0 = blockIdx.y * cta_h(TP, DESC);
     if constexpr (!DESC) {
         stage_a<TP>(at, a, q.aw, q.ah, x0, y0);
+        stage_wait();
         __syncthreads();
     }
     AQuery aq;
@@ -942,6 +1084,19 @@ bool one_pull(const QPlan &q) { return g_lean_kernels.load(std::memory_order_rel
 
 extern "C" int pt_set_lean_kernels(int on) { return g_lean_kernels.exchange(on ? 1 : 0); }
 
+/* SMs of the current device, asked once. */
+static int sm_count() {
+    static std::atomic<int> n{0};
+    int v = n.load(std::memory_order_relaxed);
+    if (!v) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) v = 148;
+        n.store(v, std::memory_order_relaxed);
+    }
+    return v;
+}
+
 static dim3 tile_grid(const QPlan &q, int tp) {
     const int w = cta_w(tp, q.adesc != nullptr), h = cta_h(tp, q.adesc != nullptr);
     return dim3((q.ew + w - 1) / w, (q.rows + h - 1) / h);
@@ -961,6 +1116,7 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     q.step = s.step < 1 ? 1 : s.step;
     q.pull_max = s.pull_max > 0 ? s.pull_max : 1 << 30;
     q.tile = s.tile > 0 ? s.tile : TILE_DEFAULT;
+    q.auto_tile = s.tile <= 0;
     q.row0 = s.rows > 0 ? s.row0 : 0;
     q.rows = s.rows > 0 ? s.rows : q.eh;
     if (s.rows > 0 && (q.row0 < 0 || q.row0 + q.rows > q.eh))
@@ -1091,6 +1247,21 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *
         else k_pull_tile<T, RR, false><<<grid, T, atile_bytes(T), st>>>( \
             q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); }
     const bool one = one_pull(q);
+    /* Small images leave most of the chip idle and wait for one warp's rounds of candidates: four
+       warps share a tile's list.  The four pulls of the default schedule, in us: 48 x 64 98 -> 58,
+       100 x 150 (2.8 tiles per SM) 119 -> 66, 140 x 200 (5.4) 124 -> 107, 180 x 260 (9.2) 137 -> 159. */
+    const dim3 tiles = tile_grid(q, 32);
+    if (q.auto_tile && !one && (long long) tiles.x * tiles.y <= (long long) SPLIT_TILES * sm_count()) {
+        constexpr int T = 32;
+        if (r1)
+            k_pull_tile<T, 1, false, false, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
+                q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+        else
+            k_pull_tile<T, 2, false, false, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
+                q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+        PT_LAUNCHED();
+        return PT_OK;
+    }
     switch (q.tile) {
         case 32: if (r1) PT_PULL_T(32, 1) else PT_PULL_T(32, 2) break;
         case 64: if (r1) PT_PULL_T(64, 1) else PT_PULL_T(64, 2) break;
@@ -1123,15 +1294,9 @@ constexpr int BATCH_TW[PT_BATCH_NTW] = {32, 64, 128, 256};
 
 template<class K>
 int persistent_grid(K kernel, int threads, size_t smem, long long work) {
-    static int nsm = 0;
-    if (!nsm) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    }
     int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess || per < 1) per = 1;
-    const long long g = (long long) per * nsm;
+    const long long g = (long long) per * sm_count();
     return (int) (work < g ? work : g);
 }
 
