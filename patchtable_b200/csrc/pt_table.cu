@@ -825,38 +825,14 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
    the same sequence as a recorded CUDA graph measured slower (1.45 against 1.29 ms at 1080p).
    Device-resident lookups keep the whole-image launches: the same bands on three streams without
    copies measured 1.10 against 0.98 ms. */
-int band_rows(const pt_table *t, int h, int w) {
-    const pt_params &p = t->p;
-    const int eh = h - 7, ew = w - 7;
-    int B = 0;
-    if (p.gpu_bands <= 0) {
-        /* Default: the band's choose launch fills whole waves.  A choose CTA of tw patches is
-           resident about 10 * 64 / tw times per SM, so one wave covers sms * 640 / (tw * segments)
-           patch rows; B is the largest multiple of 8 rows within k waves, for the smallest k giving at
-           least 32 rows and at most 24 bands (measured e2e: 720p 9 bands 0.71 ms, 1080p 20 bands
-           of 56 rows = 0.95 wave 1.35 ms against 1.41 at 16 bands of 1.22 waves, 1440p 17 bands).
-           Fewer than 8 bands would lose the overlap: then about 16 bands. */
-        static int sms = 0;
-        if (!sms) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (sms < 1) sms = 148;
-        }
-        const int tw = (p.gpu_tile == 64 || p.gpu_tile == 128 || p.gpu_tile == 256) ? p.gpu_tile : 32;
-        const double rows_wave = (double) sms * (10 * 64 / tw) / ((ew + tw - 1) / tw);
-        for (int k = 1; k <= 64; k++) {
-            B = (int) (k * rows_wave / 8) * 8;
-            if (B >= 32 && (eh + B - 1) / B <= 24) break;
-        }
-        if (B < 32 || (eh + B - 1) / B < 8 || (eh + B - 1) / B > 24) B = 0;
-    }
-    if (B == 0) {
-        const int want = p.gpu_bands > 0 ? p.gpu_bands : 16;
-        B = ((eh + want - 1) / want + 7) / 8 * 8;       /* about `want` bands, each a multiple of 8 rows */
-        if (B < 32) B = 32;
-    }
-    return B;
+int band_rows(const pt_table *t, int h) {
+    /* Default: at most 11 bands, of at least 60 rows.  Fewer bands leave more work after the last upload,
+       more cost launches and small copies; measured end to end, ms at 6 / 8 / 10 / 12 / 16 / 20 bands:
+       1080p 1.40 / 1.31 / 1.26 / 1.25 / 1.29 / 1.34, 720p 0.89 / 0.80 / 0.79 / 0.82 / 0.83 / 0.83, 360p
+       0.28 / 0.30 / 0.32 / 0.36 / 0.36 / 0.34. */
+    const int eh = h - 7;
+    const int want = t->p.gpu_bands > 0 ? t->p.gpu_bands : std::max(1, std::min(11, eh / 60));
+    return std::max(32, ((eh + want - 1) / want + 7) / 8 * 8);       /* a multiple of 8 rows */
 }
 
 /* Enqueues the band pipeline on the table's streams, starting after the work queued on t->st and
@@ -1001,7 +977,7 @@ pt_status lookup_banded(pt_table *t, const float *a, int h, int w, double *ann_o
     PT_TRY(ensure_query_buffers(t, h, w));
     for (cudaStream_t *sp : {&t->st_in, &t->st_out, &t->st_choose, &t->st_pull})
         if (!*sp) PT_CUDA(cudaStreamCreateWithFlags(sp, cudaStreamNonBlocking));
-    const std::vector<int> edge = band_edges(eh, band_rows(t, h, w));
+    const std::vector<int> edge = band_edges(eh, band_rows(t, h));
     const int nb = (int) edge.size() - 1;
     while ((int) t->band_ev.size() < 5 * nb + 6) {
         cudaEvent_t e;
