@@ -217,16 +217,17 @@ __device__ __forceinline__ void desc_tile(const DescPlan &c_plan, float *smem, c
     }
 }
 
-/* Four CTAs per SM (64 registers; shared memory sized to the plan's filters): the kernel is
-   issue-bound and the extra warps fill the barrier gaps (0.105 -> 0.093 ms at 1080p). */
-__global__ void __launch_bounds__(NT, 4)
+/* Five CTAs per SM (48 registers; shared memory sized to the plan's filters): the kernel is
+   issue-bound and the extra warps fill the barrier gaps (1080p query pass: 0.088 ms at four CTAs,
+   0.081 at five, 0.104 at six, which spills). */
+__global__ void __launch_bounds__(NT, 5)
 k_descriptor(const DescPlan c_plan, const float *__restrict__ rgb, int h, int w, int convert,
              float4 *__restrict__ rgba, float *__restrict__ desc, int ds, int eh, int ew, int ty0) {
     extern __shared__ __align__(16) float smem[];
     desc_tile(c_plan, smem, rgb, h, w, convert, rgba, desc, ds, eh, ew, blockIdx.x * TW, (blockIdx.y + ty0) * TH);
 }
 
-__global__ void __launch_bounds__(NT, 4)
+__global__ void __launch_bounds__(NT, 5)
 k_descriptor_cells(const DescPlan c_plan, const CellPlan cp, const float *__restrict__ rgb, int h, int w, int convert,
                    float4 *__restrict__ rgba, int eh, int ew, int ty0) {
     extern __shared__ __align__(16) float smem[];
@@ -238,7 +239,7 @@ k_descriptor_cells(const DescPlan c_plan, const CellPlan cp, const float *__rest
    copies and descriptors concatenated), the tiles handed out by a work counter; with CELLS the
    table entries of the patches' cells are written instead of the descriptors. */
 template<bool CELLS>
-__global__ void __launch_bounds__(NT, 4)
+__global__ void __launch_bounds__(NT, 5)
 k_descriptor_batch(const DescPlan c_plan, const CellPlan cp, const PtBatchImage *__restrict__ imgs, int n, long long ntiles,
                    const float *__restrict__ rgb, int convert, float4 *__restrict__ rgba, float *__restrict__ desc, int ds,
                    unsigned long long *work) {

@@ -27,7 +27,18 @@ namespace {
 
 constexpr int NT = 256;
 
+/* The next pass's choose, done by the pull for the match it has just found (ch_pos NULL: none). */
+struct NextChoose {
+    const int2 *kcoh;
+    int *kc_done;
+    int use_done, do_kcoh, pass;
+    int *ch_pos;
+    float *ch_d;
+    unsigned long long *counters;
+};
+
 struct QPlan {
+    NextChoose nx;
     int aw, ah;              /* a image size (pixels) */
     int ew, eh;              /* a patches */
     int bw, bh;              /* b image size */
@@ -387,8 +398,8 @@ __device__ __forceinline__ int table_entry(const QPlan &q, int v) {
 /* Random search (patchtable.h:3874-3903): one of the 8 neighbours of the best match, -1 when it lies
    outside b or is not allowed.  dx, dy + 1 for r = 0..7 are packed two bits each:
    {-1,0,1,-1,1,-1,0,1}, {-1,-1,-1,0,0,1,1,1}. */
-__device__ __forceinline__ int random_neighbour(const QPlan &q, int p, int xb, int yb) {
-    const unsigned r = mix32((unsigned) p * 2654435761u + (unsigned) q.pass * 0x9e3779b9u + 0x6a09e667u) & 7u;
+__device__ __forceinline__ int random_neighbour(const QPlan &q, int pass, int p, int xb, int yb) {
+    const unsigned r = mix32((unsigned) p * 2654435761u + (unsigned) pass * 0x9e3779b9u + 0x6a09e667u) & 7u;
     const int xs = xb + (int) ((37412u >> (2 * r)) & 3u) - 1, ys = yb + (int) ((43328u >> (2 * r)) & 3u) - 1;
     if (xs < 0 || xs >= q.bew || ys < 0 || ys >= q.beh) return -1;
     if (q.allowed && __ldg(q.allowed + (size_t) ys * q.bew + xs) != q.allowed_index) return -1;
@@ -402,6 +413,112 @@ struct LearnedArgs {
     float threshold;          /* patches below it keep the plain candidates */
     int kcoh_confident;       /* confident patches also try k-coherence */
     unsigned long long *counters;   /* [confident patches, proposals scored] or NULL */
+};
+
+/* A lane's walk through its patch's candidates in the reference's order: the table entries (TABLES),
+   k-coherence neighbours, then spatial or random search (patchtable.h:3641-3903). */
+template<bool TABLES>
+struct Walk {
+    enum { TABLE, ENTER, KCOH, WINDOW, RANDOM, DONE };
+    int ph, it;
+    int best;                             /* best match so far */
+    float dbest, dch;                     /* the distance to beat, and the distance of the choice */
+    int kc_src, kdx, kdy;
+    bool repeat, accepted;
+    const int2 *kp;
+    int wx, wy, wx0, wx1, wy1, own;
+
+    int prev;                             /* the previous table's entry */
+
+    __device__ __forceinline__ void start(const QPlan &q, bool live, int pos, float dstore) {
+        ph = live ? (TABLES ? TABLE : ENTER) : DONE;
+        it = prev = 0;
+        best = pos;
+        dbest = (float) ((double) dstore * q.prop_scale);
+        dch = dstore;
+        repeat = accepted = false;
+        kdx = kdy = 0;
+    }
+    __device__ __forceinline__ void offer(int c, float d) {
+        if (d < dbest) {
+            dbest = dch = d;
+            best = c;
+            if (ph == KCOH) accepted = true;
+        }
+    }
+    __device__ __forceinline__ bool inside(const QPlan &q) const { return pt_x(best) < q.bew && pt_y(best) < q.beh; }
+
+    /* The next candidate, or -1 when the walk has ended. */
+    __device__ __forceinline__ int next(const QPlan &q, const int2 *__restrict__ kcoh, int *kc_done, int use_done,
+                                        int do_kcoh, int pass, bool kc_here, int p, bool table = false,
+                                        const int *__restrict__ tcand = nullptr) {
+        int c = -1;
+        while (c < 0 && ph != DONE) {
+            if (TABLES && ph == TABLE) {
+                /* the first table's entry, then the further tables' (patchtable.h:3711-3735): each is
+                   scored unless it equals the best so far or the previous table's entry */
+                if (!table || it > q.ntc) { ph = ENTER; continue; }
+                const int v = it == 0 ? tcand[p] : q.tcand_more[(size_t) (it - 1) * q.ew * q.eh + p];
+                const int e = table_entry(q, v);
+                if (e >= 0 && e != best && (it == 0 || v != prev)) c = e;
+                prev = v;
+                it++;
+            } else if (ph == ENTER) {
+                ph = KCOH;
+                kc_src = best;
+                it = q.kc_try;            /* nothing to try, unless: */
+                if (do_kcoh) {
+                    repeat = use_done && kc_done[p] == kc_src;
+                    if (kc_here && !repeat && inside(q)) {
+                        const int ks = q.ks, xb = pt_x(best), yb = pt_y(best);
+                        kp = kcoh + ((size_t) (yb / ks) * q.bew + (xb / ks)) * q.kc;
+                        if (ks > 1) { kdx = xb % ks; kdy = yb % ks; }
+                        it = 0;
+                    }
+                }
+            } else if (ph == KCOH) {
+                /* the reference tries the list in order and stops at the first neighbour whose
+                   stored distance reaches triangle * best */
+                int2 e = make_int2(0, 0);
+                bool go = it < q.kc_try;
+                if (go) {
+                    e = kp[it++];
+                    go = (double) __int_as_float(e.y) < q.triangle * (double) dbest;
+                }
+                if (go) {
+                    c = pt_xy(min(pt_x(e.x) + kdx, q.bew - 1), min(pt_y(e.x) + kdy, q.beh - 1));
+                    continue;
+                }
+                ph = DONE;
+                if (do_kcoh) kc_done[p] = (repeat || !accepted) ? kc_src : -1;
+                if (inside(q)) {
+                    if (q.spatial > 0) {
+                        /* Spatial search (patchtable.h:3855-3873): every other patch of the (2s+1)^2
+                           window around the best match, rows then columns. */
+                        const int S = q.spatial, xb = pt_x(best), yb = pt_y(best);
+                        ph = WINDOW;
+                        own = best;
+                        wy = max(yb - S, 0);
+                        wy1 = min(yb + S + 1, q.beh);
+                        wx0 = max(xb - S, 0);
+                        wx1 = min(xb + S + 1, q.bew);
+                        wx = wx0;
+                    } else if (q.do_rs) {
+                        ph = RANDOM;
+                    }
+                }
+            } else if (ph == WINDOW) {
+                if (wy >= wy1) { ph = DONE; continue; }
+                const int e = pt_xy(wx, wy);
+                if (e != own && (!q.allowed || __ldg(q.allowed + (size_t) wy * q.bew + wx) == q.allowed_index)) c = e;
+                if (++wx >= wx1) { wx = wx0; wy++; }
+            } else {
+                ph = DONE;
+                c = random_neighbour(q, pass, p, pt_x(best), pt_y(best));
+            }
+        }
+        return c;
+    }
 };
 
 /* Steps 1-3 for every patch ("choose"): the chosen match and its exact distance.  Each lane walks
@@ -428,26 +545,21 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
     /* no state arrays: the initial field, x = b's ew + 1 and DIST_INFINITY (patchtable.h:3538-3547) */
     const int pos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);
     const float dstore = cur_d ? cur_d[p] : (float) PT_DIST_INF;
-    int xb = pt_x(pos), yb = pt_y(pos);
-    float dbest = (float) ((double) dstore * c_q.prop_scale);
-    float dch = dstore;
     auto entry = [&](int v) { return table_entry(c_q, v); };
     stage_a<TP>(at, a, c_q.aw, c_q.ah, x0, y0);
     if constexpr (LEAN) {
         int cand = -1;
         if (live && do_table) {
             cand = entry(tcand[p]);
-            if (cand == pt_xy(xb, yb)) cand = -1;
+            if (cand == pos) cand = -1;
         }
         stage_wait();
         __syncthreads();
+        const float dbest = (float) ((double) dstore * c_q.prop_scale);
         const float d = dist32<TP, false, false>(aq, c_q, cand, cand >= 0, dbest, rows);
-        if (cand >= 0) {
-            ne++;
-            if (d < dbest) { dch = d; xb = pt_x(cand); yb = pt_y(cand); }
-        }
-        if (live) { ch_pos[p] = pt_xy(xb, yb); ch_d[p] = dch; }
-        count_work(counters, ne, rows);
+        const bool take = cand >= 0 && d < dbest;
+        if (live) { ch_pos[p] = take ? cand : pos; ch_d[p] = take ? d : dstore; }
+        count_work(counters, cand >= 0, rows);
         return;
     }
     bool confident = false;
@@ -462,7 +574,7 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
 #pragma unroll
             for (int j = 0; j < PT_PROP_TOPK; j++) {
                 cand[j] = raw[j] >= 0 ? entry(raw[j]) : -1;
-                bool dup = cand[j] < 0 || cand[j] == pt_xy(xb, yb);
+                bool dup = cand[j] < 0 || cand[j] == pos;
 #pragma unroll
                 for (int t = 0; t < j; t++) dup |= ((keep >> t) & 1) && cand[t] == cand[j];
                 if (!dup) keep |= 1u << j;
@@ -472,90 +584,17 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
         }
     }
     const bool table = do_table && !(LEARNED && confident && la.cand);
-    enum { PROPOSALS, TABLES, KCOH, WINDOW, RANDOM, DONE };
-    int ph = live ? (LEARNED ? PROPOSALS : TABLES) : DONE;
-    int it = 0;
-    int xs1 = 0, ys1 = 0;                 /* the previous table's entry */
-    int kc_src = 0, kdx = 0, kdy = 0;
-    bool repeat = false, accepted = false;
-    const int2 *kp = kcoh;
-    int wx = 0, wy = 0, wx0 = 0, wx1 = 0, wy1 = 0, own = 0;
-    const size_t np = (size_t) c_q.ew * c_q.eh;
+    const bool kc_here = !LEARNED || !confident || la.kcoh_confident;
+    Walk<true> w;
+    w.start(c_q, live, pos, dstore);
     for (bool staged = false;;) {
         int cand = -1;
-        while (cand < 0 && ph != DONE) {
-            if (LEARNED && ph == PROPOSALS) {
-                if (!keep) { ph = TABLES; continue; }
-                const int j = __ffs(keep) - 1;
-                keep &= keep - 1;
-                cand = entry(la.cand[(size_t) p * PT_PROP_TOPK + j]);
-            } else if (ph == TABLES) {
-                /* the first table's entry, then the further tables' (patchtable.h:3711-3735): each is
-                   scored unless it equals the best so far or the previous table's entry */
-                if (!table || it > c_q.ntc) {
-                    ph = KCOH;
-                    it = 0;
-                    kc_src = pt_xy(xb, yb);
-                    if (c_q.do_kcoh) {
-                        repeat = use_done && kc_done[p] == kc_src;
-                        if ((!LEARNED || !confident || la.kcoh_confident) && !repeat && xb < c_q.bew && yb < c_q.beh) {
-                            const int ks = c_q.ks;
-                            kp = kcoh + ((size_t) (yb / ks) * c_q.bew + (xb / ks)) * c_q.kc;
-                            if (ks > 1) { kdx = xb % ks; kdy = yb % ks; }
-                            continue;
-                        }
-                    }
-                    it = c_q.kc_try;      /* nothing to try */
-                    continue;
-                }
-                const int v = it == 0 ? tcand[p] : c_q.tcand_more[(size_t) (it - 1) * np + p];
-                const int xs = pt_x(v) - 7, ys = pt_y(v) - 7;
-                const int e = entry(v);
-                if (e >= 0 && e != pt_xy(xb, yb) && (it == 0 || xs != xs1 || ys != ys1)) cand = e;
-                xs1 = xs;
-                ys1 = ys;
-                it++;
-            } else if (ph == KCOH) {
-                /* the reference tries the list in order and stops at the first neighbour whose
-                   stored distance reaches triangle * best */
-                int2 e = make_int2(0, 0);
-                bool go = it < c_q.kc_try;
-                if (go) {
-                    e = kp[it++];
-                    go = (double) __int_as_float(e.y) < c_q.triangle * (double) dbest;
-                }
-                if (go) {
-                    cand = pt_xy(min(pt_x(e.x) + kdx, c_q.bew - 1), min(pt_y(e.x) + kdy, c_q.beh - 1));
-                    continue;
-                }
-                ph = DONE;
-                if (c_q.do_kcoh) kc_done[p] = (repeat || !accepted) ? kc_src : -1;
-                if (xb < c_q.bew && yb < c_q.beh) {
-                    if (c_q.spatial > 0) {
-                        /* Spatial search (patchtable.h:3855-3873): every other patch of the (2s+1)^2
-                           window around the best match, rows then columns. */
-                        const int S = c_q.spatial;
-                        ph = WINDOW;
-                        own = pt_xy(xb, yb);
-                        wy = max(yb - S, 0);
-                        wy1 = min(yb + S + 1, c_q.beh);
-                        wx0 = max(xb - S, 0);
-                        wx1 = min(xb + S + 1, c_q.bew);
-                        wx = wx0;
-                    } else if (c_q.do_rs) {
-                        ph = RANDOM;
-                    }
-                }
-            } else if (ph == WINDOW) {
-                if (wy >= wy1) { ph = DONE; continue; }
-                const int e = pt_xy(wx, wy);
-                if (e != own && (!c_q.allowed || __ldg(c_q.allowed + (size_t) wy * c_q.bew + wx) == c_q.allowed_index)) cand = e;
-                if (++wx >= wx1) { wx = wx0; wy++; }
-            } else {
-                ph = DONE;
-                cand = random_neighbour(c_q, p, xb, yb);
-            }
+        if (LEARNED && keep) {
+            const int j = __ffs(keep) - 1;
+            keep &= keep - 1;
+            cand = entry(la.cand[(size_t) p * PT_PROP_TOPK + j]);
         }
+        if (cand < 0) cand = w.next(c_q, kcoh, kc_done, use_done, c_q.do_kcoh, c_q.pass, kc_here, p, table, tcand);
         if (!staged) {
             /* later passes find nothing new for most patches: a tile without a candidate ends here */
             stage_wait();
@@ -563,18 +602,13 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
             staged = true;
         }
         if (!__any_sync(FULL, cand >= 0)) break;
-        const float d = dist32<TP, false, true, CHOOSE_D>(aq, c_q, cand, cand >= 0, dbest, rows);
+        const float d = dist32<TP, false, true, CHOOSE_D>(aq, c_q, cand, cand >= 0, w.dbest, rows);
         if (cand >= 0) {
             ne++;
-            if (d < dbest) {
-                dbest = dch = d;
-                xb = pt_x(cand);
-                yb = pt_y(cand);
-                if (ph == KCOH) accepted = true;
-            }
+            w.offer(cand, d);
         }
     }
-    if (live) { ch_pos[p] = pt_xy(xb, yb); ch_d[p] = dch; }
+    if (live) { ch_pos[p] = w.best; ch_d[p] = w.dch; }
     count_work(counters, ne, rows);
     if (LEARNED && la.counters) {
         unsigned c = __reduce_add_sync(FULL, n_conf), n = __reduce_add_sync(FULL, n_prop);
@@ -660,7 +694,7 @@ k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__res
                         offer(pt_xy(xs, ys), dist(pt_xy(xs, ys)));
                     }
             } else if (q.do_rs) {
-                const int c = random_neighbour(q, p, xb, yb);
+                const int c = random_neighbour(q, q.pass, p, xb, yb);
                 if (c >= 0) offer(c, dist(c));
             }
         }
@@ -680,24 +714,38 @@ k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__res
 /* ONE: a single neighbour candidate per patch (pull_max 1).  The candidate is the one the
    general path would sort first -- among distinct candidates keyed by their first occurrence, the
    smallest key, the earliest on ties -- found in one streaming pass, and it is scored alone. */
-template<int TP, int R, bool DESC, bool ONE, int D = 1, int WPT = 1>
+/* NX: also the next pass's choose (c_q.nx) where asked for; without it the general pull's registers
+   are its own (-speed 1 at 540 x 960: 1.675 ms, 1.714 with the code in the kernel but unused). */
+template<int TP, int R, bool DESC, bool ONE, bool NX, int D = 1, int WPT = 1>
 __device__ __forceinline__ void
 pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
           const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos,
           float *nxt_d, unsigned long long *counters, int x0, int y0, int y1) {
     const unsigned FULL = 0xffffffffu;
     if constexpr (!DESC) stage_a<TP, TP * WPT>(at, a, c_q.aw, c_q.ah, x0, y0);
+    AQuery aq;
+    int x, y;
+    tile_lane<TP, DESC, WPT>(c_q, at, x0, y0, x, y, aq);
+    const bool live = x < c_q.ew && y < y1;
+    const int p = live ? y * c_q.ew + x : 0;
+    /* the match found: the next pass's state, or the float64 NNF of the final field (k_output fused) */
+    auto finish = [&](int pos, float d) {
+        if (c_q.ann) {
+            double *o = c_q.ann + 3 * (size_t) p;
+            o[0] = pt_x(pos);
+            o[1] = pt_y(pos);
+            o[2] = d;
+        } else {
+            nxt_pos[p] = pos;
+            nxt_d[p] = d;
+        }
+    };
     auto staged = [&]() {
         if constexpr (!DESC) {
             stage_wait();
             __syncthreads();
         }
     };
-    AQuery aq;
-    int x, y;
-    tile_lane<TP, DESC, WPT>(c_q, at, x0, y0, x, y, aq);
-    const bool live = x < c_q.ew && y < y1;
-    const int p = live ? y * c_q.ew + x : 0;
     if constexpr (DESC) pt_desc_load(c_q.adesc + (size_t) p * c_q.ds4, 4 * c_q.ds4, aq.v);
     unsigned ne = 0, rows = 0;
     int bpos = cur_pos ? cur_pos[p] : pt_xy(c_q.bew + 1, 0);      /* null: the initial field */
@@ -785,20 +833,20 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
             for (int t = 0; t < MAXC; t++)
                 if (t < nc && d[t] < bd) { bd = d[t]; bpos = cand[t]; }
         } else {
-            /* with WPT warps on the tile, warp w scores candidates w, w + WPT, ... of the list */
-            const int w = WPT > 1 ? threadIdx.x >> 5 : 0;
-            int from = -1;
-            auto next = [&]() {
+            auto shift = [&]() {
 #pragma unroll
                 for (int t = 0; t + 1 < MAXC; t++) cand[t] = cand[t + 1];
             };
-            for (int t = 0; t < w; t++) next();
-            for (int t0 = w; __any_sync(FULL, t0 < nc); t0 += WPT) {
+            /* with WPT warps on the tile, warp v scores candidates v, v + WPT, ... of the list */
+            const int v = WPT > 1 ? threadIdx.x >> 5 : 0;
+            int from = -1;
+            for (int t = 0; t < v; t++) shift();
+            for (int t0 = v; __any_sync(FULL, t0 < nc); t0 += WPT) {
                 const int c = cand[0];
                 const float d = dist32<TP, DESC, true, D>(aq, c_q, c, t0 < nc, bd, rows);
                 if (t0 < nc && d < bd) { bd = d; bpos = c; from = t0; }
 #pragma unroll
-                for (int t = 0; t < WPT; t++) next();
+                for (int t = 0; t < WPT; t++) shift();
             }
             if constexpr (WPT > 1) {
                 /* the smallest distance, the earliest in the list on ties: what one warp going through
@@ -806,41 +854,56 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
                 __shared__ float s_d[WPT][32];
                 __shared__ int s_pos[WPT][32], s_from[WPT][32];
                 const int lane = threadIdx.x & 31;
-                s_d[w][lane] = bd;
-                s_pos[w][lane] = bpos;
-                s_from[w][lane] = from;
+                s_d[v][lane] = bd;
+                s_pos[v][lane] = bpos;
+                s_from[v][lane] = from;
                 __syncthreads();
-                if (w > 0) { count_work(counters, 0, rows); return; }
+                if (v > 0) { count_work(counters, 0, rows); return; }
 #pragma unroll
-                for (int v = 1; v < WPT; v++) {
-                    const int f = s_from[v][lane];
-                    const float d = s_d[v][lane];
-                    if (f >= 0 && (d < bd || (d == bd && from >= 0 && f < from))) { bd = d; bpos = s_pos[v][lane]; from = f; }
+                for (int u = 1; u < WPT; u++) {
+                    const int f = s_from[u][lane];
+                    const float d = s_d[u][lane];
+                    if (f >= 0 && (d < bd || (d == bd && from >= 0 && f < from))) { bd = d; bpos = s_pos[u][lane]; from = f; }
                 }
             }
+            if (live) finish(bpos, bd);
+            count_work(counters, ne, rows);
+            if constexpr (!NX) return;
+            if (!c_q.nx.ch_pos) return;
+            /* The next pass's choose for the match just found: its k-coherence neighbours and searches
+               (the table step belongs to the first pass).  A choose launch of its own reads the state
+               again and stages the tile for few candidates (0.02 per patch after the first pass of the
+               default schedule): 48 x 64 92 us with, 80 without them, 355 x 611 472 and 444, 540 x 960
+               959 and 918.  Walking on inside the loop above, lane by lane, keeps both candidate
+               lists' state in registers and spills: 1080p 4.3 ms instead of 3.5. */
+            Walk<false> w;
+            w.start(c_q, live, bpos, bd);
+            ne = rows = 0;
+            for (;;) {
+                const int c = w.next(c_q, c_q.nx.kcoh, c_q.nx.kc_done, c_q.nx.use_done, c_q.nx.do_kcoh, c_q.nx.pass, true, p);
+                if (!__any_sync(FULL, c >= 0)) break;
+                const float d = dist32<TP, DESC, true, D>(aq, c_q, c, c >= 0, w.dbest, rows);
+                if (c >= 0) {
+                    ne++;
+                    w.offer(c, d);
+                }
+            }
+            if (live) { c_q.nx.ch_pos[p] = w.best; c_q.nx.ch_d[p] = w.dch; }
+            count_work(c_q.nx.counters, ne, rows);
+            return;
         }
     }
-    if (live) {
-        if (c_q.ann) {                          /* k_output fused: x, y, dist of the final field */
-            double *o = c_q.ann + 3 * (size_t) p;
-            o[0] = pt_x(bpos);
-            o[1] = pt_y(bpos);
-            o[2] = bd;
-        } else {
-            nxt_pos[p] = bpos;
-            nxt_d[p] = bd;
-        }
-    }
+    if (live) finish(bpos, bd);
     count_work(counters, ne, rows);
 }
 
-template<int TP, int R, bool DESC, bool ONE = false, int D = 1, int WPT = 1>
+template<int TP, int R, bool DESC, bool ONE = false, bool NX = false, int D = 1, int WPT = 1>
 __global__ void __launch_bounds__(TP * WPT, min_ctas(WPT > 1 ? 2 * TP * WPT : ONE ? PULL_ONE_LANES : PULL_LANES, TP * WPT))
 k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
             const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
             int *nxt_pos, float *nxt_d, unsigned long long *counters) {
     extern __shared__ float at[];
-    pull_tile<TP, R, DESC, ONE, D, WPT>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
+    pull_tile<TP, R, DESC, ONE, NX, D, WPT>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
                                 blockIdx.x * cta_w(TP, DESC), blockIdx.y * cta_h(TP, DESC) + c_q.row0, c_q.row0 + c_q.rows);
 }
 
@@ -904,7 +967,7 @@ k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, l
     });
 }
 
-template<int TP, int R, bool ONE = false>
+template<int TP, int R, bool ONE = false, bool NX = false>
 __global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES, TP))
 k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
              const float *__restrict__ a, const int *__restrict__ cur_pos,
@@ -920,7 +983,8 @@ k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, lon
         q.aw = g.w; q.ah = g.h; q.ew = g.ew; q.eh = g.eh;
         const long long o = g.patch_off;
         if (base.ann) q.ann = base.ann + 3 * o;        /* last pass: this image's NNF records */
-        pull_tile<TP, R, false, ONE>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
+        if (base.nx.ch_pos) { q.nx.ch_pos += o; q.nx.ch_d += o; q.nx.kc_done += o; }
+        pull_tile<TP, R, false, ONE, NX>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
                                      cur_d ? cur_d + o : nullptr, ch_pos + o, ch_d + o, nxt_pos + o, nxt_d + o, counters,
                                      (ls % spr) * tile_w(TP), (ls / spr) * tile_h(TP), g.eh);
     });
@@ -1068,22 +1132,6 @@ __global__ void k_output(int n, const int *__restrict__ pos, const float *__rest
 
 }  // namespace
 
-namespace {
-
-std::atomic<int> g_lean_kernels{1};
-
-/* The specialised variants apply: the choose of a pass with only the table step, the pull of a
-   schedule with one neighbour candidate (image mode; descriptor mode keeps the general kernels). */
-bool lean_choose(const QPlan &q) {
-    return g_lean_kernels.load(std::memory_order_relaxed) && !q.adesc && !q.do_kcoh && q.ntc == 0 && q.spatial == 0 &&
-           !q.do_rs;
-}
-bool one_pull(const QPlan &q) { return g_lean_kernels.load(std::memory_order_relaxed) && !q.adesc && q.pull_max == 1; }
-
-}  // namespace
-
-extern "C" int pt_set_lean_kernels(int on) { return g_lean_kernels.exchange(on ? 1 : 0); }
-
 /* SMs of the current device, asked once. */
 static int sm_count() {
     static std::atomic<int> n{0};
@@ -1096,6 +1144,31 @@ static int sm_count() {
     }
     return v;
 }
+
+namespace {
+
+std::atomic<int> g_lean_kernels{1};
+
+/* The specialised variants apply: the choose of a pass with only the table step, the pull of a
+   schedule with one neighbour candidate (image mode; descriptor mode keeps the general kernels). */
+bool lean_choose(const QPlan &q) {
+    return g_lean_kernels.load(std::memory_order_relaxed) && !q.adesc && !q.do_kcoh && q.ntc == 0 && q.spatial == 0 &&
+           !q.do_rs;
+}
+/* (a pull that does the next pass's choose is a general one) */
+bool one_pull(const QPlan &q) { return g_lean_kernels.load(std::memory_order_relaxed) && !q.adesc && q.pull_max == 1; }
+
+}  // namespace
+
+/* Schedules whose later chooses have much to do (a spatial search) or whose pulls have (24 neighbours)
+   gain from the launches saved only while the image is small: -speed 1, in us, 355 x 611 829 apart and
+   797 together, 540 x 960 1,675 and 1,705; -speed 6 653 and 649, 1,491 and 1,505. */
+bool pt_pull_chooses(const QuerySetup &s, long long patches) {
+    if (s.adesc || (g_lean_kernels.load(std::memory_order_relaxed) && s.pull_max == 1)) return false;
+    return (s.spatial <= 0 && s.radius <= 1) || patches <= 64ll * 32 * sm_count();
+}
+
+extern "C" int pt_set_lean_kernels(int on) { return g_lean_kernels.exchange(on ? 1 : 0); }
 
 static dim3 tile_grid(const QPlan &q, int tp) {
     const int w = cta_w(tp, q.adesc != nullptr), h = cta_h(tp, q.adesc != nullptr);
@@ -1137,6 +1210,14 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     q.do_rs = s.do_rs;
     q.pass = s.pass;
     q.ann = s.ann;
+    q.nx.kcoh = s.nx_kcoh;
+    q.nx.kc_done = s.nx_kc_done;
+    q.nx.use_done = s.nx_use_done;
+    q.nx.do_kcoh = s.nx_do_kcoh;
+    q.nx.pass = s.nx_pass;
+    q.nx.ch_pos = s.nx_ch_pos;
+    q.nx.ch_d = s.nx_ch_d;
+    q.nx.counters = s.nx_evals;
     if (q.adesc) {
         if (!q.bdesc || (s.ds != 8 && s.ds != 16) || q.nd < 3 || q.nd > s.ds)
             return pt_fail(PT_BAD_ARG, "descriptor query: store of %d floats for %d dimensions", s.ds, q.nd);
@@ -1244,9 +1325,11 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *
 #define PT_PULL_T(T, RR) { const dim3 grid = tile_grid(q, T); \
         if (one) k_pull_tile<T, RR, false, true><<<grid, T, atile_bytes(T), st>>>( \
             q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
+        else if (q.nx.ch_pos) k_pull_tile<T, RR, false, false, true><<<grid, T, atile_bytes(T), st>>>( \
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
         else k_pull_tile<T, RR, false><<<grid, T, atile_bytes(T), st>>>( \
             q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); }
-    const bool one = one_pull(q);
+    const bool one = one_pull(q) && !q.nx.ch_pos;
     /* Small images leave most of the chip idle and wait for one warp's rounds of candidates: four
        warps share a tile's list.  The four pulls of the default schedule, in us: 48 x 64 98 -> 58,
        100 x 150 (2.8 tiles per SM) 119 -> 66, 140 x 200 (5.4) 124 -> 107, 180 x 260 (9.2) 137 -> 159. */
@@ -1254,10 +1337,10 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *
     if (q.auto_tile && !one && (long long) tiles.x * tiles.y <= (long long) SPLIT_TILES * sm_count()) {
         constexpr int T = 32;
         if (r1)
-            k_pull_tile<T, 1, false, false, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
+            k_pull_tile<T, 1, false, false, true, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
                 q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
         else
-            k_pull_tile<T, 2, false, false, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
+            k_pull_tile<T, 2, false, false, true, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
                 q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
         PT_LAUNCHED();
         return PT_OK;
@@ -1348,10 +1431,13 @@ pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, in
         if (one) { const int g = persistent_grid(k_pull_batch<T, RR, true>, T, sm, nseg); \
             k_pull_batch<T, RR, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, \
                                                         nxt_d, evals, work); } \
+        else if (q.nx.ch_pos) { const int g = persistent_grid(k_pull_batch<T, RR, false, true>, T, sm, nseg); \
+            k_pull_batch<T, RR, false, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, \
+                                                               nxt_pos, nxt_d, evals, work); } \
         else { const int g = persistent_grid(k_pull_batch<T, RR>, T, sm, nseg); \
             k_pull_batch<T, RR><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, \
                                                   evals, work); } }
-    const bool one = one_pull(q);
+    const bool one = one_pull(q) && !q.nx.ch_pos;
     const bool r1 = q.radius <= 1;
     switch (BATCH_TW[twi]) {
         case 32: if (r1) PT_PULL_B(32, 1) else PT_PULL_B(32, 2) break;

@@ -31,8 +31,8 @@ struct pt_batch {
     long long npix = 0, P = 0, ntiles = 0, nseg[PT_BATCH_NTW] = {0, 0, 0, 0};
     int twi = PT_BATCH_NTW - 1;           /* 256 query patches per CTA until tuned */
     DevBuf<float> rgb;                    /* copy of a query buffer that shares memory with the NNF */
-    DevBuf<int> tcand, pos[2], chpos, kcdone;
-    DevBuf<float> dd[2], chd;
+    DevBuf<int> tcand, pos[2], chpos, chpos1, kcdone;
+    DevBuf<float> dd[2], chd, chd1;       /* ch*1: choices a pull makes for the next pass */
     DevBuf<unsigned long long> work;      /* work counters of the persistent launches */
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -83,6 +83,10 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     const int passes = pt_default_passes(p);
     const bool direct_out = p.do_prop && passes > 0;
     const int jump = pt_default_jump(p, passes);
+    /* from the second pass on, the choices are made by the pull before (as in single lookups) */
+    const bool fuse = passes > 1 && p.do_prop && pt_pull_chooses(qs, B->P);
+    int *const chpos[2] = {B->chpos.p, fuse ? B->chpos1.p : B->chpos.p};
+    float *const chd[2] = {B->chd.p, fuse ? B->chd1.p : B->chd.p};
     int cur = 0;
     for (int i = 0; i < passes; i++) {
         const bool do_table = i == 0 && p.do_table_lookup;
@@ -90,15 +94,26 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
         qi.pass = i;
         if (!pt_pass_kcoh(p, i, passes)) qi.kcoherence = 0;
         const int use_done = i > 0 && pt_pass_kcoh(p, i - 1, passes);
-        PT_TRY(pt_launch_choose_batch(qi, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
-                                      i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->tcand.p, v.kcoh,
-                                      do_table, B->chpos.p, B->chd.p, B->kcdone.p, use_done, nullptr, B->work.p + 1, st));
+        if (!fuse || i == 0)
+            PT_TRY(pt_launch_choose_batch(qi, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
+                                          i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->tcand.p,
+                                          v.kcoh, do_table, B->chpos.p, B->chd.p, B->kcdone.p, use_done, nullptr,
+                                          B->work.p + 1, st));
         if (p.do_prop) {
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
             if (i == passes - 1 && direct_out) qp.ann = d_ann;
+            if (fuse && i + 1 < passes) {
+                qp.nx_kcoh = v.kcoh;
+                qp.nx_kc_done = B->kcdone.p;
+                qp.nx_use_done = pt_pass_kcoh(p, i, passes);
+                qp.nx_do_kcoh = pt_pass_kcoh(p, i + 1, passes);
+                qp.nx_pass = i + 1;
+                qp.nx_ch_pos = chpos[(i + 1) & 1];
+                qp.nx_ch_d = chd[(i + 1) & 1];
+            }
             PT_TRY(pt_launch_pull_batch(qp, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
-                                        i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->chpos.p, B->chd.p,
+                                        i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, chpos[i & 1], chd[i & 1],
                                         B->pos[1 - cur].p, B->dd[1 - cur].p, nullptr, B->work.p + 2, st));
             cur = 1 - cur;
         } else {
@@ -155,7 +170,7 @@ pt_status pt_batch_create(pt_table *t, int n, const int *h, const int *w, pt_bat
     auto fail = [&](pt_status s) { delete B; return s; };
     if (B->d_imgs.reserve(n) || B->tcand.reserve(pat) ||
         B->pos[0].reserve(pat) || B->pos[1].reserve(pat) || B->dd[0].reserve(pat) || B->dd[1].reserve(pat) ||
-        B->chpos.reserve(pat) || B->chd.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
+        B->chpos.reserve(pat) || B->chd.reserve(pat) || B->chpos1.reserve(pat) || B->chd1.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
         return fail(pt_fail(PT_OOM, "batch buffers for %lld pixels / %lld patches", pix, pat));
     if (cudaMemcpy(B->d_imgs.p, B->imgs.data(), sizeof(PtBatchImage) * n, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(pt_fail(PT_CUDA_ERR, "batch geometry upload"));

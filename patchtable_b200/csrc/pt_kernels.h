@@ -141,8 +141,19 @@ struct QuerySetup {
     /* Last pull of a query: the NNF is written here directly (x, y, dist as float64 per patch,
        the output step fused) instead of the next state arrays; NULL otherwise. */
     double *ann = nullptr;
+    /* A pull that also does the next pass's choose (pt_pull_chooses): its k-coherence arguments as
+       pt_launch_choose takes them, and the choices' arrays, which differ from the ones it reads. */
+    const int2 *nx_kcoh = nullptr;
+    int *nx_kc_done = nullptr;
+    int nx_use_done = 0, nx_do_kcoh = 0, nx_pass = 0;
+    int *nx_ch_pos = nullptr;
+    float *nx_ch_d = nullptr;
+    unsigned long long *nx_evals = nullptr;
     cudaStream_t stream;
 };
+/* Whether the pulls of a query of so many patches do the next pass's choose (image mode, more than one
+   neighbour candidate). */
+bool pt_pull_chooses(const QuerySetup &s, long long patches);
 /* Query schedule.  By default two choose + pull passes stand in for each of the reference's
    sequential sweeps (prop_iters, patchtable.h:3608), and the first pull reaches neighbours
    min(8, 2^(passes-1)) patches away, halving on each pass (jump flooding). */

@@ -140,8 +140,8 @@ struct pt_table {
     DevBuf<float> q_rgb;
     DevBuf<float> q_desc;
     DevBuf<int> q_tcand;
-    DevBuf<int> q_pos[2], q_chpos, q_kcdone;
-    DevBuf<float> q_d[2], q_chd;
+    DevBuf<int> q_pos[2], q_chpos, q_chpos1, q_kcdone;
+    DevBuf<float> q_d[2], q_chd, q_chd1;    /* q_ch*1: choices a pull makes for the next pass */
     DevBuf<double> q_ann;
     DevBuf<int> q_lcand;              /* learned proposals, P x PT_PROP_TOPK */
     DevBuf<double> q_prev, q_torig;   /* temporal lookups: previous NNF (host path), restored distances */
@@ -620,6 +620,8 @@ pt_status ensure_query_buffers(pt_table *t, int h, int w) {
     PT_CUDA(t->q_tcand.reserve(P));
     for (int k = 0; k < 2; k++) { PT_CUDA(t->q_pos[k].reserve(P)); PT_CUDA(t->q_d[k].reserve(P)); }
     PT_CUDA(t->q_chpos.reserve(P));
+    PT_CUDA(t->q_chpos1.reserve(P));
+    PT_CUDA(t->q_chd1.reserve(P));
     PT_CUDA(t->q_kcdone.reserve(P));
     PT_CUDA(t->q_chd.reserve(P));
     PT_CUDA(t->q_counters.reserve(6));
@@ -766,6 +768,11 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     int passes = pt_default_passes(p);
     int jump = pt_default_jump(p, passes);
     int cur = 0;
+    /* From the second pass on, a pull makes the next pass's choices in the same launch: choices
+       alternate between two pairs of arrays, since its neighbours still read the ones it started from. */
+    const bool fuse = passes > 1 && p.do_prop && !learned && pt_pull_chooses(qs, P);
+    int *const chpos[2] = {t->q_chpos.p, fuse ? t->q_chpos1.p : t->q_chpos.p};
+    float *const chd[2] = {t->q_chd.p, fuse ? t->q_chd1.p : t->q_chd.p};
     for (int i = 0; i < passes; i++) {
         /* Pass 0 plays the reference's first iteration (table lookup, :3641); k-coherence runs
            on the passes of the sweeps that kcoherence_iter selects.  A pass skips a repeated
@@ -782,7 +789,7 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
                                             ext ? ext->conf : t->q_lconf.p, ext ? ext->threshold : pt_prop_threshold(net),
                                             ext ? ext->kcoh_confident : pt_prop_kcoh_confident(net), ctr,
                                             ctr ? ctr + 4 : nullptr, st));
-        else
+        else if (!fuse || i == 0)
             PT_TRY(pt_launch_choose(qi, n, a_rgb, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
                                     fresh && i == 0 ? nullptr : t->q_d[cur].p, t->q_tcand.p, t->kcoh.p, do_table,
                                     t->q_chpos.p, t->q_chd.p, t->q_kcdone.p, use_done, ctr, st));
@@ -791,8 +798,18 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
             if (i == passes - 1 && direct_out) qp.ann = d_ann;
+            if (fuse && i + 1 < passes) {
+                qp.nx_kcoh = t->kcoh.p;
+                qp.nx_kc_done = t->q_kcdone.p;
+                qp.nx_use_done = pt_pass_kcoh(p, i, passes);
+                qp.nx_do_kcoh = pt_pass_kcoh(p, i + 1, passes);
+                qp.nx_pass = i + 1;
+                qp.nx_ch_pos = chpos[(i + 1) & 1];
+                qp.nx_ch_d = chd[(i + 1) & 1];
+                qp.nx_evals = ctr;
+            }
             PT_TRY(pt_launch_pull(qp, n, a_rgb, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
-                                  fresh && i == 0 ? nullptr : t->q_d[cur].p, t->q_chpos.p, t->q_chd.p,
+                                  fresh && i == 0 ? nullptr : t->q_d[cur].p, chpos[i & 1], chd[i & 1],
                                   t->q_pos[1 - cur].p, t->q_d[1 - cur].p, ctr ? ctr + 2 : nullptr, st));
             PT_TRY(mark(t, prof, LookupProfile::PULL, st));
             cur = 1 - cur;
