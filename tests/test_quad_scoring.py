@@ -46,6 +46,33 @@ def test_edges_of_tiles_and_lines(gpu, oracle, libc, size, bsize, sched):
     t.close()
 
 
+@pytest.mark.parametrize("sw", ["", " -speed 1", " -speed 6"])
+def test_ties_keep_the_list_order(gpu, libc, sw):
+    """Flat images: many candidates tie exactly in distance and key.  Four warps sharing a tile's list
+    (tile 0), one warp per tile, and the zero-allocation lookup's separate chooses pick the same one."""
+    import torch
+    rng = np.random.default_rng(3)
+    a, b = (np.repeat(np.repeat(rng.integers(0, 2, (h // 12 + 1, w // 12 + 1, 3)), 12, 0), 12, 1)[:h, :w].astype(np.float32)
+            for h, w in ((60, 75), (50, 90)))
+    srand_all(libc, 1)
+    p = ptb.PatchTableParams("-coherence_spatial 4 -limit 0.1 -kcoherence 0" + sw)
+    p.kcoherence = 0
+    t = ptb.PatchTable(p, np.ascontiguousarray(b))
+    a = np.ascontiguousarray(a)
+    want = _lookup(t, a)
+    for tile in (32, 64, 128, 256):
+        p.gpu_tile = tile
+        assert np.array_equal(_lookup(t, a), want), tile
+    f = ptb.lib().pt_table_lookup_device_noalloc
+    f.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]
+    da = torch.from_numpy(a).cuda()
+    ann = torch.empty(want.shape, dtype=torch.float64, device="cuda")
+    assert f(t._h, da.data_ptr(), a.shape[0], a.shape[1], ann.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(ann.cpu().numpy(), want)
+    t.close()
+
+
 def test_query_image_inside_the_field_buffer(gpu, libc):
     """A caller may hand over a query image that lies in the buffer the field is written to."""
     import torch
