@@ -74,6 +74,12 @@ __device__ __forceinline__ unsigned mix32(unsigned x) {
     return x;
 }
 
+/* Programmatic dependent launch: a query's kernels let the next one start as soon as all their CTAs run
+   (pdl_trigger), and wait for the ones before them to end (pdl_wait) after what reads only the query
+   image.  Every CTA waits, so a kernel never ends before its predecessors. */
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float finf() { return __int_as_float(0x7f800000); }
 
 /* Adds per-thread counts to counters[0..1] with one atomic per warp (profiling only). */
@@ -622,6 +628,8 @@ k_choose_tile(const QPlan c_q, const float *__restrict__ a, const int *__restric
               const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
               int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs la) {
     extern __shared__ float at[];
+    pdl_trigger();
+    pdl_wait();
     choose_tile<TP, LEARNED, LEAN>(c_q, at, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done,
                                    counters, la, blockIdx.x * tile_w(TP), blockIdx.y * tile_h(TP) + c_q.row0,
                                    c_q.row0 + c_q.rows);
@@ -705,6 +713,8 @@ __global__ void __launch_bounds__(TILE_DESC, 10 * 64 / TILE_DESC)
 k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restrict__ cur_d,
               const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table, int *ch_pos, float *ch_d,
               int *kc_done, int use_done, unsigned long long *counters) {
+    pdl_trigger();
+    pdl_wait();
     const int x = blockIdx.x * TILE_DESC + threadIdx.x, y = blockIdx.y + q.row0;
     DescLane l;
     l.ne = 0;
@@ -741,6 +751,8 @@ k_pull_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restr
             const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos, float *nxt_d,
             unsigned long long *counters) {
     constexpr int W = 2 * R + 1, MAXC = W * W - 1, G = 8;
+    pdl_trigger();
+    pdl_wait();
     const int x = blockIdx.x * TILE_DESC + threadIdx.x, y = blockIdx.y + q.row0;
     const bool live = x < q.ew;
     unsigned ne = 0;
@@ -1042,6 +1054,10 @@ k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict_
             const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
             int *nxt_pos, float *nxt_d, unsigned long long *counters) {
     extern __shared__ float at[];
+    if constexpr (DESC || ONE || WPT > 1) {      /* the others are launched in order */
+        pdl_trigger();
+        pdl_wait();
+    }
     pull_tile<TP, R, DESC, ONE, NX, D, WPT>(c_q, at, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, counters,
                                 blockIdx.x * cta_w(TP, DESC), blockIdx.y * cta_h(TP, DESC) + c_q.row0, c_q.row0 + c_q.rows);
 }
@@ -1310,6 +1326,34 @@ bool pt_pull_chooses(const QuerySetup &s, long long patches) {
 
 extern "C" int pt_set_lean_kernels(int on) { return g_lean_kernels.exchange(on ? 1 : 0); }
 
+/* Whether a launch may start while the kernel before it in the stream ends: descriptor mode always
+   (540 x 960 208 -> 194 us), one candidate per patch up to 24 tiles per SM (48 x 64 27.7 -> 22.6 us, 180 x
+   260 29.8 -> 26.7, 290 x 440 43.0 -> 41.5, 355 x 611 59.0 and 59.1), candidate lists up to 4 (48 x 64 79.9
+   -> 73.9, 100 x 150 89.7 -> 83.7, 140 x 200 143 and 149, 228 x 350 200 and 256: the early CTAs leave the
+   SMs unevenly loaded). */
+static bool early(const QuerySetup &s, const QPlan &q, bool single) {
+    if (!s.pdl) return false;
+    if (q.adesc) return true;
+    const long long tiles = (long long) ((q.ew + WTW - 1) / WTW) * ((q.rows + WTH - 1) / WTH);
+    return tiles <= (long long) (single ? 24 : SPLIT_TILES) * sm_count();
+}
+
+/* A launch that may start early or not (the kernel waits for the one before it by itself). */
+template<class... KA, class... A>
+static cudaError_t launch(bool pdl, void (*kernel)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, KA(args)...);
+}
+
 static dim3 tile_grid(const QPlan &q, int tp) {
     const int w = cta_w(tp, q.adesc != nullptr), h = cta_h(tp, q.adesc != nullptr);
     return dim3((q.ew + w - 1) / w, (q.rows + h - 1) / h);
@@ -1396,15 +1440,16 @@ pt_status pt_launch_choose(const QuerySetup &s, int n, const float *a, const int
     if (q.adesc) {                       /* descriptor mode: one tile width, nothing staged */
         constexpr int T = TILE_DESC;
         const dim3 grid = tile_grid(q, T);
-        k_choose_desc<<<grid, T, 0, st>>>(q, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals);
+        PT_CUDA(launch(early(s, q, false), k_choose_desc, grid, T, 0, st, q, cur_pos, cur_d, tcand, kcoh, do_table,
+                       ch_pos, ch_d, kc_done, use_done, evals));
         PT_LAUNCHED();
         return PT_OK;
     }
 #define PT_CHOOSE_T(T) { const dim3 grid = tile_grid(q, T); \
-        if (lean) k_choose_tile<T, false, true><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); \
-        else k_choose_tile<T, false><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none); }
+        if (lean) PT_CUDA(launch(early(s, q, lean), (k_choose_tile<T, false, true>), grid, T, atile_bytes(T), st, \
+            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none)); \
+        else PT_CUDA(launch(early(s, q, lean), (k_choose_tile<T, false>), grid, T, atile_bytes(T), st, \
+            q, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, ch_d, kc_done, use_done, evals, none)); }
     const bool lean = lean_choose(q);
     switch (q.tile) {
         case 32: PT_CHOOSE_T(32) break;
@@ -1458,21 +1503,25 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *
         constexpr int T = TILE_DESC;
         const dim3 grid = tile_grid(q, T);
         if (q.pull_max >= 24) {          /* every neighbour's candidate */
-            if (r1) k_pull_desc<1><<<grid, T, 0, st>>>(q, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
-            else k_pull_desc<2><<<grid, T, 0, st>>>(q, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+            if (r1) PT_CUDA(launch(early(s, q, false), k_pull_desc<1>, grid, T, 0, st, q, cur_pos, cur_d, ch_pos, ch_d,
+                                   nxt_pos, nxt_d, evals));
+            else PT_CUDA(launch(early(s, q, false), k_pull_desc<2>, grid, T, 0, st, q, cur_pos, cur_d, ch_pos, ch_d,
+                                nxt_pos, nxt_d, evals));
         }
-        else if (r1) k_pull_tile<T, 1, true><<<grid, T, 0, st>>>(q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
-        else k_pull_tile<T, 2, true><<<grid, T, 0, st>>>(q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+        else if (r1) PT_CUDA(launch(early(s, q, false), (k_pull_tile<T, 1, true>), grid, T, 0, st, q, a, cur_pos, cur_d,
+                            ch_pos, ch_d, nxt_pos, nxt_d, evals));
+        else PT_CUDA(launch(early(s, q, false), (k_pull_tile<T, 2, true>), grid, T, 0, st, q, a, cur_pos, cur_d,
+                            ch_pos, ch_d, nxt_pos, nxt_d, evals));
         PT_LAUNCHED();
         return PT_OK;
     }
 #define PT_PULL_T(T, RR) { const dim3 grid = tile_grid(q, T); \
-        if (one) k_pull_tile<T, RR, false, true><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
-        else if (q.nx.ch_pos) k_pull_tile<T, RR, false, false, true><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); \
-        else k_pull_tile<T, RR, false><<<grid, T, atile_bytes(T), st>>>( \
-            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals); }
+        if (one) PT_CUDA(launch(early(s, q, one), (k_pull_tile<T, RR, false, true>), grid, T, atile_bytes(T), st, \
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals)); \
+        else if (q.nx.ch_pos) PT_CUDA(launch(false, (k_pull_tile<T, RR, false, false, true>), grid, T, atile_bytes(T), st, \
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals)); \
+        else PT_CUDA(launch(false, (k_pull_tile<T, RR, false>), grid, T, atile_bytes(T), st, \
+            q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals)); }
     const bool one = one_pull(q) && !q.nx.ch_pos;
     /* Small images leave most of the chip idle and wait for one warp's rounds of candidates: four
        warps share a tile's list.  The four pulls of the default schedule, in us: 48 x 64 98 -> 58,
@@ -1481,11 +1530,11 @@ pt_status pt_launch_pull(const QuerySetup &s, int n, const float *a, const int *
     if (q.auto_tile && !one && (long long) tiles.x * tiles.y <= (long long) SPLIT_TILES * sm_count()) {
         constexpr int T = 32;
         if (r1)
-            k_pull_tile<T, 1, false, false, true, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
-                q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+            PT_CUDA(launch(early(s, q, one), (k_pull_tile<T, 1, false, false, true, SPLIT_D, SPLIT_W>), tiles, T * SPLIT_W,
+                           atile_bytes(T), st, q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals));
         else
-            k_pull_tile<T, 2, false, false, true, SPLIT_D, SPLIT_W><<<tiles, T * SPLIT_W, atile_bytes(T), st>>>(
-                q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals);
+            PT_CUDA(launch(early(s, q, one), (k_pull_tile<T, 2, false, false, true, SPLIT_D, SPLIT_W>), tiles, T * SPLIT_W,
+                           atile_bytes(T), st, q, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, evals));
         PT_LAUNCHED();
         return PT_OK;
     }

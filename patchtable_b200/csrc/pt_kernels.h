@@ -149,6 +149,7 @@ struct QuerySetup {
     int *nx_ch_pos = nullptr;
     float *nx_ch_d = nullptr;
     unsigned long long *nx_evals = nullptr;
+    int pdl = 0;             /* may start while the kernel before it in the stream ends */
     cudaStream_t stream;
 };
 /* Whether the pulls of a query of so many patches do the next pass's choose (image mode, more than one

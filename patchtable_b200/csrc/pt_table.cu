@@ -730,6 +730,7 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     qs.allowed = t->allowed.p;
     qs.allowed_index = p.allowed_index;
     qs.stream = st;
+    qs.pdl = prof == nullptr;
     if (t->desc_mode) {
         qs.adesc = t->q_desc.p;
         qs.bdesc = t->b_desc.p;
