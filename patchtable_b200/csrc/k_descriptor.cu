@@ -1,4 +1,4 @@
-/* Patch descriptor kernel: RGB -> (RGBA copy, YUV, Walsh-Hadamard projections of every 8x8 patch).
+/* Patch descriptor kernels: RGB -> YUV -> Walsh-Hadamard projections of every 8x8 patch.
 
    Replaces get_padded_descriptor (patchtable/patchtable.h:2492-2546): ARRAY_RGB2YUV
    (solver/array.h:1116-1127) followed by gck_8 (patchtable/gck.h:29-1950).  The reference
@@ -11,8 +11,8 @@
    coalesced loads, converts it to YUV in double precision exactly as the reference does (double
    constants, left-to-right sum, rounded to float), applies each needed horizontal sign vector
    per row, then each vertical sign vector per patch, and writes the descriptor as ndims floats
-   padded to a 32- or 64-byte record.  The same pass writes the RGBA (float4) copy of the image
-   used by the distance kernels. */
+   padded to a 32- or 64-byte record.  A table's own image also has its RGBA (float4) copy written by
+   the same pass. */
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <mutex>
@@ -222,28 +222,25 @@ __device__ __forceinline__ void desc_tile(const DescPlan &c_plan, float *smem, c
    0.081 at five, 0.104 at six, which spills). */
 __global__ void __launch_bounds__(NT, 5)
 k_descriptor(const DescPlan c_plan, const float *__restrict__ rgb, int h, int w, int convert,
-             float4 *__restrict__ rgba, float *__restrict__ desc, int ds, int eh, int ew, int ty0) {
+             float4 *__restrict__ rgba, float *__restrict__ desc, int ds, int eh, int ew) {
     extern __shared__ __align__(16) float smem[];
-    desc_tile(c_plan, smem, rgb, h, w, convert, rgba, desc, ds, eh, ew, blockIdx.x * TW, (blockIdx.y + ty0) * TH);
+    desc_tile(c_plan, smem, rgb, h, w, convert, rgba, desc, ds, eh, ew, blockIdx.x * TW, blockIdx.y * TH);
 }
 
 __global__ void __launch_bounds__(NT, 5)
 k_descriptor_cells(const DescPlan c_plan, const CellPlan cp, const float *__restrict__ rgb, int h, int w, int convert,
-                   float4 *__restrict__ rgba, int eh, int ew, int ty0) {
+                   int eh, int ew, int ty0) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");    /* the choose may stage its tiles */
     extern __shared__ __align__(16) float smem[];
-    desc_tile<true>(c_plan, smem, rgb, h, w, convert, rgba, nullptr, 0, eh, ew, blockIdx.x * TW, (blockIdx.y + ty0) * TH, &cp,
-                    cp.tcand);
+    desc_tile<true>(c_plan, smem, rgb, h, w, convert, nullptr, nullptr, 0, eh, ew, blockIdx.x * TW, (blockIdx.y + ty0) * TH,
+                    &cp, cp.tcand);
 }
 
-/* Persistent descriptor pass over the 64 x 8 tiles of every image of a batch (images, RGBA
-   copies and descriptors concatenated), the tiles handed out by a work counter; with CELLS the
-   table entries of the patches' cells are written instead of the descriptors. */
-template<bool CELLS>
+/* Persistent form of k_descriptor_cells over the 64 x 8 tiles of every image of a batch (images and
+   patches concatenated), the tiles handed out by a work counter. */
 __global__ void __launch_bounds__(NT, 5)
 k_descriptor_batch(const DescPlan c_plan, const CellPlan cp, const PtBatchImage *__restrict__ imgs, int n, long long ntiles,
-                   const float *__restrict__ rgb, int convert, float4 *__restrict__ rgba, float *__restrict__ desc, int ds,
-                   unsigned long long *work) {
+                   const float *__restrict__ rgb, int convert, unsigned long long *work) {
     extern __shared__ __align__(16) float smem[];
     __shared__ long long s_next;
     /* tiles go out one at a time; a CTA claims its next tile when it starts the current one and
@@ -262,9 +259,8 @@ k_descriptor_batch(const DescPlan c_plan, const CellPlan cp, const PtBatchImage 
         const PtBatchImage &g = imgs[lo];
         const long long lt = t - g.tile_off;
         const int tpr = (g.ew + TW - 1) / TW;
-        desc_tile<CELLS>(c_plan, smem, rgb + 3 * g.pix_off, g.h, g.w, convert, rgba ? rgba + g.pix_off : nullptr,
-                         CELLS ? nullptr : desc + g.patch_off * ds, ds, g.eh, g.ew, (int) (lt % tpr) * TW, (int) (lt / tpr) * TH,
-                         &cp, CELLS ? cp.tcand + g.patch_off : nullptr);
+        desc_tile<true>(c_plan, smem, rgb + 3 * g.pix_off, g.h, g.w, convert, nullptr, nullptr, 0, g.eh, g.ew,
+                        (int) (lt % tpr) * TW, (int) (lt / tpr) * TH, &cp, cp.tcand + g.patch_off);
         __syncthreads();                                 /* the next tile reuses the shared memory and s_next */
         if (threadIdx.x == 0) s_next = claim;
         __syncthreads();
@@ -369,11 +365,6 @@ size_t pt_descriptor_smem(int ndims) {
 
 pt_status pt_launch_descriptor(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
                                float *desc, int ds, cudaStream_t st) {
-    return pt_launch_descriptor_rows(ndims, nchroma, rgb, h, w, convert, rgba, desc, ds, 0, (h - 7 + TH - 1) / TH, st);
-}
-
-pt_status pt_launch_descriptor_rows(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
-                                    float *desc, int ds, int trow0, int trows, cudaStream_t st) {
     if (convert == PT_COLOR_LAB) PT_TRY(pt_lab_tables_ready());
     int eh = h - 7, ew = w - 7;
     DescPlan plan;
@@ -385,16 +376,13 @@ pt_status pt_launch_descriptor_rows(int ndims, int nchroma, const float *rgb, in
         PT_CUDA(cudaFuncSetAttribute(k_descriptor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) pt_descriptor_smem(0)));
         attr = true;
     }
-    const int ntr = (eh + TH - 1) / TH;
-    if (trow0 < 0 || trows < 1 || trow0 + trows > ntr)
-        return pt_fail(PT_BAD_ARG, "descriptor tile rows [%d, %d) outside 0..%d", trow0, trow0 + trows, ntr);
-    dim3 grid((ew + TW - 1) / TW, trows);
-    k_descriptor<<<grid, NT, smem, st>>>(plan, rgb, h, w, convert, rgba, desc, ds, eh, ew, trow0);
+    dim3 grid((ew + TW - 1) / TW, (eh + TH - 1) / TH);
+    k_descriptor<<<grid, NT, smem, st>>>(plan, rgb, h, w, convert, rgba, desc, ds, eh, ew);
     PT_LAUNCHED();
     return PT_OK;
 }
 
-pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
+pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, int h, int w, int convert,
                                      const PtBins &bins, const int *to_bin, const int *table, int *tcand, int trow0,
                                      int trows, cudaStream_t st) {
     if (convert == PT_COLOR_LAB) PT_TRY(pt_lab_tables_ready());
@@ -420,17 +408,22 @@ pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, i
     if (trow0 < 0 || trows < 1 || trow0 + trows > ntr)
         return pt_fail(PT_BAD_ARG, "descriptor tile rows [%d, %d) outside 0..%d", trow0, trow0 + trows, ntr);
     dim3 grid((ew + TW - 1) / TW, trows);
-    k_descriptor_cells<<<grid, NT, smem, st>>>(plan, cp, rgb, h, w, convert, rgba, eh, ew, trow0);
+    k_descriptor_cells<<<grid, NT, smem, st>>>(plan, cp, rgb, h, w, convert, eh, ew, trow0);
     PT_LAUNCHED();
     return PT_OK;
 }
 
-namespace {
-
-template<bool CELLS>
-pt_status launch_descriptor_batch(int ndims, int nchroma, const CellPlan &cp, const PtBatchImage *imgs, int n,
-                                  long long ntiles, const float *rgb, int convert, float4 *rgba, float *desc, int ds,
-                                  unsigned long long *work, cudaStream_t st) {
+pt_status pt_launch_descriptor_cells_batch(int ndims, int nchroma, const PtBatchImage *imgs, int n, long long ntiles,
+                                           const float *rgb, int convert, const PtBins &bins, const int *to_bin,
+                                           const int *table, int *tcand, unsigned long long *work, cudaStream_t st) {
+    if (bins.G < 1 || bins.G > ndims) return pt_fail(PT_BAD_ARG, "grid dims %d outside 1..%d", bins.G, ndims);
+    CellPlan cp;
+    memset(&cp, 0, sizeof(cp));
+    cp.G = bins.G;
+    for (int d = 0; d < bins.G; d++) { cp.min_val[d] = bins.min_val[d]; cp.range[d] = bins.range[d]; cp.stride[d] = bins.stride[d]; }
+    cp.to_bin = to_bin;
+    cp.table = table;
+    cp.tcand = tcand;
     if (convert == PT_COLOR_LAB) PT_TRY(pt_lab_tables_ready());
     DescPlan plan;
     PT_TRY(make_plan(ndims, nchroma, plan));
@@ -444,38 +437,21 @@ pt_status launch_descriptor_batch(int ndims, int nchroma, const CellPlan &cp, co
         int dev = 0;
         PT_CUDA(cudaGetDevice(&dev));
         PT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        PT_CUDA(cudaFuncSetAttribute(k_descriptor_batch<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        PT_CUDA(cudaFuncSetAttribute(k_descriptor_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int) pt_descriptor_smem(0)));
     }
     const int slot = plan.ncombo;
     if (per_smem[slot] != smem) {
         int per = 0;
-        PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_descriptor_batch<CELLS>, NT, smem));
+        PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_descriptor_batch, NT, smem));
         per_n[slot] = per < 1 ? 1 : per;
         per_smem[slot] = smem;
     }
     const long long g = (long long) per_n[slot] * nsm;
     PT_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), st));
-    k_descriptor_batch<CELLS><<<(unsigned) (ntiles < g ? ntiles : g), NT, smem, st>>>(plan, cp, imgs, n, ntiles, rgb, convert,
-                                                                                     rgba, desc, ds, work);
+    k_descriptor_batch<<<(unsigned) (ntiles < g ? ntiles : g), NT, smem, st>>>(plan, cp, imgs, n, ntiles, rgb, convert, work);
     PT_LAUNCHED();
     return PT_OK;
-}
-
-}  // namespace
-
-pt_status pt_launch_descriptor_cells_batch(int ndims, int nchroma, const PtBatchImage *imgs, int n, long long ntiles,
-                                           const float *rgb, int convert, float4 *rgba, const PtBins &bins, const int *to_bin,
-                                           const int *table, int *tcand, unsigned long long *work, cudaStream_t st) {
-    if (bins.G < 1 || bins.G > ndims) return pt_fail(PT_BAD_ARG, "grid dims %d outside 1..%d", bins.G, ndims);
-    CellPlan cp;
-    memset(&cp, 0, sizeof(cp));
-    cp.G = bins.G;
-    for (int d = 0; d < bins.G; d++) { cp.min_val[d] = bins.min_val[d]; cp.range[d] = bins.range[d]; cp.stride[d] = bins.stride[d]; }
-    cp.to_bin = to_bin;
-    cp.table = table;
-    cp.tcand = tcand;
-    return launch_descriptor_batch<true>(ndims, nchroma, cp, imgs, n, ntiles, rgb, convert, rgba, nullptr, 0, work, st);
 }
 
 namespace {

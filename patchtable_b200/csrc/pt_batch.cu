@@ -61,7 +61,7 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     }
     /* descriptors are needed only for the table step: one fused pass writes the table entries */
     PT_TRY(pt_launch_descriptor_cells_batch(p.ndims, p.nchroma, B->d_imgs.p, B->n, B->ntiles, d_rgb, pt_color_mode(p),
-                                            nullptr, v.bins, v.to_bin, v.table, B->tcand.p, B->work.p, st));
+                                            v.bins, v.to_bin, v.table, B->tcand.p, B->work.p, st));
     QuerySetup qs;
     qs.aw = 0; qs.ah = 0; qs.bw = v.w; qs.bh = v.h;
     qs.prop_scale = 1.0 / (1 + p.coherence_spatial);

@@ -23,9 +23,6 @@ pt_status pt_descriptor_check(int ndims, int nchroma);
 /* desc may be NULL (only the RGBA copy is written); rgba may be NULL. */
 pt_status pt_launch_descriptor(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
                                float *desc, int ds, cudaStream_t st);
-/* Rows [trow0, trow0 + trows) of 8-patch descriptor tiles only (for banded lookups). */
-pt_status pt_launch_descriptor_rows(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
-                                    float *desc, int ds, int trow0, int trows, cudaStream_t st);
 /* -dim_algo pca: the basis fit on the host (pt_pca.cpp: mean[PT_PCA_DIM], basis[ncomp][PT_PCA_DIM],
    consuming 2 x samples rand() values like the reference) and the projection of every patch of an
    RGB image (k_descriptor.cu), which also writes the RGBA copy when rgba is set. */
@@ -72,8 +69,8 @@ struct PtBins {
 pt_status pt_launch_table_candidates(const PtBins &bins, const float *desc, int ds, long long P, const int *to_bin,
                                      const int *table, int *tcand, cudaStream_t st);
 /* The descriptor pass of query tile rows [trow0, trow0 + trows) fused with the table step: writes
-   the RGBA copy and tcand[p] = table[cell(p)] for every patch of those rows, no descriptors. */
-pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, int h, int w, int convert, float4 *rgba,
+   tcand[p] = table[cell(p)] for every patch of those rows, no descriptors. */
+pt_status pt_launch_descriptor_cells(int ndims, int nchroma, const float *rgb, int h, int w, int convert,
                                      const PtBins &bins, const int *to_bin, const int *table, int *tcand, int trow0,
                                      int trows, cudaStream_t st);
 /* k_table_build.cu: the table's cells in one cooperative launch -- fill with TABLE_UNUSED, populate in
@@ -244,7 +241,7 @@ pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, in
 /* The batch's descriptor pass fused with the table step: tcand[p] = table[cell(p)] for every
    patch of every image, no descriptors stored. */
 pt_status pt_launch_descriptor_cells_batch(int ndims, int nchroma, const PtBatchImage *imgs, int n, long long ntiles,
-                                           const float *rgb, int convert, float4 *rgba, const PtBins &bins, const int *to_bin,
+                                           const float *rgb, int convert, const PtBins &bins, const int *to_bin,
                                            const int *table, int *tcand, unsigned long long *work, cudaStream_t st);
 
 /* Read-only view of a built table, for entry points outside pt_table.cu. */

@@ -692,7 +692,7 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     /* The plain single-table query needs its descriptors only for the table step: one fused pass. */
     const bool fused = !t->desc_mode && !t->pca && !learned && t->subs.empty();
     if (fused)
-        PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), nullptr, t->bins,
+        PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), t->bins,
                                           t->to_bin.p, t->table.p, t->q_tcand.p, 0, (h - 7 + 7) / 8, st));
     PT_TRY(mark(t, prof, LookupProfile::DESC, st));
     if (!fused)
@@ -927,7 +927,7 @@ pt_status enqueue_bands(pt_table *t, const BandIO &io, int h, int w, const std::
         if (b < nb) {
             const int r0 = edge[b], r1 = edge[b + 1];
             PT_CUDA(cudaStreamWaitEvent(sa, ev_in[b], 0));
-            PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, rgb, h, w, pt_color_mode(p), nullptr,
+            PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, rgb, h, w, pt_color_mode(p),
                                               t->bins, t->to_bin.p, t->table.p, t->q_tcand.p, r0 / 8, (r1 - r0 + 7) / 8, sa));
             PT_CUDA(cudaEventRecord(ev_a[b], sa));
         }
