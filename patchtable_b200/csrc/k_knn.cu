@@ -182,6 +182,29 @@ __global__ void k_bucket_box(const float *__restrict__ sp, int N, int nd, int dp
         for (int d = nd; d < dp; d++) rows[(size_t) j * 2 * dp + d] = rows[(size_t) j * 2 * dp + dp + d] = 0.f;
 }
 
+/* Keys that put the warps whose queries lie farthest apart (the diagonals of their boxes) first,
+   since those open the most buckets: a sort of 30 us with its keys for 64,000 warps. */
+__global__ void k_warp_spread(const float *__restrict__ qdesc, const int *__restrict__ qorder, int Q, int nd,
+                              unsigned long long *key, int *warp) {
+    const int t = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31;
+    if (t - lane >= Q) return;
+    const int q = qorder[min(t, Q - 1)];
+    float sum = 0.f;
+    for (int d = 0; d < nd; d++) {
+        float a = qdesc[(size_t) q * nd + d], b = a;
+        for (int o = 16 / KNN_SUB; o; o >>= 1) {
+            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+        }
+        sum += (b - a) * (b - a);
+    }
+    for (int o = 16 / KNN_SUB * 2; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) {
+        key[t >> 5] = 0xffffffffu - __float_as_uint(sum);
+        warp[t >> 5] = t >> 5;
+    }
+}
+
 /* Boxes of level l + 1 from groups of 32 boxes of level l: one warp per box. */
 __global__ void k_group_box(const float *__restrict__ in, int nd, int sin, int n, int stride, float *box) {
     const int j = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -441,20 +464,23 @@ struct KnnWarp {
 
    Bound: instruction issue, of which the list insertions take the largest part (214 per query); at
    1920x1080 (2.05 M queries, 12 neighbours, 6 dimensions) a warp opens 480 buckets, screens 247 and
-   inserts from 95 of them.  27.7 ms, against 109 ms for the exact evaluation of every point of the
-   1,500 buckets a binary tree's bounds left open; with two boxes 27.9 ms, with eight 30.5, with a
-   Morton order and one box 53.8. */
+   inserts from 95 of them.  24.1 ms, against 109 ms for the exact evaluation of every point of the
+   1,500 buckets a binary tree's bounds left open.  The heaviest warps run for half of that time, so
+   they start first (worder); started in the curve's order 27.7 ms (with two boxes 27.9, with eight
+   30.5, with a Morton order and one box 53.8). */
 template<int K, int KS>
 __global__ void __launch_bounds__(KNN_NT)
 k_knn_mma(const float *__restrict__ sp, const int *__restrict__ sidx, int N, int nd, const KnnTree tr, float scale,
-          const float *__restrict__ qdesc, const int *__restrict__ qorder, int Q, int *out) {
+          const float *__restrict__ qdesc, const int *__restrict__ qorder, const int *__restrict__ worder, int Q,
+          int *out) {
     typedef KnnWarp<K, KS> W;
     constexpr int DP = W::DP;
     const unsigned FULL = 0xffffffffu;
     __shared__ float gbox_s[KNN_NT / 32][2 * KNN_SUB * DP];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int t = blockIdx.x * KNN_NT + threadIdx.x;
-    if (t - lane >= Q) return;
+    const int slot = blockIdx.x * (KNN_NT / 32) + wid;
+    if (32ll * slot >= Q) return;
+    const int t = worder[slot] * 32 + lane;
     const bool active = t < Q;
     const int q = qorder[active ? t : t - lane];
     W w{sp, sidx, tr, N, nd, scale, gbox_s[wid]};
@@ -749,11 +775,18 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
        Without a scale (0: ranges whose squares leave float's range) every pair is evaluated exactly. */
     const float reach = sqrtf(60000.f / nd);
     const float scale = rmax > 1e-10f && rmax < 1e30f ? reach / rmax : 0.f;
+    const int nw = (Q + 31) / 32;
+    DevBuf<int> worder(st);
+    PT_CUDA(worder.reserve(nw));
+    k_warp_spread<<<(Q + 255) / 256, 256, 0, st>>>(qdesc, qorder.p, Q, nd, codes.p, idx.p);
+    PT_LAUNCHED();
+    PT_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, codes.p, codes2.p, idx.p, worder.p, nw, 0, 32, st));
+    pt_count_launches(4);
     const dim3 mgrid((Q + KNN_NT - 1) / KNN_NT);
 #define PT_KNN_K(KK) case KK: \
-        if (nd <= 6) k_knn_mma<KK, 1><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, Q, out); \
-        else if (nd <= 14) k_knn_mma<KK, 2><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, Q, out); \
-        else k_knn_mma<KK, 3><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, Q, out); \
+        if (nd <= 6) k_knn_mma<KK, 1><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, worder.p, Q, out); \
+        else if (nd <= 14) k_knn_mma<KK, 2><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, worder.p, Q, out); \
+        else k_knn_mma<KK, 3><<<mgrid, KNN_NT, 0, st>>>(sp.p, perm.p, N, nd, tr, scale, qdesc, qorder.p, worder.p, Q, out); \
         break;
     switch (K) {
         PT_KNN_K(12) PT_KNN_K(16) PT_KNN_K(24) PT_KNN_K(32) PT_KNN_K(48) PT_KNN_K(64)
