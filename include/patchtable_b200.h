@@ -62,7 +62,7 @@ typedef struct pt_params {
        neighbour spacing of the first pass, halved on each later pass down to 1 (jump
        flooding; 0 or 1 = plain neighbours), and the most neighbour offsets a pull pass scores per
        patch, best-first by the neighbour's own distance (0 = all of them), and the query patches one
-       CTA covers in the choose and pull kernels (32, 64, 128 or 256; 0 picks the default, 32; the
+       CTA covers in the choose and pull kernels (32, 64, 128 or 256; 0 picks by the image's size; the
        result does not depend on it). */
     int gpu_prop_passes;
     int gpu_jump;
@@ -176,7 +176,7 @@ pt_status pt_table_lookup_device_temporal(pt_table *t, const float *d_a, int h, 
 /* Zero-allocation form of pt_table_lookup_device (no counterpart in the reference).  For
    callers that may not allocate device memory during queries -- a frame loop with a fixed
    latency budget (cudaMalloc/cudaFree synchronise the device), or an application whose own
-   allocator owns the GPU's memory -- every intermediate buffer comes from one 20 MiB file-scope
+   allocator owns the GPU's memory -- every intermediate buffer comes from one 19 MiB file-scope
    device array instead of cudaMalloc.  Limits: at most PT_NOALLOC_MAX_PIXELS query pixels and
    ndims <= 8 (PT_BAD_ARG / PT_UNSUPPORTED otherwise).  All calls share that array, so calls
    that overlap on the GPU race and must be serialised.  The first call on a device resolves the

@@ -556,7 +556,7 @@ k_knn_mma(const float *__restrict__ sp, const int *__restrict__ sidx, int N, int
    sorted list lives in global memory (wd: distances, out: indices, K per query); a leaf's
    admissible points are first sorted in a 32-entry buffer and then merged into the list from the
    back in one pass, keeping the K smallest.  Traversal, rounding and tie rule are those of
-   k_knn_warp, so its first 64 entries equal that kernel's result. */
+   k_knn_mma, so its first 64 entries equal that kernel's result. */
 __global__ void __launch_bounds__(NT)
 k_knn_wide(const float *__restrict__ sp, const int *__restrict__ sidx, int N, int nd, int L,
            const float *__restrict__ lo, const float *__restrict__ hi, const float *__restrict__ qdesc,
