@@ -785,7 +785,7 @@ k_pull_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restr
             if (xs < 0 || ys < 0 || xs >= q.bew || ys >= q.beh) continue;
             if (q.allowed && __ldg(q.allowed + (size_t) ys * q.bew + xs) != q.allowed_index) continue;
             const int c = pt_xy(xs, ys);
-            bool dup = c == own;
+            bool dup = c == own || !(key[i] < finf());      /* as the sorted list: finite keys only */
 #pragma unroll
             for (int t = 0; t < i; t++) dup |= cand[t] == c;
             if (!dup) cand[i] = c;
@@ -953,7 +953,10 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
         }
     } else {
         /* distinct neighbour candidates sorted by the neighbour's own distance (ties keep the
-           neighbour order), kept in registers: every slot index is known at compile time */
+           neighbour order), kept in registers: every slot index is known at compile time.  A neighbour
+           whose distance is +inf or NaN (the seed of a field may be) has no place in the order: the
+           insertion leaves its offset out and it is not counted, or the walk would score the empty
+           slots at the list's end. */
         int cand[MAXC];
         float key[MAXC];
 #pragma unroll
@@ -964,6 +967,7 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
             for (int t = 0; t < MAXC; t++) dup |= cand[t] == c;
             if (dup) return;
             float k = *kp;
+            const bool finite = k < finf();
 #pragma unroll
             for (int t = 0; t < MAXC; t++) {
                 if (k < key[t]) {
@@ -971,7 +975,7 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
                     const int tc = cand[t]; cand[t] = c; c = tc;
                 }
             }
-            nc++;
+            nc += finite;
         });
         if (nc > c_q.pull_max) nc = c_q.pull_max;   /* the best-first prefix of the list */
         ne = nc;
