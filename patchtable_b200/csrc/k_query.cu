@@ -75,8 +75,10 @@ __device__ __forceinline__ unsigned mix32(unsigned x) {
 }
 
 /* Programmatic dependent launch: a query's kernels let the next one start as soon as all their CTAs run
-   (pdl_trigger), and wait for the ones before them to end (pdl_wait) after what reads only the query
-   image.  Every CTA waits, so a kernel never ends before its predecessors. */
+   (pdl_trigger), and wait for the ones before them to end (pdl_wait) before they read anything.  Every
+   CTA waits, so a kernel never ends before its predecessors.  What a predecessor may still be writing
+   when the kernel starts -- table entries, states and choices -- is not read-only for the kernel's
+   life: those pointers carry no __restrict__, which would allow non-coherent loads. */
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -457,7 +459,7 @@ struct Walk {
     /* The next candidate, or -1 when the walk has ended. */
     __device__ __forceinline__ int next(const QPlan &q, const int2 *__restrict__ kcoh, int *kc_done, int use_done,
                                         int do_kcoh, int pass, bool kc_here, int p, bool table = false,
-                                        const int *__restrict__ tcand = nullptr) {
+                                        const int *tcand = nullptr) {
         int c = -1;
         while (c < 0 && ph != DONE) {
             if (TABLES && ph == TABLE) {
@@ -537,8 +539,8 @@ struct Walk {
    candidate per patch, without the registers of the walk. */
 template<int TP, bool LEARNED, bool LEAN>
 __device__ __forceinline__ void
-choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
-            const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
+choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *cur_pos,
+            const float *cur_d, const int *tcand, const int2 *__restrict__ kcoh, int do_table,
             int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs &la,
             int x0, int y0, int y1) {
     const unsigned FULL = 0xffffffffu;
@@ -624,8 +626,8 @@ choose_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int 
 
 template<int TP, bool LEARNED, bool LEAN = false>
 __global__ void __launch_bounds__(TP, min_ctas(LEAN ? CHOOSE_LEAN_LANES : CHOOSE_LANES, TP))
-k_choose_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
-              const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
+k_choose_tile(const QPlan c_q, const float *__restrict__ a, const int *cur_pos,
+              const float *cur_d, const int *tcand, const int2 *__restrict__ kcoh, int do_table,
               int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters, const LearnedArgs la) {
     extern __shared__ float at[];
     pdl_trigger();
@@ -710,8 +712,8 @@ struct DescLane {
 /* The choose in descriptor mode.  (The lockstep walk of choose_tile measured 0.129 against 0.124 ms
    here: 540 x 960, 8 channels, the four chooses of the default schedule.) */
 __global__ void __launch_bounds__(TILE_DESC, 10 * 64 / TILE_DESC)
-k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restrict__ cur_d,
-              const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table, int *ch_pos, float *ch_d,
+k_choose_desc(const QPlan q, const int *cur_pos, const float *cur_d,
+              const int *tcand, const int2 *__restrict__ kcoh, int do_table, int *ch_pos, float *ch_d,
               int *kc_done, int use_done, unsigned long long *counters) {
     pdl_trigger();
     pdl_wait();
@@ -747,8 +749,8 @@ k_choose_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__res
    with a sorted list and chooses of their own, 203 so. */
 template<int R>
 __global__ void __launch_bounds__(TILE_DESC)
-k_pull_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restrict__ cur_d,
-            const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos, float *nxt_d,
+k_pull_desc(const QPlan q, const int *cur_pos, const float *cur_d,
+            const int *ch_pos, const float *ch_d, int *nxt_pos, float *nxt_d,
             unsigned long long *counters) {
     constexpr int W = 2 * R + 1, MAXC = W * W - 1, G = 8;
     pdl_trigger();
@@ -869,8 +871,8 @@ k_pull_desc(const QPlan q, const int *__restrict__ cur_pos, const float *__restr
    are its own (-speed 1 at 540 x 960: 1.675 ms, 1.714 with the code in the kernel but unused). */
 template<int TP, int R, bool DESC, bool ONE, bool NX, int D = 1, int WPT = 1>
 __device__ __forceinline__ void
-pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *__restrict__ cur_pos,
-          const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d, int *nxt_pos,
+pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *cur_pos,
+          const float *cur_d, const int *ch_pos, const float *ch_d, int *nxt_pos,
           float *nxt_d, unsigned long long *counters, int x0, int y0, int y1) {
     const unsigned FULL = 0xffffffffu;
     if constexpr (!DESC) stage_a<TP, TP * WPT>(at, a, c_q.aw, c_q.ah, x0, y0);
@@ -1054,8 +1056,8 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *_
 
 template<int TP, int R, bool DESC, bool ONE = false, bool NX = false, int D = 1, int WPT = 1>
 __global__ void __launch_bounds__(TP * WPT, min_ctas(WPT > 1 ? 2 * TP * WPT : ONE ? PULL_ONE_LANES : PULL_LANES, TP * WPT))
-k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *__restrict__ cur_pos,
-            const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
+k_pull_tile(const QPlan c_q, const float *__restrict__ a, const int *cur_pos,
+            const float *cur_d, const int *ch_pos, const float *ch_d,
             int *nxt_pos, float *nxt_d, unsigned long long *counters) {
     extern __shared__ float at[];
     if constexpr (DESC || ONE || WPT > 1) {      /* the others are launched in order */
@@ -1104,8 +1106,8 @@ __device__ __forceinline__ void for_each_tile(unsigned long long *work, long lon
 template<int TP, bool LEAN = false>
 __global__ void __launch_bounds__(TP, min_ctas(LEAN ? CHOOSE_LEAN_LANES : CHOOSE_LANES, TP))
 k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
-               const float *__restrict__ a, const int *__restrict__ cur_pos,
-               const float *__restrict__ cur_d, const int *__restrict__ tcand, const int2 *__restrict__ kcoh, int do_table,
+               const float *__restrict__ a, const int *cur_pos,
+               const float *cur_d, const int *tcand, const int2 *__restrict__ kcoh, int do_table,
                int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters,
                unsigned long long *work) {
     extern __shared__ float at[];
@@ -1129,8 +1131,8 @@ k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, l
 template<int TP, int R, bool ONE = false, bool NX = false>
 __global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES, TP))
 k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
-             const float *__restrict__ a, const int *__restrict__ cur_pos,
-             const float *__restrict__ cur_d, const int *__restrict__ ch_pos, const float *__restrict__ ch_d,
+             const float *__restrict__ a, const int *cur_pos,
+             const float *cur_d, const int *ch_pos, const float *ch_d,
              int *nxt_pos, float *nxt_d, unsigned long long *counters, unsigned long long *work) {
     extern __shared__ float at[];
     for_each_tile(work, nseg, [&](long long s) {
