@@ -358,8 +358,8 @@ int64_t pt_set_spin_limit(int64_t polls);
 int64_t pt_set_device_alloc_limit(int64_t bytes);
 int64_t pt_device_bytes_in_use(void);
 /* Gives the memory kept for reuse back: freed buffers stay with the library, at most 4 GiB of device
-   memory per device and 256 MiB of page-locked host memory, so that the next build or lookup need
-   not allocate again. */
+   memory per device beside what is in use and 256 MiB of page-locked host memory, so that the next
+   build or lookup need not allocate again. */
 pt_status pt_release_memory(void);
 
 /* Host threads that widen the downloaded NNF to float64 in pt_table_lookup (no reference

@@ -66,7 +66,7 @@ struct PtPartition {
 #ifdef __CUDACC__
 /* pt_memory.cu: device and page-locked memory, pooled. */
 cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch);
-void pt_dev_free(void *p, int dev, cudaStream_t st, bool scratch);
+void pt_dev_free(void *p, size_t bytes, int dev, cudaStream_t st, bool scratch);
 cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got);
 void pt_pinned_free(void *p, size_t bytes);
 
@@ -93,7 +93,7 @@ template<class T> struct DevBuf {
         return e;
     }
     void release() {
-        if (p) { pt_dev_free(p, dev, st, scratch); pt_alloc_release(held); }
+        if (p) { pt_dev_free(p, held, dev, st, scratch); pt_alloc_release(held); }
         p = nullptr; n = 0; held = 0;
     }
 private:

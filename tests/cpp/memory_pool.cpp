@@ -1,0 +1,88 @@
+/* Checks of the library's memory code (pt_memory.cu and the buffers of pt_internal.h) over a stand-in
+   for the CUDA runtime.  Usage: memory_pool CHECK; prints what failed and returns 1. */
+#include <cstdio>
+#include <cstring>
+#include <memory>
+
+#include "pt_memory.cu"
+
+#include <atomic>
+
+pt_status pt_fail(pt_status s, const char *, ...) { return s; }
+bool pt_alloc_admit(size_t) { return true; }
+void pt_alloc_release(size_t) {}
+
+#define EXPECT(c) do { if (!(c)) { printf("%s:%d: %s\n", __FILE__, __LINE__, #c); return 1; } } while (0)
+
+static const size_t GiB = 1ull << 30;
+static fake::Pool &pool(int dev = 0) {
+    for (fake::Pool *p : fake::pools) if (p->dev == dev) return *p;
+    abort();
+}
+
+/* A build's scratch, freed in its stream's order, with a wait at the end as every build has. */
+static void build(cudaStream_t st) {
+    DevBuf<char> a(st), b(st), c(st);
+    a.reserve(GiB); b.reserve(GiB); c.reserve(GiB / 2);
+    a.release(); b.release(); c.release();
+    cudaStreamSynchronize(st);
+}
+
+/* What is kept for reuse does not depend on how much is live. */
+static int reuse_beside_live() {
+    cudaStream_t st;
+    cudaStreamCreateWithFlags(&st, 0);
+    DevBuf<char> tables[6];
+    for (auto &t : tables) EXPECT(t.reserve(GiB) == cudaSuccess);
+    build(st);
+    const int maps = fake::maps;
+    for (int i = 0; i < 3; i++) build(st);
+    EXPECT(fake::maps == maps);
+    EXPECT(pool().reserved == 6 * GiB + 2 * GiB + GiB / 2);
+    return 0;
+}
+
+/* At most 4 GiB stay beside the live buffers, whatever is freed last. */
+static int bound() {
+    {
+        DevBuf<char> big[3], small;
+        for (auto &t : big) EXPECT(t.reserve(3 * GiB) == cudaSuccess);
+        EXPECT(small.reserve(GiB) == cudaSuccess);
+        big[0].release();
+        big[1].release();
+        EXPECT(pool().reserved <= 4 * GiB + 4 * GiB);
+    }
+    EXPECT(pool().reserved <= 4 * GiB);
+    {
+        DevBuf<char> one;
+        EXPECT(one.reserve(9 * GiB) == cudaSuccess);
+    }
+    EXPECT(pool().reserved <= 4 * GiB);
+    EXPECT(pt_release_memory() == PT_OK && pool().reserved == 0);
+    return 0;
+}
+
+/* An allocation that does not fit beside what is kept for reuse is made in its place; one that does not
+   fit at all fails, and leaves the accounts as they were. */
+static int retry() {
+    fake::capacity = 5 * GiB;
+    { DevBuf<char> a; EXPECT(a.reserve(3 * GiB) == cudaSuccess); }
+    EXPECT(pool().reserved == 3 * GiB);
+    DevBuf<char> b, c;
+    EXPECT(b.reserve(4 * GiB) == cudaSuccess && b.p);
+    EXPECT(c.reserve(2 * GiB) == cudaErrorMemoryAllocation && !c.p);
+    EXPECT(pool().threshold == 8 * GiB);
+    b.release();
+    EXPECT(pt_release_memory() == PT_OK && pool().reserved == 0 && pool().threshold == 4 * GiB);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    const struct { const char *name; int (*run)(); } checks[] = {
+        {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry},
+    };
+    for (const auto &c : checks)
+        if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();
+    printf("unknown check\n");
+    return 2;
+}
