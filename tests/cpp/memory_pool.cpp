@@ -77,9 +77,26 @@ static int retry() {
     return 0;
 }
 
+/* A page-locked allocation that fails is tried again without the blocks kept for reuse, of which at most
+   256 MiB are. */
+static int pinned() {
+    const size_t MiB = 1u << 20;
+    {
+        PinnedBuf<char> b[4];
+        for (auto &x : b) EXPECT(x.reserve(100 * MiB) == cudaSuccess);
+    }
+    EXPECT(fake::host.size() == 2);                       /* 200 of 400 MiB kept */
+    fake::fail_host_allocs = 1;
+    PinnedBuf<char> c, d;
+    EXPECT(c.reserve(500 * MiB) == cudaSuccess && c.p && fake::host.size() == 1);
+    fake::fail_host_allocs = 1;                           /* nothing left to give back */
+    EXPECT(d.reserve(500 * MiB) == cudaErrorMemoryAllocation && !d.p);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const struct { const char *name; int (*run)(); } checks[] = {
-        {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry},
+        {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry}, {"pinned", pinned},
     };
     for (const auto &c : checks)
         if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();
