@@ -68,7 +68,7 @@ struct PtPartition {
 cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch);
 void pt_dev_free(void *p, size_t bytes, int dev, cudaStream_t st, bool scratch);
 cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got);
-void pt_pinned_free(void *p, size_t bytes);
+void pt_pinned_free(void *p, size_t bytes, int dev);
 
 /* A device buffer.  DevBuf() may be used on any stream, and its release waits for the device.
    DevBuf(st) is scratch: used on st only (or on streams joined into it before the release), and
@@ -103,7 +103,8 @@ private:
     int dev = 0;
 };
 
-/* Page-locked host memory owned by a table (download staging). */
+/* Page-locked host memory owned by a table (download staging), for copies of the device that is current
+   when it is reserved. */
 template<class T> struct PinnedBuf {
     T *p = nullptr;
     size_t n = 0;
@@ -114,17 +115,19 @@ template<class T> struct PinnedBuf {
     cudaError_t reserve(size_t count) {
         if (count <= n && p) return cudaSuccess;
         release();
+        cudaGetDevice(&dev);
         cudaError_t e = pt_pinned_alloc((void **) &p, sizeof(T) * (count ? count : 1), &held);
         if (e == cudaSuccess) n = count;
         else p = nullptr;
         return e;
     }
     void release() {
-        if (p) pt_pinned_free(p, held);
+        if (p) pt_pinned_free(p, held, dev);
         p = nullptr; n = 0; held = 0;
     }
 private:
     size_t held = 0;
+    int dev = 0;
 };
 #endif
 

@@ -4,7 +4,8 @@
    costs 0.1 ms and up (with the mapping of large blocks, 18 of the 31 ms of a 240 x 320 build; a
    cudaFree also waits for the whole device).  Buffers therefore come from one CUDA memory pool per
    device.  Scratch buffers (DevBuf given a stream) are freed in that stream's order; all others may
-   have been used on any stream, so their release waits for the device first, as cudaFree did.
+   have been used on any stream, so their release waits for the device first, as cudaFree did; while
+   that wait is refused (another thread's stream capture forbids it) they are held back from reuse.
    Reuse across streams that would make one stream wait for another is switched off: the steps of a
    build run beside each other.
 
@@ -29,17 +30,19 @@ constexpr unsigned long long PT_POOL_KEEP = 4ull << 30;
 constexpr size_t PT_PINNED_KEEP = 256u << 20;
 constexpr int MAX_DEVICES = 64;
 
+struct Block { void *p; size_t bytes; };
+
 struct DevicePool {
     std::mutex mu;
     cudaMemPool_t pool = nullptr;
     cudaStream_t st = nullptr;            /* order of the buffers that belong to no stream */
     unsigned long long live = 0;          /* bytes of the buffers in use */
+    std::vector<Block> held;              /* released, but their device could not be waited for */
 };
 DevicePool g_pool[MAX_DEVICES];
 
-struct Pinned { void *p; size_t bytes; };
 std::mutex g_pinned_mu;
-std::vector<Pinned> g_pinned;             /* free page-locked blocks */
+std::vector<Block> g_pinned;             /* free page-locked blocks */
 size_t g_pinned_bytes = 0;
 
 /* The current device's pool, created on first use. */
@@ -82,15 +85,50 @@ bool set_keep(DevicePool &d, long long bytes) {
     return reserved > keep;
 }
 
+/* Waits for the current device (d's) and gives b and the blocks held back before to the pool; holds
+   them all back when the wait is refused. */
+void wait_and_free(DevicePool &d, Block b) {
+    std::vector<Block> blocks;
+    {
+        std::lock_guard<std::mutex> lock(d.mu);
+        blocks.swap(d.held);
+    }
+    if (b.p) blocks.push_back(b);
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        std::lock_guard<std::mutex> lock(d.mu);
+        d.held.insert(d.held.end(), blocks.begin(), blocks.end());
+        return;
+    }
+    long long bytes = 0;
+    for (const Block &x : blocks) {
+        cudaFreeAsync(x.p, d.st);
+        bytes += (long long) x.bytes;
+    }
+    /* the threshold takes effect at a wait; the last of many frees may have none after it */
+    if (bytes && set_keep(d, -bytes)) cudaStreamSynchronize(d.st);
+}
+
+/* Makes a device current for a scope. */
+struct OnDevice {
+    int cur;
+    explicit OnDevice(int dev) : cur(dev) {
+        cudaGetDevice(&cur);
+        if (cur != dev) cudaSetDevice(dev);
+        else cur = -1;
+    }
+    ~OnDevice() { if (cur >= 0) cudaSetDevice(cur); }
+};
+
 /* Frees the page-locked blocks kept for reuse; returns whether there were any. */
 bool drop_pinned() {
-    std::vector<Pinned> held;
+    std::vector<Block> held;
     {
         std::lock_guard<std::mutex> lock(g_pinned_mu);
         held.swap(g_pinned);
         g_pinned_bytes = 0;
     }
-    for (const Pinned &b : held) cudaFreeHost(b.p);
+    for (const Block &b : held) cudaFreeHost(b.p);
     return !held.empty();
 }
 
@@ -105,7 +143,7 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch) 
     e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        cudaDeviceSynchronize();
+        wait_and_free(*d, {});
         cudaMemPoolTrimTo(d->pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
         if (e != cudaSuccess) cudaGetLastError();
@@ -117,17 +155,14 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch) 
 }
 
 void pt_dev_free(void *p, size_t bytes, int dev, cudaStream_t st, bool scratch) {
-    int cur = dev;
-    cudaGetDevice(&cur);
-    if (cur != dev) cudaSetDevice(dev);
+    const OnDevice on(dev);
+    DevicePool &d = g_pool[dev];
     if (!scratch) {
-        cudaDeviceSynchronize();
-        st = g_pool[dev].st;
+        wait_and_free(d, {p, bytes});
+        return;
     }
     cudaFreeAsync(p, st);
-    /* the threshold takes effect at a wait; the last of many frees may have none after it */
-    if (set_keep(g_pool[dev], -(long long) bytes) && !scratch) cudaStreamSynchronize(st);
-    if (cur != dev) cudaSetDevice(cur);
+    set_keep(d, -(long long) bytes);
 }
 
 cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got) {
@@ -156,26 +191,37 @@ cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got) {
     return e;
 }
 
-void pt_pinned_free(void *p, size_t bytes) {
-    cudaDeviceSynchronize();              /* no copy of a failed call may still use it */
-    {
+void pt_pinned_free(void *p, size_t bytes, int dev) {
+    const OnDevice on(dev);
+    /* no copy of a failed call may still use a block that is kept */
+    if (cudaDeviceSynchronize() == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_pinned_mu);
         if (g_pinned_bytes + bytes <= PT_PINNED_KEEP) {
             g_pinned.push_back({p, bytes});
             g_pinned_bytes += bytes;
             return;
         }
+    } else {
+        cudaGetLastError();
     }
     cudaFreeHost(p);
 }
 
 extern "C" pt_status pt_release_memory(void) {
-    for (DevicePool &d : g_pool) {
-        std::lock_guard<std::mutex> lock(d.mu);
-        if (d.pool) {
-            cudaStreamSynchronize(d.st);
-            PT_CUDA(cudaMemPoolTrimTo(d.pool, 0));
+    for (int dev = 0; dev < MAX_DEVICES; dev++) {
+        DevicePool &d = g_pool[dev];
+        bool held;
+        {
+            std::lock_guard<std::mutex> lock(d.mu);
+            if (!d.pool) continue;
+            held = !d.held.empty();
         }
+        if (held) {
+            const OnDevice on(dev);
+            wait_and_free(d, {});
+        }
+        cudaStreamSynchronize(d.st);
+        PT_CUDA(cudaMemPoolTrimTo(d.pool, 0));
     }
     drop_pinned();
     return PT_OK;

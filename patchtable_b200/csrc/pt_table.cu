@@ -1046,14 +1046,13 @@ pt_status lookup_banded(pt_table *t, const float *a, int h, int w, double *ann_o
     const pt_status est = enqueue_bands(t, io, h, w, edge, nb);
     if (est != PT_OK) stop.store(true, std::memory_order_release);
     if (widener.joinable()) widener.join();
-    if (est != PT_OK) {
+    if (est != PT_OK || widen_err != cudaSuccess) {
         for (cudaStream_t s2 : {t->st, t->st_in, t->st_choose, t->st_pull, t->st_out})
             cudaStreamSynchronize(s2);       /* nothing of this call stays in flight */
-        return est;
+        return est != PT_OK ? est : pt_fail(PT_CUDA_ERR, "band download: %s", cudaGetErrorString(widen_err));
     }
     t->last_h2d = (long long) sizeof(float) * h * w * 3;
     t->last_d2h = (long long) (widen ? sizeof(int) + sizeof(float) : 3 * sizeof(double)) * P;
-    if (widen_err != cudaSuccess) return pt_fail(PT_CUDA_ERR, "band download: %s", cudaGetErrorString(widen_err));
     PT_CUDA(cudaStreamSynchronize(t->st));
     return PT_OK;
 }

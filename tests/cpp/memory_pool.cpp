@@ -94,9 +94,53 @@ static int pinned() {
     return 0;
 }
 
+/* Memory of one device released while another is current: its own device is waited for, and goes back to
+   its own pool. */
+static int other_device() {
+    cudaSetDevice(2);
+    PinnedBuf<char> h;
+    DevBuf<char> b;
+    EXPECT(h.reserve(1000) == cudaSuccess && b.reserve(1000) == cudaSuccess);
+    cudaSetDevice(0);
+    h.release();
+    EXPECT(fake::synced.size() == 1 && fake::synced[0] == 2 && fake::device == 0);
+    b.release();
+    EXPECT(fake::synced.size() == 2 && fake::synced[1] == 2 && fake::device == 0);
+    EXPECT(pt_release_memory() == PT_OK && pool(2).reserved == 0 && fake::device == 0);
+    return 0;
+}
+
+/* A block whose device could not be waited for is not used again before a wait succeeds. */
+static int refused_wait() {
+    char *b0;
+    {
+        PinnedBuf<char> h;
+        DevBuf<char> b;
+        EXPECT(h.reserve(1000) == cudaSuccess && b.reserve(1000) == cudaSuccess);
+        b0 = b.p;
+        fake::refuse_device_sync = 2;
+    }
+    EXPECT(fake::host.empty());                           /* not kept */
+    DevBuf<char> c, d;
+    EXPECT(c.reserve(1000) == cudaSuccess && c.p != b0);
+    EXPECT(pool().threshold == 4 * GiB + 2000);
+    c.release();                                          /* waits, and frees b's block too */
+    EXPECT(pool().threshold == 4 * GiB);
+    EXPECT(d.reserve(1000) == cudaSuccess && (d.p == b0 || pool().blocks.size() == 2));
+    d.release();
+    {
+        DevBuf<char> e;
+        EXPECT(e.reserve(1000) == cudaSuccess);
+        fake::refuse_device_sync = 1;
+    }
+    EXPECT(pt_release_memory() == PT_OK && pool().reserved == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const struct { const char *name; int (*run)(); } checks[] = {
-        {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry}, {"pinned", pinned},
+        {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry}, {"pinned", pinned}, {"other_device", other_device},
+        {"refused_wait", refused_wait},
     };
     for (const auto &c : checks)
         if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();

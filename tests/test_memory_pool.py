@@ -9,7 +9,7 @@ import pytest
 from tests.conftest import ROOT
 
 CPP = os.path.join(ROOT, "tests", "cpp")
-CHECKS = ["reuse_beside_live", "bound", "retry", "pinned"]
+CHECKS = ["reuse_beside_live", "bound", "retry", "pinned", "other_device", "refused_wait"]
 
 
 @pytest.fixture(scope="module")
