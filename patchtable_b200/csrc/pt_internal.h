@@ -10,6 +10,8 @@
 
 #ifdef __CUDACC__
 #include <cuda_runtime.h>
+
+#include <thread>
 #endif
 
 #define PT_NMAP 16384                      /* PATCH_PARTITION_NMAP, patchtable.h:216 */
@@ -69,6 +71,16 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch);
 void pt_dev_free(void *p, size_t bytes, int dev, cudaStream_t st, bool scratch);
 cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got);
 void pt_pinned_free(void *p, size_t bytes, int dev);
+
+/* A host thread that works on the calling thread's device (a new thread's own choice is device 0). */
+template<class F> std::thread pt_device_thread(F fn) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return std::thread([dev, fn]() mutable {
+        cudaSetDevice(dev);
+        fn();
+    });
+}
 
 /* A device buffer.  DevBuf() may be used on any stream, and its release waits for the device.
    DevBuf(st) is scratch: used on st only (or on streams joined into it before the release), and

@@ -515,7 +515,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     PtPartScratch part_scratch(t->st2);       /* freed when the build returns, after the search has ended */
     std::string part_err;
     pt_status part_st = PT_OK;
-    std::thread partitioner([&] {
+    std::thread partitioner = pt_device_thread([&] {
         part_st = timed(part_ms, [&]() -> pt_status {
             cudaStream_t s2 = t->st2;
             t->min_val.assign(t->G, 0.f);
@@ -1029,7 +1029,7 @@ pt_status lookup_banded(pt_table *t, const float *a, int h, int w, double *ann_o
     std::thread widener;
     if (widen) {
         io.recorded = &recorded;
-        widener = std::thread([&] {
+        widener = pt_device_thread([&] {
             for (int b = 0; b < nb; b++) {
                 while (recorded.load(std::memory_order_acquire) <= b) {
                     if (stop.load(std::memory_order_acquire)) return;

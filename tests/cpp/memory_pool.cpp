@@ -137,10 +137,23 @@ static int refused_wait() {
     return 0;
 }
 
+/* A worker thread's buffers come from the device that its caller works on. */
+static int worker_device() {
+    cudaSetDevice(3);
+    DevBuf<char> b;
+    int dev = -1;
+    pt_device_thread([&] {
+        cudaGetDevice(&dev);
+        b.reserve(1000);
+    }).join();
+    EXPECT(dev == 3 && b.p && pool(3).reserved == 1000 && fake::pools.size() == 1);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const struct { const char *name; int (*run)(); } checks[] = {
         {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry}, {"pinned", pinned}, {"other_device", other_device},
-        {"refused_wait", refused_wait},
+        {"refused_wait", refused_wait}, {"worker_device", worker_device},
     };
     for (const auto &c : checks)
         if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();

@@ -9,7 +9,7 @@ import pytest
 from tests.conftest import ROOT
 
 CPP = os.path.join(ROOT, "tests", "cpp")
-CHECKS = ["reuse_beside_live", "bound", "retry", "pinned", "other_device", "refused_wait"]
+CHECKS = ["reuse_beside_live", "bound", "retry", "pinned", "other_device", "refused_wait", "worker_device"]
 
 
 @pytest.fixture(scope="module")
@@ -93,3 +93,24 @@ def test_memory_kept_after_closing_stays_within_the_bound(gpu):
     ptb.release_memory()
     assert free - torch.cuda.mem_get_info()[0] <= slack
     t.close()
+
+
+@pytest.mark.gpu
+def test_a_table_on_another_device(gpu, libc):
+    """Build and query with device 1 current: the build's worker threads work there too."""
+    import numpy as np
+    import torch
+
+    import patchtable_b200 as ptb
+    from patchtable_b200 import synth
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    a, b = synth.pair(300, 200, 83)
+    got = []
+    for dev in range(2):
+        with torch.cuda.device(dev):
+            libc.srand(1)
+            t = ptb.PatchTable(ptb.PatchTableParams("-limit 1"), b)
+            got.append((t.table(), t.lookup(a)))
+            t.close()
+    assert all(np.array_equal(x, y) for x, y in zip(*got))
