@@ -351,10 +351,12 @@ int64_t pt_set_spin_limit(int64_t polls);
 
 /* Cap on the device memory this library holds at once (no reference counterpart): an allocation
    that would pass `bytes` fails as if the device were full and the call returns PT_OOM, leaving
-   earlier tables intact.  Process-wide; returns the previous cap; a negative value removes the
+   earlier tables intact.  What a device keeps for reuse (pt_release_memory) stays within it, beside
+   the buffers in use; CUDA rounds what it reserves up to whole granules (MiB).  Process-wide; returns the previous cap; a negative value removes the
    cap (the default).  Lets an application share the GPU with a fixed budget, and lets the tests
    drive the out-of-memory path without exhausting the device.  pt_device_bytes_in_use gives the
-   bytes the library currently holds (the zero-allocation query's static array is not counted). */
+   bytes of the library's buffers in use (the memory kept for reuse and the zero-allocation query's
+   static array are not counted). */
 int64_t pt_set_device_alloc_limit(int64_t bytes);
 int64_t pt_device_bytes_in_use(void);
 /* Gives the memory kept for reuse back: freed buffers stay with the library, at most 4 GiB of device

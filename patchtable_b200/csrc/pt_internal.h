@@ -43,9 +43,11 @@ void pt_count_launches(int n);
 /* Polls after which a device-side wait gives up (pt_set_spin_limit). */
 long long pt_spin_limit();
 /* Device-allocation accounting of DevBuf (pt_set_device_alloc_limit): admits `bytes` more or
-   refuses when the library's live device allocations would exceed the limit. */
+   refuses when the library's live device allocations would exceed the limit.  The room is what it
+   still admits, -1 without a limit. */
 bool pt_alloc_admit(size_t bytes);
 void pt_alloc_release(size_t bytes);
+long long pt_alloc_room();
 
 #define PT_TRY(expr) do { pt_status _s = (expr); if (_s != PT_OK) return _s; } while (0)
 
@@ -71,6 +73,8 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch);
 void pt_dev_free(void *p, size_t bytes, int dev, cudaStream_t st, bool scratch);
 cudaError_t pt_pinned_alloc(void **p, size_t bytes, size_t *got);
 void pt_pinned_free(void *p, size_t bytes, int dev);
+/* The limit was set: what is kept for reuse shrinks to it. */
+void pt_dev_cap_changed();
 
 /* A host thread that works on the calling thread's device (a new thread's own choice is device 0). */
 template<class F> std::thread pt_device_thread(F fn) {

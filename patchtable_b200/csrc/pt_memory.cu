@@ -18,6 +18,7 @@
    PT_PINNED_KEEP bytes per process, and given back before a failed allocation's second try.  Both are safe with any number of threads and streams. */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -74,15 +75,25 @@ cudaError_t device_pool(DevicePool **out) {
     return cudaSuccess;
 }
 
-/* Adds to the device's live bytes and moves the pool's release threshold with them; returns whether
-   more than that is reserved now. */
-bool set_keep(DevicePool &d, long long bytes) {
+/* What a device's pool has reserved and may keep reserved, beside its live bytes. */
+struct Reserve {
+    unsigned long long reserved, keep, live;
+    bool over() const { return reserved > keep; }
+};
+
+/* Adds to the device's live bytes and moves the pool's release threshold with them.  Under a cap
+   (pt_set_device_alloc_limit) what is kept for reuse stays within it too; a release still counts as
+   live there. */
+Reserve set_keep(DevicePool &d, long long bytes) {
+    const long long room = pt_alloc_room();
     std::lock_guard<std::mutex> lock(d.mu);
     d.live += bytes;
-    unsigned long long keep = d.live + PT_POOL_KEEP, reserved = 0;
+    unsigned long long spare = PT_POOL_KEEP, reserved = 0;
+    if (room >= 0) spare = std::min(spare, (unsigned long long) (room + (bytes < 0 ? -bytes : 0)));
+    unsigned long long keep = d.live + spare;
     cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (bytes < 0) cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
-    return reserved > keep;
+    if (bytes <= 0 || room >= 0) cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
+    return {reserved, keep, d.live};
 }
 
 /* Waits for the current device (d's) and gives b and the blocks held back before to the pool; holds
@@ -106,7 +117,7 @@ void wait_and_free(DevicePool &d, Block b) {
         bytes += (long long) x.bytes;
     }
     /* the threshold takes effect at a wait; the last of many frees may have none after it */
-    if (bytes && set_keep(d, -bytes)) cudaStreamSynchronize(d.st);
+    if (bytes && set_keep(d, -bytes).over()) cudaStreamSynchronize(d.st);
 }
 
 /* Makes a device current for a scope. */
@@ -139,7 +150,12 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch) 
     cudaError_t e = device_pool(&d);
     if (e != cudaSuccess) return e;
     if (!scratch) st = d->st;
-    set_keep(*d, (long long) bytes);
+    const bool capped = pt_alloc_room() >= 0;
+    Reserve r = set_keep(*d, (long long) bytes);
+    if (capped && r.reserved < r.live && r.reserved + bytes > r.keep) {      /* needs new memory, beyond the cap */
+        wait_and_free(*d, {});
+        cudaMemPoolTrimTo(d->pool, r.keep - bytes);
+    }
     e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
@@ -147,6 +163,10 @@ cudaError_t pt_dev_alloc(void **p, size_t bytes, cudaStream_t st, bool scratch) 
         cudaMemPoolTrimTo(d->pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
         if (e != cudaSuccess) cudaGetLastError();
+    }
+    if (capped && e == cudaSuccess && (r = set_keep(*d, 0)).over()) {        /* no free block was large enough */
+        wait_and_free(*d, {});
+        cudaMemPoolTrimTo(d->pool, r.keep);
     }
     /* a buffer of no stream must be usable on every stream when this returns */
     if (e == cudaSuccess && !scratch && (e = cudaStreamSynchronize(st)) != cudaSuccess) cudaFreeAsync(*p, st);
@@ -205,6 +225,16 @@ void pt_pinned_free(void *p, size_t bytes, int dev) {
         cudaGetLastError();
     }
     cudaFreeHost(p);
+}
+
+void pt_dev_cap_changed() {
+    for (DevicePool &d : g_pool) {
+        {
+            std::lock_guard<std::mutex> lock(d.mu);
+            if (!d.pool) continue;
+        }
+        if (set_keep(d, 0).over()) cudaStreamSynchronize(d.st);
+    }
 }
 
 extern "C" pt_status pt_release_memory(void) {

@@ -93,7 +93,16 @@ bool pt_alloc_admit(size_t bytes) {
 
 void pt_alloc_release(size_t bytes) { g_alloc_live.fetch_sub((long long) bytes); }
 
-extern "C" int64_t pt_set_device_alloc_limit(int64_t bytes) { return g_alloc_limit.exchange(bytes < 0 ? -1 : bytes); }
+long long pt_alloc_room() {
+    const long long lim = g_alloc_limit.load();
+    return lim < 0 ? -1 : std::max(0ll, lim - g_alloc_live.load());
+}
+
+extern "C" int64_t pt_set_device_alloc_limit(int64_t bytes) {
+    const int64_t old = g_alloc_limit.exchange(bytes < 0 ? -1 : bytes);
+    pt_dev_cap_changed();
+    return old;
+}
 
 extern "C" int64_t pt_device_bytes_in_use(void) { return g_alloc_live.load(); }
 

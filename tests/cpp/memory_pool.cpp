@@ -9,8 +9,14 @@
 #include <atomic>
 
 pt_status pt_fail(pt_status s, const char *, ...) { return s; }
-bool pt_alloc_admit(size_t) { return true; }
-void pt_alloc_release(size_t) {}
+static long long limit = -1, live = 0;
+bool pt_alloc_admit(size_t n) {
+    if (limit >= 0 && live + (long long) n > limit) return false;
+    live += n;
+    return true;
+}
+void pt_alloc_release(size_t n) { live -= n; }
+long long pt_alloc_room() { return limit < 0 ? -1 : limit < live ? 0 : limit - live; }
 
 #define EXPECT(c) do { if (!(c)) { printf("%s:%d: %s\n", __FILE__, __LINE__, #c); return 1; } } while (0)
 
@@ -150,10 +156,38 @@ static int worker_device() {
     return 0;
 }
 
+/* Under a cap, live buffers and what is kept for reuse stay within it together. */
+static int cap() {
+    cudaStream_t st;
+    cudaStreamCreateWithFlags(&st, 0);
+    DevBuf<char> table;
+    EXPECT(table.reserve(GiB) == cudaSuccess);
+    build(st);
+    EXPECT(pool().reserved == 3 * GiB + GiB / 2);
+    limit = 2 * GiB;
+    pt_dev_cap_changed();
+    EXPECT(pool().reserved <= 2 * GiB);
+    {
+        DevBuf<char> a(st), b;
+        EXPECT(a.reserve(GiB - 1) == cudaSuccess && pool().reserved <= 2 * GiB);
+        EXPECT(b.reserve(2) == cudaErrorMemoryAllocation);
+        a.release();
+        EXPECT(b.reserve(GiB - 2) == cudaSuccess && pool().reserved <= 2 * GiB);
+    }
+    EXPECT(pool().reserved <= 2 * GiB);
+    const int maps = fake::maps;
+    { DevBuf<char> a; EXPECT(a.reserve(GiB - 2) == cudaSuccess); }      /* kept, and used again */
+    EXPECT(fake::maps == maps);
+    limit = -1;
+    pt_dev_cap_changed();
+    EXPECT(pool().threshold == GiB + 4 * GiB);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const struct { const char *name; int (*run)(); } checks[] = {
         {"reuse_beside_live", reuse_beside_live}, {"bound", bound}, {"retry", retry}, {"pinned", pinned}, {"other_device", other_device},
-        {"refused_wait", refused_wait}, {"worker_device", worker_device},
+        {"refused_wait", refused_wait}, {"worker_device", worker_device}, {"cap", cap},
     };
     for (const auto &c : checks)
         if (argc == 2 && !strcmp(argv[1], c.name)) return c.run();

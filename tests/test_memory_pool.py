@@ -9,7 +9,7 @@ import pytest
 from tests.conftest import ROOT
 
 CPP = os.path.join(ROOT, "tests", "cpp")
-CHECKS = ["reuse_beside_live", "bound", "retry", "pinned", "other_device", "refused_wait", "worker_device"]
+CHECKS = ["reuse_beside_live", "bound", "retry", "pinned", "other_device", "refused_wait", "worker_device", "cap"]
 
 
 @pytest.fixture(scope="module")
@@ -114,3 +114,30 @@ def test_a_table_on_another_device(gpu, libc):
             got.append((t.table(), t.lookup(a)))
             t.close()
     assert all(np.array_equal(x, y) for x, y in zip(*got))
+
+
+@pytest.mark.gpu
+def test_memory_kept_stays_within_the_cap(gpu):
+    import torch
+
+    import patchtable_b200 as ptb
+    from patchtable_b200 import synth
+    a, b = synth.pair(60, 80, 84)
+    t = ptb.PatchTable(ptb.PatchTableParams("-limit 1"), b)
+    want = t.lookup(a)
+    ptb.release_memory()
+    used = ptb.device_bytes_in_use()
+    free = torch.cuda.mem_get_info()[0]
+    slack = 64 << 20                              # the pool reserves whole granules
+    t.batch([(4000, 4000)] * 4).close()
+    old = ptb.set_device_alloc_limit(used + (1 << 30))
+    try:
+        assert free - torch.cuda.mem_get_info()[0] <= (1 << 30) + slack
+        with pytest.raises(ptb.PatchTableError):
+            t.batch([(4000, 4000)] * 4)
+        t.batch([(1000, 4000)]).close()
+        assert (t.lookup(a) == want).all()
+        assert free - torch.cuda.mem_get_info()[0] <= (1 << 30) + slack
+    finally:
+        ptb.set_device_alloc_limit(old)
+    t.close()
