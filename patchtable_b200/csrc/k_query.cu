@@ -34,7 +34,6 @@ struct NextChoose {
     int use_done, do_kcoh, pass;
     int *ch_pos;
     float *ch_d;
-    unsigned long long *counters;
 };
 
 struct QPlan {
@@ -344,7 +343,6 @@ __device__ __forceinline__ float score_warp(const QPlan &q, const float *al, int
     if (valid) {
         const unsigned x = (unsigned) pt_x(cand);
         v = (((unsigned) pt_y(cand) * (unsigned) q.nline + (x >> 1)) << 1) | (x & 1);
-        rows += 8;
     }
     float d = finf();
     while (mask) {
@@ -352,7 +350,7 @@ __device__ __forceinline__ float score_warp(const QPlan &q, const float *al, int
         unsigned rest = mask;
 #pragma unroll
         for (int i = 0; i < 8; i++) rest &= rest - 1;
-        if (((mask & ~rest) >> lane) & 1) d = e;
+        if (((mask & ~rest) >> lane) & 1) { d = e; rows += EXIT && e == finf() ? 4 : 8; }      /* +inf: abandoned */
         mask = rest;
     }
     return d;
@@ -854,7 +852,6 @@ k_pull_desc(const QPlan q, const int *cur_pos, const float *cur_d,
         }
     }
     count_work(counters, ne, ne);
-    if (q.nx.ch_pos) count_work(q.nx.counters, l.ne, l.ne);
 }
 
 /* Step 4 as a pull: the best of the stored match and every neighbour's chosen offset applied to
@@ -1035,18 +1032,13 @@ pull_tile(const QPlan &c_q, float *at, const float *__restrict__ a, const int *c
                lists' state in registers and spills: 1080p 4.3 ms instead of 3.5. */
             Walk<false> w;
             w.start(c_q, live, bpos, bd);
-            ne = rows = 0;
             for (;;) {
                 const int c = w.next(c_q, c_q.nx.kcoh, c_q.nx.kc_done, c_q.nx.use_done, c_q.nx.do_kcoh, c_q.nx.pass, true, p);
                 if (!__any_sync(FULL, c >= 0)) break;
                 const float d = dist32<TP, DESC, true, D>(aq, c_q, c, c >= 0, w.dbest, rows);
-                if (c >= 0) {
-                    ne++;
-                    w.offer(c, d);
-                }
+                if (c >= 0) w.offer(c, d);
             }
             if (live) { c_q.nx.ch_pos[p] = w.best; c_q.nx.ch_d[p] = w.dch; }
-            count_work(c_q.nx.counters, ne, rows);
             return;
         }
     }
@@ -1108,8 +1100,7 @@ __global__ void __launch_bounds__(TP, min_ctas(LEAN ? CHOOSE_LEAN_LANES : CHOOSE
 k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
                const float *__restrict__ a, const int *cur_pos,
                const float *cur_d, const int *tcand, const int2 *__restrict__ kcoh, int do_table,
-               int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *counters,
-               unsigned long long *work) {
+               int *ch_pos, float *ch_d, int *kc_done, int use_done, unsigned long long *work) {
     extern __shared__ float at[];
     LearnedArgs none;
     none.cand = nullptr; none.conf = nullptr; none.threshold = 0.f; none.kcoh_confident = 0; none.counters = nullptr;
@@ -1123,7 +1114,7 @@ k_choose_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, l
         const long long o = g.patch_off;
         choose_tile<TP, false, LEAN>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
                                             cur_d ? cur_d + o : nullptr, tcand + o, kcoh, do_table, ch_pos + o, ch_d + o,
-                                            kc_done + o, use_done, counters, none, (ls % spr) * tile_w(TP),
+                                            kc_done + o, use_done, nullptr, none, (ls % spr) * tile_w(TP),
                                             (ls / spr) * tile_h(TP), g.eh);
     });
 }
@@ -1133,7 +1124,7 @@ __global__ void __launch_bounds__(TP, min_ctas(ONE ? PULL_ONE_LANES : PULL_LANES
 k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, long long nseg, int twi,
              const float *__restrict__ a, const int *cur_pos,
              const float *cur_d, const int *ch_pos, const float *ch_d,
-             int *nxt_pos, float *nxt_d, unsigned long long *counters, unsigned long long *work) {
+             int *nxt_pos, float *nxt_d, unsigned long long *work) {
     extern __shared__ float at[];
     for_each_tile(work, nseg, [&](long long s) {
         const int i = owner(imgs, n, s, twi);
@@ -1146,7 +1137,7 @@ k_pull_batch(const QPlan base, const PtBatchImage *__restrict__ imgs, int n, lon
         if (base.ann) q.ann = base.ann + 3 * o;        /* last pass: this image's NNF records */
         if (base.nx.ch_pos) { q.nx.ch_pos += o; q.nx.ch_d += o; q.nx.kc_done += o; }
         pull_tile<TP, R, false, ONE, NX>(q, at, a + 3 * g.pix_off, cur_pos ? cur_pos + o : nullptr,
-                                     cur_d ? cur_d + o : nullptr, ch_pos + o, ch_d + o, nxt_pos + o, nxt_d + o, counters,
+                                     cur_d ? cur_d + o : nullptr, ch_pos + o, ch_d + o, nxt_pos + o, nxt_d + o, nullptr,
                                      (ls % spr) * tile_w(TP), (ls / spr) * tile_h(TP), g.eh);
     });
 }
@@ -1407,7 +1398,6 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
     q.nx.pass = s.nx_pass;
     q.nx.ch_pos = s.nx_ch_pos;
     q.nx.ch_d = s.nx_ch_d;
-    q.nx.counters = s.nx_evals;
     if (q.adesc) {
         if (!q.bdesc || (s.ds != 8 && s.ds != 16) || q.nd < 3 || q.nd > s.ds)
             return pt_fail(PT_BAD_ARG, "descriptor query: store of %d floats for %d dimensions", s.ds, q.nd);
@@ -1594,7 +1584,7 @@ long long pt_batch_tiles(int twi, int ew, int eh) {
 pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
                                  const float *a, const int *cur_pos, const float *cur_d,
                                  const int *tcand, const int2 *kcoh, int do_table, int *ch_pos, float *ch_d, int *kc_done,
-                                 int use_done, unsigned long long *evals, unsigned long long *work, cudaStream_t st) {
+                                 int use_done, unsigned long long *work, cudaStream_t st) {
     QPlan q;
     PT_TRY(make_qplan(s, q));
     if (nseg <= 0) return PT_OK;
@@ -1602,10 +1592,10 @@ pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, 
 #define PT_CHOOSE_B(T) { const size_t sm = atile_bytes(T); \
         if (lean) { const int g = persistent_grid(k_choose_batch<T, true>, T, sm, nseg); \
             k_choose_batch<T, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, tcand, kcoh, do_table, \
-                                                      ch_pos, ch_d, kc_done, use_done, evals, work); } \
+                                                      ch_pos, ch_d, kc_done, use_done, work); } \
         else { const int g = persistent_grid(k_choose_batch<T>, T, sm, nseg); \
             k_choose_batch<T><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, tcand, kcoh, do_table, ch_pos, \
-                                                ch_d, kc_done, use_done, evals, work); } }
+                                                ch_d, kc_done, use_done, work); } }
     const bool lean = lean_choose(q);
     switch (BATCH_TW[twi]) {
         case 32: PT_CHOOSE_B(32) break;
@@ -1620,8 +1610,8 @@ pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, 
 
 pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
                                const float *a, const int *cur_pos, const float *cur_d, const int *ch_pos,
-                               const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *evals,
-                               unsigned long long *work, cudaStream_t st) {
+                               const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *work,
+                               cudaStream_t st) {
     QPlan q;
     PT_TRY(make_qplan(s, q));
     if (nseg <= 0) return PT_OK;
@@ -1629,13 +1619,13 @@ pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, in
 #define PT_PULL_B(T, RR) { const size_t sm = atile_bytes(T); \
         if (one) { const int g = persistent_grid(k_pull_batch<T, RR, true>, T, sm, nseg); \
             k_pull_batch<T, RR, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, \
-                                                        nxt_d, evals, work); } \
+                                                        nxt_d, work); } \
         else if (q.nx.ch_pos) { const int g = persistent_grid(k_pull_batch<T, RR, false, true>, T, sm, nseg); \
             k_pull_batch<T, RR, false, true><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, \
-                                                               nxt_pos, nxt_d, evals, work); } \
+                                                               nxt_pos, nxt_d, work); } \
         else { const int g = persistent_grid(k_pull_batch<T, RR>, T, sm, nseg); \
             k_pull_batch<T, RR><<<g, T, sm, st>>>(q, imgs, n, nseg, twi, a, cur_pos, cur_d, ch_pos, ch_d, nxt_pos, nxt_d, \
-                                                  evals, work); } }
+                                                  work); } }
     const bool one = one_pull(q) && !q.nx.ch_pos;
     const bool r1 = q.radius <= 1;
     switch (BATCH_TW[twi]) {

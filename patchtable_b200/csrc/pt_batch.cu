@@ -97,8 +97,8 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
         if (!fuse || i == 0)
             PT_TRY(pt_launch_choose_batch(qi, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
                                           i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, B->tcand.p,
-                                          v.kcoh, do_table, B->chpos.p, B->chd.p, B->kcdone.p, use_done, nullptr,
-                                          B->work.p + 1, st));
+                                          v.kcoh, do_table, B->chpos.p, B->chd.p, B->kcdone.p, use_done, B->work.p + 1,
+                                          st));
         if (p.do_prop) {
             QuerySetup qp = qs;
             qp.step = pt_pass_step(i, passes, jump);
@@ -114,7 +114,7 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
             }
             PT_TRY(pt_launch_pull_batch(qp, B->d_imgs.p, B->n, B->nseg[B->twi], B->twi, d_rgb,
                                         i == 0 ? nullptr : B->pos[cur].p, i == 0 ? nullptr : B->dd[cur].p, chpos[i & 1], chd[i & 1],
-                                        B->pos[1 - cur].p, B->dd[1 - cur].p, nullptr, B->work.p + 2, st));
+                                        B->pos[1 - cur].p, B->dd[1 - cur].p, B->work.p + 2, st));
             cur = 1 - cur;
         } else {
             PT_CUDA(cudaMemcpyAsync(B->pos[cur].p, B->chpos.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));

@@ -145,7 +145,6 @@ struct QuerySetup {
     int nx_use_done = 0, nx_do_kcoh = 0, nx_pass = 0;
     int *nx_ch_pos = nullptr;
     float *nx_ch_d = nullptr;
-    unsigned long long *nx_evals = nullptr;
     int pdl = 0;             /* may start while the kernel before it in the stream ends */
     cudaStream_t stream;
 };
@@ -233,11 +232,11 @@ long long pt_batch_tiles(int twi, int ew, int eh);
 pt_status pt_launch_choose_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
                                  const float *a, const int *cur_pos, const float *cur_d,
                                  const int *tcand, const int2 *kcoh, int do_table, int *ch_pos, float *ch_d, int *kc_done,
-                                 int use_done, unsigned long long *evals, unsigned long long *work, cudaStream_t st);
+                                 int use_done, unsigned long long *work, cudaStream_t st);
 pt_status pt_launch_pull_batch(const QuerySetup &s, const PtBatchImage *imgs, int n, long long nseg, int twi,
                                const float *a, const int *cur_pos, const float *cur_d, const int *ch_pos,
-                               const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *evals,
-                               unsigned long long *work, cudaStream_t st);
+                               const float *ch_d, int *nxt_pos, float *nxt_d, unsigned long long *work,
+                               cudaStream_t st);
 /* The batch's descriptor pass fused with the table step: tcand[p] = table[cell(p)] for every
    patch of every image, no descriptors stored. */
 pt_status pt_launch_descriptor_cells_batch(int ndims, int nchroma, const PtBatchImage *imgs, int n, long long ntiles,

@@ -779,8 +779,9 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     int jump = pt_default_jump(p, passes);
     int cur = 0;
     /* From the second pass on, a pull makes the next pass's choices in the same launch: choices
-       alternate between two pairs of arrays, since its neighbours still read the ones it started from. */
-    const bool fuse = passes > 1 && p.do_prop && !learned && pt_pull_chooses(qs, P);
+       alternate between two pairs of arrays, since its neighbours still read the ones it started from.
+       (Not under a profile, whose stages are apart.) */
+    const bool fuse = !prof && passes > 1 && p.do_prop && !learned && pt_pull_chooses(qs, P);
     int *const chpos[2] = {t->q_chpos.p, fuse ? t->q_chpos1.p : t->q_chpos.p};
     float *const chd[2] = {t->q_chd.p, fuse ? t->q_chd1.p : t->q_chd.p};
     for (int i = 0; i < passes; i++) {
@@ -816,7 +817,6 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
                 qp.nx_pass = i + 1;
                 qp.nx_ch_pos = chpos[(i + 1) & 1];
                 qp.nx_ch_d = chd[(i + 1) & 1];
-                qp.nx_evals = ctr;
             }
             PT_TRY(pt_launch_pull(qp, n, a_rgb, fresh && i == 0 ? nullptr : t->q_pos[cur].p,
                                   fresh && i == 0 ? nullptr : t->q_d[cur].p, chpos[i & 1], chd[i & 1],
