@@ -30,7 +30,8 @@ struct pt_batch {
     DevBuf<PtBatchImage> d_imgs;
     long long npix = 0, P = 0, ntiles = 0, nseg[PT_BATCH_NTW] = {0, 0, 0, 0};
     int twi = PT_BATCH_NTW - 1;           /* 256 query patches per CTA until tuned */
-    DevBuf<float> rgb;                    /* copy of a query buffer that shares memory with the NNF */
+    DevBuf<float> rgb;                    /* copy of a query buffer that shares memory with the NNF (reserved at
+                                             once: a run may be captured) */
     DevBuf<int> tcand, pos[2], chpos, chpos1, kcdone;
     DevBuf<float> dd[2], chd, chd1;       /* ch*1: choices a pull makes for the next pass */
     DevBuf<unsigned long long> work;      /* work counters of the persistent launches */
@@ -55,7 +56,6 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     /* the distance kernels read the images themselves: a buffer that shares memory with the NNF is copied */
     const size_t rgb_bytes = sizeof(float) * 3 * (size_t) B->npix;
     if (pt_overlap(d_rgb, rgb_bytes, d_ann, sizeof(double) * 3 * (size_t) B->P)) {
-        PT_CUDA(B->rgb.reserve(3 * (size_t) B->npix));
         PT_CUDA(cudaMemcpyAsync(B->rgb.p, d_rgb, rgb_bytes, cudaMemcpyDeviceToDevice, st));
         d_rgb = B->rgb.p;
     }
@@ -168,7 +168,7 @@ pt_status pt_batch_create(pt_table *t, int n, const int *h, const int *w, pt_bat
     B->ntiles = tiles;
     for (int k = 0; k < PT_BATCH_NTW; k++) B->nseg[k] = seg[k];
     auto fail = [&](pt_status s) { delete B; return s; };
-    if (B->d_imgs.reserve(n) || B->tcand.reserve(pat) ||
+    if (B->d_imgs.reserve(n) || B->rgb.reserve(3 * (size_t) pix) || B->tcand.reserve(pat) ||
         B->pos[0].reserve(pat) || B->pos[1].reserve(pat) || B->dd[0].reserve(pat) || B->dd[1].reserve(pat) ||
         B->chpos.reserve(pat) || B->chd.reserve(pat) || B->chpos1.reserve(pat) || B->chd1.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
         return fail(pt_fail(PT_OOM, "batch buffers for %lld pixels / %lld patches", pix, pat));
