@@ -32,8 +32,8 @@ struct pt_batch {
     int twi = PT_BATCH_NTW - 1;           /* 256 query patches per CTA until tuned */
     DevBuf<float> rgb;                    /* copy of a query buffer that shares memory with the NNF (reserved at
                                              once: a run may be captured) */
-    DevBuf<int> tcand, pos[2], chpos, chpos1, kcdone;
-    DevBuf<float> dd[2], chd, chd1;       /* ch*1: choices a pull makes for the next pass */
+    DevBuf<int> tcand, pos[2], chpos, kcdone;
+    DevBuf<float> dd[2], chd, chd1;       /* chd1: distances of the choices a pull makes for the next pass */
     DevBuf<unsigned long long> work;      /* work counters of the persistent launches */
     cudaStream_t cap_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -83,9 +83,10 @@ pt_status run(pt_batch *B, const float *d_rgb, double *d_ann, cudaStream_t st) {
     const int passes = pt_default_passes(p);
     const bool direct_out = p.do_prop && passes > 0;
     const int jump = pt_default_jump(p, passes);
-    /* from the second pass on, the choices are made by the pull before (as in single lookups) */
+    /* from the second pass on, the choices are made by the pull before (as in single lookups), the first
+       of them where the table entries were, which only the first choose reads */
     const bool fuse = passes > 1 && p.do_prop && pt_pull_chooses(qs, B->P);
-    int *const chpos[2] = {B->chpos.p, fuse ? B->chpos1.p : B->chpos.p};
+    int *const chpos[2] = {B->chpos.p, fuse ? B->tcand.p : B->chpos.p};
     float *const chd[2] = {B->chd.p, fuse ? B->chd1.p : B->chd.p};
     int cur = 0;
     for (int i = 0; i < passes; i++) {
@@ -170,7 +171,7 @@ pt_status pt_batch_create(pt_table *t, int n, const int *h, const int *w, pt_bat
     auto fail = [&](pt_status s) { delete B; return s; };
     if (B->d_imgs.reserve(n) || B->rgb.reserve(3 * (size_t) pix) || B->tcand.reserve(pat) ||
         B->pos[0].reserve(pat) || B->pos[1].reserve(pat) || B->dd[0].reserve(pat) || B->dd[1].reserve(pat) ||
-        B->chpos.reserve(pat) || B->chd.reserve(pat) || B->chpos1.reserve(pat) || B->chd1.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
+        B->chpos.reserve(pat) || B->chd.reserve(pat) || B->chd1.reserve(pat) || B->kcdone.reserve(pat) || B->work.reserve(3))
         return fail(pt_fail(PT_OOM, "batch buffers for %lld pixels / %lld patches", pix, pat));
     if (cudaMemcpy(B->d_imgs.p, B->imgs.data(), sizeof(PtBatchImage) * n, cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(pt_fail(PT_CUDA_ERR, "batch geometry upload"));

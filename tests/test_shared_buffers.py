@@ -55,3 +55,14 @@ def test_image_inside_the_field(gpu, libc, batched, captured):
     torch.cuda.synchronize()
     assert torch.equal(ann, want)
     t.close()
+
+
+def test_a_batch_holds_48_bytes_per_pixel_and_patch(gpu, libc):
+    """12 bytes per pixel (the image's copy) and 36 per patch: entries, choices and states."""
+    srand_all(libc, 1)
+    t = ptb.PatchTable(ptb.PatchTableParams("-limit 0.5"), synth.pair(40, 50, 30)[1])
+    sizes = [(400, 500), (333, 61), (8, 8)] * 3
+    before = ptb.device_bytes_in_use()
+    qb = t.batch(sizes)
+    assert ptb.device_bytes_in_use() - before <= 12 * qb.pixels + 36 * qb.patches + 4096
+    t.close()
