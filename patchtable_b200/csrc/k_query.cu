@@ -16,6 +16,7 @@
    already reaches the value it must beat (the partial sum can only grow). */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 
@@ -1411,6 +1412,17 @@ static pt_status make_qplan(const QuerySetup &s, QPlan &q) {
 int pt_row_lines(int bw) { return (bw - 7 + 1) / 2; }       /* lines of patch columns 0 .. bw - 8 */
 
 size_t pt_row_store_floats(int bw, int bh) { return (size_t) pt_row_lines(bw) * bh * 32; }
+
+void pt_row_image(const float *row, int bw, float *rgb) {
+    const int last = pt_row_lines(bw) - 1;
+    for (int x = 0; x < bw; x++) {
+        const int line = std::min(x / 2, last);
+        for (int ch = 0; ch < 3; ch++) {
+            const int i = 3 * (x - 2 * line) + ch;
+            rgb[3 * x + ch] = row[32 * (size_t) line + 8 * (i & 3) + i / 4];
+        }
+    }
+}
 
 pt_status pt_launch_row_store(const float4 *b, int bw, int bh, float *out, cudaStream_t st) {
     const long long n = (long long) pt_row_store_floats(bw, bh);

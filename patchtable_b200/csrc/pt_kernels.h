@@ -185,6 +185,8 @@ inline int pt_pass_step(int i, int n, int jump) {
    floats, and the kernel that writes it from the RGBA image. */
 int pt_row_lines(int bw);
 size_t pt_row_store_floats(int bw, int bh);
+/* An image row (3 floats per pixel) from its lines. */
+void pt_row_image(const float *row, int bw, float *rgb);
 pt_status pt_launch_row_store(const float4 *b, int bw, int bh, float *out, cudaStream_t st);
 pt_status pt_launch_init(int n, int pos, float d, int *cur_pos, float *cur_d, cudaStream_t st);
 pt_status pt_launch_choose(const QuerySetup &s, int n, const float *a, const int *cur_pos, const float *cur_d,

@@ -121,7 +121,7 @@ struct pt_table {
     cudaStream_t st = nullptr;
     bool own_stream = false;
     cudaStream_t st2 = nullptr;       /* the build's second stream (range and partition) */
-    DevBuf<float4> b_rgba;
+    DevBuf<float4> b_rgba;            /* b until the k-coherence set is built; from then on the row store holds it */
     DevBuf<float> b_row;              /* row store of b the query's distances read (pt_launch_row_store) */
     DevBuf<float> b_desc;
     DevBuf<int> allowed;
@@ -565,6 +565,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     t->build_ms[PT_BUILD_PARTITION] = part_ms;
     t->build_ms[PT_BUILD_SHUFFLE] = shuffle_ms;
     if (order_xy.empty()) return pt_fail(PT_BAD_ARG, "no allowed patches");
+    t->b_rgba.release();
     {
         DevBuf<int> d_order(t->st);
         PT_CUDA(d_order.reserve(order_xy.size()));
@@ -1142,14 +1143,20 @@ pt_status save_impl(const pt_table *t, const char *filename) {
     if (t->desc_mode || t->pca) return pt_fail(PT_UNSUPPORTED, "saving a descriptor mode or PCA table");
     const int h = t->h, w = t->w, nd = t->nd;
     std::vector<int> cells((size_t) t->ncells);
-    std::vector<float4> rgba((size_t) h * w);
     std::vector<float> desc((size_t) t->eh * t->ew * t->ds);
     PT_CUDA(cudaMemcpyAsync(cells.data(), t->table.p, sizeof(int) * cells.size(), cudaMemcpyDeviceToHost, t->st));
-    PT_CUDA(cudaMemcpyAsync(rgba.data(), t->b_rgba.p, sizeof(float4) * rgba.size(), cudaMemcpyDeviceToHost, t->st));
     PT_CUDA(cudaMemcpyAsync(desc.data(), t->b_desc.p, sizeof(float) * desc.size(), cudaMemcpyDeviceToHost, t->st));
     PT_CUDA(cudaStreamSynchronize(t->st));
     std::vector<float> b0((size_t) h * w * 3);
-    for (size_t i = 0; i < rgba.size(); i++) { b0[3 * i] = rgba[i].x; b0[3 * i + 1] = rgba[i].y; b0[3 * i + 2] = rgba[i].z; }
+    /* b from its row store, some rows at a time */
+    const size_t pitch = pt_row_store_floats(w, 1);
+    std::vector<float> rows(pitch * std::min(h, 64));
+    for (int y0 = 0; y0 < h; y0 += 64) {
+        const int n = std::min(64, h - y0);
+        PT_CUDA(cudaMemcpyAsync(rows.data(), t->b_row.p + y0 * pitch, sizeof(float) * n * pitch, cudaMemcpyDeviceToHost, t->st));
+        PT_CUDA(cudaStreamSynchronize(t->st));
+        for (int y = 0; y < n; y++) pt_row_image(rows.data() + y * pitch, w, b0.data() + (size_t) (y0 + y) * w * 3);
+    }
     /* wh0 holds the descriptor of the patch with top-left (x, y) at (y + 7, x + 7); the partial
        windows of the reference's "full" padding are not kept by this library and are written as 0 */
     std::vector<float> wh0((size_t) (h + 7) * (w + 7) * nd, 0.f);
@@ -1275,6 +1282,8 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
     /* the file has no k-coherence set (the reference's load leaves it empty); it is rebuilt from
        the stored descriptors */
     if (p.kcoherence > 0) PT_TRY(build_kcoherence(t.get(), std::vector<int>()));
+    PT_CUDA(cudaStreamSynchronize(t->st));
+    t->b_rgba.release();
     t->nslices = nslices;
     t->stride.assign(G, 1);
     t->ncells = 1;

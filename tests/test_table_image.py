@@ -1,0 +1,48 @@
+"""A finished table holds its image once, as the row store of the query: 64 bytes per pixel.  A saved file's
+b0 is read back from it, at every width of a row's last line."""
+import numpy as np
+import pytest
+
+import patchtable_b200 as ptb
+from patchtable_b200 import synth
+from tests.conftest import srand_all
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w", [8, 9, 10, 11, 46, 47])
+@pytest.mark.parametrize("h", [8, 63, 65])
+def test_saved_image_is_the_image(gpu, libc, tmp_path, h, w):
+    _, b = synth.pair(h, w, 12)
+    b[0, 0, 0] = -0.0
+    p = ptb.PatchTableParams("-limit 0.01")
+    p.kcoherence = 0
+    srand_all(libc, 1)
+    t = ptb.PatchTable(p, b)
+    t.save(tmp_path / "t.bin")
+    assert np.ascontiguousarray(b).tobytes() in (tmp_path / "t.bin").read_bytes()
+    t.close()
+    t = ptb.PatchTable.load(p, tmp_path / "t.bin")
+    t.save(tmp_path / "u.bin")
+    assert (tmp_path / "t.bin").read_bytes() == (tmp_path / "u.bin").read_bytes()
+    t.close()
+
+
+@pytest.mark.parametrize("loaded", [False, True])
+@pytest.mark.parametrize("kcoherence", [0, 4])
+def test_bytes_of_a_table(gpu, libc, tmp_path, loaded, kcoherence):
+    h, w = 400, 500
+    _, b = synth.pair(h, w, 13)
+    p = ptb.PatchTableParams("-limit 0.05")
+    p.kcoherence = kcoherence
+    before = ptb.device_bytes_in_use()
+    srand_all(libc, 1)
+    t = ptb.PatchTable(p, b)
+    if loaded:
+        t.save(tmp_path / "t.bin")
+        t.close()
+        t = ptb.PatchTable.load(p, tmp_path / "t.bin")
+    cells, patches = t.table().size, (h - 7) * (w - 7)
+    image, descriptors, bins = 64 * h * w, 32 * patches, p.ndims * 16384 * 4
+    assert ptb.device_bytes_in_use() - before <= image + descriptors + 4 * cells + 8 * kcoherence * patches + bins + 65536
+    t.close()
