@@ -230,7 +230,7 @@ k_descriptor(const DescPlan c_plan, const float *__restrict__ rgb, int h, int w,
 __global__ void __launch_bounds__(NT, 5)
 k_descriptor_cells(const DescPlan c_plan, const CellPlan cp, const float *__restrict__ rgb, int h, int w, int convert,
                    int eh, int ew, int ty0) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");    /* the choose may stage its tiles */
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");    /* the choose may start: it waits before it reads */
     extern __shared__ __align__(16) float smem[];
     desc_tile<true>(c_plan, smem, rgb, h, w, convert, nullptr, nullptr, 0, eh, ew, blockIdx.x * TW, (blockIdx.y + ty0) * TH,
                     &cp, cp.tcand);

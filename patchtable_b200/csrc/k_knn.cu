@@ -700,7 +700,7 @@ pt_status pt_launch_knn(const float *train, int N, int nd, const float *qdesc, i
     for (int d = 0; d < nd; d++) qz.scale[d] = rmax > 0.f ? (float) ((1u << qz.bits) - 1) / rmax : 0.f;
     /* sort train points and queries along the curve */
     DevBuf<unsigned long long> codes(st), codes2(st);
-    DevBuf<int> idx(st), perm(st), qidx(st), qorder(st), sidx(st);
+    DevBuf<int> idx(st), perm(st), qorder(st);
     DevBuf<float> sp(st);
     PT_CUDA(codes.reserve(std::max(N, Q)));
     PT_CUDA(codes2.reserve(std::max(N, Q)));

@@ -195,7 +195,7 @@ __device__ __forceinline__ float quad_total(const float (&acc)[4]) {
    shared memory once for all of them (11 rows instead of 32).
 
    Bound: the L1 data pipe (128 bytes per clock: 256 wavefronts for 32 candidates' lines, 66 for the
-   query rows, 24 for the exchanges) at 83 % of its peak in the general pull, issue slots at 60 %.
+   query rows, 24 for the exchanges) at 77-82 % of its peak in the general pulls, issue slots at 53-64 %.
    The gather this replaced -- each lane its own candidate's 8 pixels, four 32-byte loads from 32
    different lines, 24 shared loads per row -- spent one wavefront on every lane's load and ran at
    89 % of the same pipe: at 1080p the lean choose took 0.265 ms (now 0.150), the one-candidate pull

@@ -29,7 +29,7 @@
                order of the reference's next frontier list.
    A filled cell holds its packed position (below 2^30), an empty one 0xffffffff, and a claimed one
    the claim's key, 2^30 + (element, edge), which its winner overwrites: the claims need no array of
-   their own while every key fits (FUSED), and a neighbour's one read says whether it is empty and
+   their own while every key fits, and a neighbour's one read says whether it is empty and
    whether an earlier element already holds it.
    The filled table is therefore bit-identical to the reference's.  Data written by other CTAs in
    an earlier phase is read with L2-only loads (ld.global.cg), never from a CTA's own L1. */
@@ -64,7 +64,7 @@ struct CellBuild {
     const int *order_xy;         /* packed position of each shuffle rank */
     unsigned *table;
     long long ncells;
-    unsigned *claim;             /* the table itself (FUSED), or one key per cell */
+    unsigned *claim;             /* the table itself while the keys fit, or one key per cell */
     unsigned key_base;
     int ebits;                   /* edge bits of a key */
     unsigned div_mul[PT_DESC_MAX];   /* division by nslices: floor(x / n) = umulhi(x, mul) >> shift for x < 2^31 */
@@ -203,11 +203,12 @@ __device__ __forceinline__ void claim_neighbours(const CellBuild &a, unsigned *e
     if (won) atomicXor(emask + i, won);
 }
 
-/* Bound: the latency of the levels' random accesses (98 M elements over 20 levels in a 1920x1080
+/* Bound: the latency of the levels' random accesses (98 M elements over 25 levels in a 1920x1080
    table).  6.4 ms there, of which claims 2.9, counts 0.16, emission 2.8 and the rest 0.5 ms; 14.8 ms
    (6.5, 4.2, 3.2, 0.9) with claims in an array of their own, one dependent read per edge with 64-bit
    divisions, a count phase that read every claim again and lists written a thread's run at a time.
-   Claims unrolled over 8 dimensions instead of 6 take 3.2 ms; 6 CTAs per SM instead of 4, 3.5. */
+   Claims unrolled over 8 dimensions instead of 6 take 3.2 ms; a register cap of 5 CTAs per SM (3 fit
+   as compiled, 80 registers) changes nothing, one of 6 makes the whole build 7.3. */
 template<int MAXG>
 __global__ void __launch_bounds__(NT) k_table_build(const CellBuild a) {
     __shared__ Shared sh;

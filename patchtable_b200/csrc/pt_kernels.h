@@ -38,8 +38,8 @@ pt_status pt_launch_descriptor_input(const float *in, int H, int W, int nd, int 
 
 /* k_build.cu */
 /* Device scratch of the range and partition stages.  The build runs them beside the k-coherence
-   search, so the scratch is owned by the caller and freed after both have finished: a cudaFree
-   inside the stages would wait for the whole device, the search included. */
+   search; the scratch belongs to the caller, is used on the stages' stream only and is released in
+   that stream's order, which waits for nothing. */
 #ifdef __CUDACC__
 struct PtPartScratch {
     DevBuf<float> pmin, pmax, keys, sorted, picked;
@@ -118,7 +118,8 @@ struct QuerySetup {
     int kc_try = 0;          /* k-coherence neighbours tried per patch (0 = all kcoherence) */
     int step = 1;            /* neighbour spacing of a pull pass */
     int pull_max = 0;        /* most neighbour candidates a pull scores per patch (0 = all) */
-    int tile = 0;            /* query patches per CTA in choose / pull: 32, 64, 128, 256 (0 = 64) */
+    int tile = 0;            /* query patches per CTA in choose / pull: 32, 64, 128, 256 (0: 128, or four
+                                warps on a tile of 32 in the pulls of a small image) */
     int row0 = 0, rows = 0;  /* patch rows [row0, row0 + rows) of a single-image launch (rows 0 = all) */
     const float *brow = nullptr;  /* row store of the table image (pt_launch_row_store) */
     const int *allowed = nullptr; /* b patches a match may use (allowed[p] == allowed_index), or NULL */

@@ -521,7 +521,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         if (e != cudaSuccess) { shuffler.join(); return pt_fail(PT_CUDA_ERR, "stream: %s", cudaGetErrorString(e)); }
     }
     double part_ms = 0.0;
-    PtPartScratch part_scratch(t->st2);       /* freed when the build returns, after the search has ended */
+    PtPartScratch part_scratch(t->st2);
     std::string part_err;
     pt_status part_st = PT_OK;
     std::thread partitioner = pt_device_thread([&] {
