@@ -344,6 +344,7 @@ __device__ __forceinline__ float score_warp(const QPlan &q, const float *al, int
     if (valid) {
         const unsigned x = (unsigned) pt_x(cand);
         v = (((unsigned) pt_y(cand) * (unsigned) q.nline + (x >> 1)) << 1) | (x & 1);
+        rows += 8;
     }
     float d = finf();
     while (mask) {
@@ -351,9 +352,10 @@ __device__ __forceinline__ float score_warp(const QPlan &q, const float *al, int
         unsigned rest = mask;
 #pragma unroll
         for (int i = 0; i < 8; i++) rest &= rest - 1;
-        if (((mask & ~rest) >> lane) & 1) { d = e; rows += EXIT && e == finf() ? 4 : 8; }      /* +inf: abandoned */
+        if (((mask & ~rest) >> lane) & 1) d = e;
         mask = rest;
     }
+    if (EXIT && valid && d == finf()) rows -= 4;      /* abandoned */
     return d;
 }
 
