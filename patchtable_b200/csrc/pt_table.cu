@@ -121,8 +121,7 @@ struct pt_table {
     cudaStream_t st = nullptr;
     bool own_stream = false;
     cudaStream_t st2 = nullptr;       /* the build's second stream (range and partition) */
-    DevBuf<float4> b_rgba;            /* b until the k-coherence set is built; from then on the row store holds it */
-    DevBuf<float> b_row;              /* row store of b the query's distances read (pt_launch_row_store) */
+    DevBuf<float> b_row;              /* b, as the row store the query's distances read (pt_launch_row_store) */
     DevBuf<float> b_desc;
     DevBuf<int> allowed;
     std::vector<int> nslices;
@@ -313,7 +312,8 @@ bool host_allowed(const std::vector<int> &allowed, int idx, int py, int px, int 
     return allowed.empty() || allowed[(size_t) py * ew + px] == idx;
 }
 
-pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
+/* b_rgba: b's pixels (NULL in descriptor mode). */
+pt_status build_kcoherence(pt_table *t, const float4 *b_rgba, const std::vector<int> &allowed) {
     const pt_params &p = t->p;
     const int ew = t->ew, eh = t->eh;
     {
@@ -339,7 +339,7 @@ pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
             PT_CUDA(train.reserve((size_t) N * t->nd)); PT_CUDA(qdesc.reserve((size_t) Q * t->nd));
             PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_trows.p, N, train.p, t->st));
             PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_qrows.p, Q, qdesc.p, t->st));
-            return pt_kcoherence(t->b_rgba.p, t->w, t->desc_mode ? t->b_desc.p : nullptr, t->ds, t->ew, train.p, N, t->nd,
+            return pt_kcoherence(b_rgba, t->w, t->desc_mode ? t->b_desc.p : nullptr, t->ds, t->ew, train.p, N, t->nd,
                                  d_tpos.p, qdesc.p, d_qpos.p, d_qcell.p, Q, d_seg.p, nseg, p.kcoherence,
                                  p.kcoherence_min_dist, t->kcoh.p, &t->kc_list, t->st);
         }
@@ -381,7 +381,7 @@ pt_status build_kcoherence(pt_table *t, const std::vector<int> &allowed) {
     PT_CUDA(cudaMemcpyAsync(d_seg.p, seg.data(), sizeof(int) * nseg, cudaMemcpyHostToDevice, t->st));
     PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_trows.p, N, train.p, t->st));
     PT_TRY(pt_gather_rows(t->b_desc.p, t->ds, t->nd, d_qrows.p, Q, qdesc.p, t->st));
-    PT_TRY(pt_kcoherence(t->b_rgba.p, t->w, t->desc_mode ? t->b_desc.p : nullptr, t->ds, t->ew, train.p, N, t->nd,
+    PT_TRY(pt_kcoherence(b_rgba, t->w, t->desc_mode ? t->b_desc.p : nullptr, t->ds, t->ew, train.p, N, t->nd,
                          d_tpos.p, qdesc.p, d_qpos.p, d_qcell.p, Q, d_seg.p, nseg, p.kcoherence, p.kcoherence_min_dist,
                          t->kcoh.p, &t->kc_list, t->st));
     return PT_OK;
@@ -432,6 +432,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         return PT_OK;
     };
 
+    DevBuf<float4> b_rgba(t->st);     /* given back once the k-coherence set is built: the row store holds b too */
     if (t->desc_mode) {
         DevBuf<float> in(t->st);
         const size_t nin = (size_t) h * w * channels;
@@ -441,11 +442,11 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         PT_TRY(pt_launch_descriptor_input(in.p, h, w, channels, t->in_padded, t->b_desc.p, t->ds, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     } else {
-    /* Descriptor of b (get_padded_descriptor, patchtable.h:2492-2546) and the RGBA copy kept as b0. */
+    /* Descriptor of b (get_padded_descriptor, patchtable.h:2492-2546), its RGBA copy and row store. */
         DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve((size_t) h * w * 3));
         PT_CUDA(cudaMemcpyAsync(rgb.p, b, sizeof(float) * (size_t) h * w * 3, cudaMemcpyHostToDevice, t->st));
-        PT_CUDA(t->b_rgba.reserve((size_t) h * w));
+        PT_CUDA(b_rgba.reserve((size_t) h * w));
         PT_CUDA(t->b_desc.reserve((size_t) P * t->ds));
         if (p.dim_algo == 1) {
             /* reduce_dim with TABLE_DIM_ALGO_PCA (patchtable.h:1709-1713): fit on b, then project */
@@ -456,11 +457,11 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
             PT_CUDA(t->pca_basis.reserve(basis.size()));
             PT_CUDA(cudaMemcpyAsync(t->pca_mean.p, mean.data(), sizeof(float) * mean.size(), cudaMemcpyHostToDevice, t->st));
             PT_CUDA(cudaMemcpyAsync(t->pca_basis.p, basis.data(), sizeof(float) * basis.size(), cudaMemcpyHostToDevice, t->st));
-            PT_TRY(pt_launch_pca(rgb.p, h, w, pt_color_mode(p), t->b_rgba.p, t->pca_mean.p, t->pca_basis.p, p.ndims,
+            PT_TRY(pt_launch_pca(rgb.p, h, w, pt_color_mode(p), b_rgba.p, t->pca_mean.p, t->pca_basis.p, p.ndims,
                                  t->b_desc.p, t->ds, t->st));
             PT_CUDA(cudaStreamSynchronize(t->st));     /* the host vectors go out of scope */
         } else {
-            PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, rgb.p, h, w, pt_color_mode(p), t->b_rgba.p, t->b_desc.p,
+            PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, rgb.p, h, w, pt_color_mode(p), b_rgba.p, t->b_desc.p,
                                         t->ds, t->st));
         }
         if (wh0) {
@@ -473,7 +474,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
             PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
         }
         PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
-        PT_TRY(pt_launch_row_store(t->b_rgba.p, w, h, t->b_row.p, t->st));
+        PT_TRY(pt_launch_row_store(b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     std::vector<int> allowed_h;
@@ -555,7 +556,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         if (part_st != PT_OK) part_err = pt_last_error();
     });
     pt_status kc_st = PT_OK;
-    if (p.kcoherence > 0) kc_st = build_kcoherence(t.get(), allowed_h);
+    if (p.kcoherence > 0) kc_st = build_kcoherence(t.get(), b_rgba.p, allowed_h);
     if (kc_st == PT_OK) kc_st = stage_done(PT_BUILD_KCOHERENCE);
     partitioner.join();
     shuffler.join();
@@ -565,7 +566,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     t->build_ms[PT_BUILD_PARTITION] = part_ms;
     t->build_ms[PT_BUILD_SHUFFLE] = shuffle_ms;
     if (order_xy.empty()) return pt_fail(PT_BAD_ARG, "no allowed patches");
-    t->b_rgba.release();
+    b_rgba.release();
     {
         DevBuf<int> d_order(t->st);
         PT_CUDA(d_order.reserve(order_xy.size()));
@@ -1262,12 +1263,13 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
     PT_CUDA(cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking));
     t->own_stream = true;
     const long long P = (long long) t->eh * t->ew;
+    DevBuf<float4> b_rgba(t->st);     /* given back once the k-coherence set is built */
     {
         DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve(b0.size()));
         PT_CUDA(cudaMemcpyAsync(rgb.p, b0.data(), sizeof(float) * b0.size(), cudaMemcpyHostToDevice, t->st));
-        PT_CUDA(t->b_rgba.reserve((size_t) h * w));
-        PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, rgb.p, h, w, pt_color_mode(p), t->b_rgba.p, nullptr, t->ds, t->st));
+        PT_CUDA(b_rgba.reserve((size_t) h * w));
+        PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, rgb.p, h, w, pt_color_mode(p), b_rgba.p, nullptr, t->ds, t->st));
         std::vector<float> packed((size_t) P * t->ds, 0.0f);
         for (int y = 0; y < t->eh; y++)
             for (int x = 0; x < t->ew; x++)
@@ -1276,14 +1278,13 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
         PT_CUDA(t->b_desc.reserve(packed.size()));
         PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
         PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
-        PT_TRY(pt_launch_row_store(t->b_rgba.p, w, h, t->b_row.p, t->st));
+        PT_TRY(pt_launch_row_store(b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     /* the file has no k-coherence set (the reference's load leaves it empty); it is rebuilt from
        the stored descriptors */
-    if (p.kcoherence > 0) PT_TRY(build_kcoherence(t.get(), std::vector<int>()));
-    PT_CUDA(cudaStreamSynchronize(t->st));
-    t->b_rgba.release();
+    if (p.kcoherence > 0) PT_TRY(build_kcoherence(t.get(), b_rgba.p, std::vector<int>()));
+    b_rgba.release();
     t->nslices = nslices;
     t->stride.assign(G, 1);
     t->ncells = 1;

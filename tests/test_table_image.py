@@ -46,3 +46,26 @@ def test_bytes_of_a_table(gpu, libc, tmp_path, loaded, kcoherence):
     image, descriptors, bins = 64 * h * w, 32 * patches, p.ndims * 16384 * 4
     assert ptb.device_bytes_in_use() - before <= image + descriptors + 4 * cells + 8 * kcoherence * patches + bins + 65536
     t.close()
+
+
+def test_a_load_waits_for_no_other_stream(gpu, libc, tmp_path):
+    """A load beside a kernel of about a second on another stream ends before that kernel: the image's
+    copy goes back in the load's own order.  (A build's cooperative launch waits for a free GPU.)"""
+    import torch
+    _, b = synth.pair(60, 80, 14)
+    p = ptb.PatchTableParams("-limit 0.05")
+    path = tmp_path / "t.bin"
+    srand_all(libc, 1)
+    tables = [ptb.PatchTable(p, b)]
+    tables[0].save(path)
+    for _ in range(2):                            # kernels loaded, memory in the pool
+        tables.append(ptb.PatchTable.load(p, path))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(2_000_000_000)
+    tables.append(ptb.PatchTable.load(p, path))
+    assert not side.query()
+    side.synchronize()
+    for t in tables:
+        t.close()
