@@ -28,7 +28,6 @@
 namespace {
 
 constexpr unsigned long long PT_POOL_KEEP = 4ull << 30;
-constexpr unsigned long long PT_KEEP_STEP = 64ull << 20;
 constexpr size_t PT_PINNED_KEEP = 256u << 20;
 constexpr int MAX_DEVICES = 64;
 
@@ -39,7 +38,6 @@ struct DevicePool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t st = nullptr;            /* order of the buffers that belong to no stream */
     unsigned long long live = 0;          /* bytes of the buffers in use */
-    unsigned long long keep = 0;          /* the release threshold that was set */
     std::vector<Block> held;              /* released, but their device could not be waited for */
 };
 DevicePool g_pool[MAX_DEVICES];
@@ -83,21 +81,17 @@ struct Reserve {
     bool over() const { return reserved > keep; }
 };
 
-/* Adds to the device's live bytes and moves the pool's release threshold with them, in whole steps of
-   64 MiB: setting it costs a microsecond, and a lookup of a new size reserves some ten buffers (the first
-   one of 48 x 64: 163 us with a call for each, 153 with none).  Under a cap
+/* Adds to the device's live bytes and moves the pool's release threshold with them.  Under a cap
    (pt_set_device_alloc_limit) what is kept for reuse stays within it too; a release still counts as
    live there. */
 Reserve set_keep(DevicePool &d, long long bytes) {
     const long long room = pt_alloc_room();
     std::lock_guard<std::mutex> lock(d.mu);
     d.live += bytes;
-    unsigned long long keep = d.live / PT_KEEP_STEP * PT_KEEP_STEP + PT_POOL_KEEP, reserved = 0;
-    if (room >= 0) keep = std::min(keep, d.live + (unsigned long long) (room + (bytes < 0 ? -bytes : 0)));
-    if (keep != d.keep) {
-        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        d.keep = keep;
-    }
+    unsigned long long spare = PT_POOL_KEEP, reserved = 0;
+    if (room >= 0) spare = std::min(spare, (unsigned long long) (room + (bytes < 0 ? -bytes : 0)));
+    unsigned long long keep = d.live + spare;
+    cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (bytes <= 0 || room >= 0) cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
     return {reserved, keep, d.live};
 }

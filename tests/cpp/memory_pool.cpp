@@ -129,9 +129,9 @@ static int refused_wait() {
     EXPECT(fake::host.empty());                           /* not kept */
     DevBuf<char> c, d;
     EXPECT(c.reserve(1000) == cudaSuccess && c.p != b0);
-    EXPECT(g_pool[0].live == 2000);
+    EXPECT(pool().threshold == 4 * GiB + 2000);
     c.release();                                          /* waits, and frees b's block too */
-    EXPECT(g_pool[0].live == 0 && pool().threshold == 4 * GiB);
+    EXPECT(pool().threshold == 4 * GiB);
     EXPECT(d.reserve(1000) == cudaSuccess && (d.p == b0 || pool().blocks.size() == 2));
     d.release();
     {
