@@ -110,7 +110,7 @@ pt_status pt_kcoherence(const float4 *b_rgba, int bw, const float *bdesc, int ds
                         const float *qdesc, const int *qpos, const int *qcell, int Q, const int *seg_start, int nseg,
                         int kc, int min_dist, int2 *kcoh, int *max_knn_out, cudaStream_t st);
 
-/* k_query.cu */
+/* k_query.cu, k_query_tiles.cu, k_query_desc.cu, k_query_batch.cu */
 struct QuerySetup {
     int aw, ah, bw, bh;
     double prop_scale, triangle_factor;
