@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <optional>
 #include <string>
 #include <thread>
 #include <vector>
@@ -387,6 +388,14 @@ pt_status build_kcoherence(pt_table *t, const float4 *b_rgba, const std::vector<
     return PT_OK;
 }
 
+/* The table's image as the queries read it, in place of the build's copy. */
+pt_status store_rows(pt_table *t, DevBuf<float4> &b_rgba) {
+    PT_CUDA(t->b_row.reserve(pt_row_store_floats(t->w, t->h)));
+    PT_TRY(pt_launch_row_store(b_rgba.p, t->w, t->h, t->b_row.p, t->st));
+    b_rgba.release();
+    return PT_OK;
+}
+
 pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int channels, const float *wh0,
                       const int32_t *allowed, pt_table **out) {
     if (!out) return pt_fail(PT_BAD_ARG, "null output pointer");
@@ -432,7 +441,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         return PT_OK;
     };
 
-    DevBuf<float4> b_rgba(t->st);     /* given back once the k-coherence set is built: the row store holds b too */
+    DevBuf<float4> b_rgba(t->st);     /* b during the build, whose peak a row store would add four times as much to */
     if (t->desc_mode) {
         DevBuf<float> in(t->st);
         const size_t nin = (size_t) h * w * channels;
@@ -442,7 +451,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         PT_TRY(pt_launch_descriptor_input(in.p, h, w, channels, t->in_padded, t->b_desc.p, t->ds, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     } else {
-    /* Descriptor of b (get_padded_descriptor, patchtable.h:2492-2546), its RGBA copy and row store. */
+    /* Descriptor of b (get_padded_descriptor, patchtable.h:2492-2546), and its RGBA copy. */
         DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve((size_t) h * w * 3));
         PT_CUDA(cudaMemcpyAsync(rgb.p, b, sizeof(float) * (size_t) h * w * 3, cudaMemcpyHostToDevice, t->st));
@@ -473,8 +482,6 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
                         packed[((size_t) y * t->ew + x) * t->ds + d] = wh0[((size_t) (y + 7) * (w + 7) + (x + 7)) * t->nd + d];
             PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
         }
-        PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
-        PT_TRY(pt_launch_row_store(b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     std::vector<int> allowed_h;
@@ -522,7 +529,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
         if (e != cudaSuccess) { shuffler.join(); return pt_fail(PT_CUDA_ERR, "stream: %s", cudaGetErrorString(e)); }
     }
     double part_ms = 0.0;
-    PtPartScratch part_scratch(t->st2);
+    std::optional<PtPartScratch> part_scratch(std::in_place, t->st2);
     std::string part_err;
     pt_status part_st = PT_OK;
     std::thread partitioner = pt_device_thread([&] {
@@ -530,7 +537,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
             cudaStream_t s2 = t->st2;
             t->min_val.assign(t->G, 0.f);
             t->max_val.assign(t->G, 0.f);
-            PT_TRY(pt_launch_minmax(part_scratch, t->b_desc.p, t->ds, t->G, P, t->allowed.p, p.allowed_index, t->min_val.data(),
+            PT_TRY(pt_launch_minmax(*part_scratch, t->b_desc.p, t->ds, t->G, P, t->allowed.p, p.allowed_index, t->min_val.data(),
                                     t->max_val.data(), s2));
             t->range.resize(t->G);
             for (int d = 0; d < t->G; d++) t->range[d] = t->max_val[d] - t->min_val[d];
@@ -549,7 +556,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
             t->ncells = 1;
             for (int d = t->G - 1; d >= 0; d--) { t->stride[d] = t->ncells; t->ncells *= t->nslices[d]; }
             if (t->ncells >= (1ll << 31)) return pt_fail(PT_UNSUPPORTED, "table of %lld cells exceeds 2^31", t->ncells);
-            PT_TRY(build_partition(t.get(), part_scratch, s2));
+            PT_TRY(build_partition(t.get(), *part_scratch, s2));
             PT_CUDA(cudaStreamSynchronize(s2));
             return PT_OK;
         });
@@ -559,6 +566,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     if (p.kcoherence > 0) kc_st = build_kcoherence(t.get(), b_rgba.p, allowed_h);
     if (kc_st == PT_OK) kc_st = stage_done(PT_BUILD_KCOHERENCE);
     partitioner.join();
+    part_scratch.reset();
     shuffler.join();
     t_mark = now_s();
     if (kc_st != PT_OK) return kc_st;
@@ -566,7 +574,6 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
     t->build_ms[PT_BUILD_PARTITION] = part_ms;
     t->build_ms[PT_BUILD_SHUFFLE] = shuffle_ms;
     if (order_xy.empty()) return pt_fail(PT_BAD_ARG, "no allowed patches");
-    b_rgba.release();
     {
         DevBuf<int> d_order(t->st);
         PT_CUDA(d_order.reserve(order_xy.size()));
@@ -591,6 +598,7 @@ pt_status create_impl(const pt_params *pin, const float *b, int h, int w, int ch
             PT_TRY(pt_dt_other(t->table.p, t->G, t->nslices.data(), p.dt_algo, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
+    if (!t->desc_mode) PT_TRY(store_rows(t.get(), b_rgba));
     PT_TRY(stage_done(PT_BUILD_POPULATE_DT));
     t->build_ms[PT_BUILD_TOTAL] = 1000.0 * (now_s() - t_start);
     *out = t.release();
@@ -1263,7 +1271,7 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
     PT_CUDA(cudaStreamCreateWithFlags(&t->st, cudaStreamNonBlocking));
     t->own_stream = true;
     const long long P = (long long) t->eh * t->ew;
-    DevBuf<float4> b_rgba(t->st);     /* given back once the k-coherence set is built */
+    DevBuf<float4> b_rgba(t->st);
     {
         DevBuf<float> rgb(t->st);
         PT_CUDA(rgb.reserve(b0.size()));
@@ -1277,14 +1285,12 @@ pt_status load_impl(const pt_params *pin, const char *filename, pt_table **out) 
                     packed[((size_t) y * t->ew + x) * t->ds + d] = wh0[((size_t) (y + 7) * (w + 7) + (x + 7)) * nd + d];
         PT_CUDA(t->b_desc.reserve(packed.size()));
         PT_CUDA(cudaMemcpyAsync(t->b_desc.p, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, t->st));
-        PT_CUDA(t->b_row.reserve(pt_row_store_floats(w, h)));
-        PT_TRY(pt_launch_row_store(b_rgba.p, w, h, t->b_row.p, t->st));
         PT_CUDA(cudaStreamSynchronize(t->st));
     }
     /* the file has no k-coherence set (the reference's load leaves it empty); it is rebuilt from
        the stored descriptors */
     if (p.kcoherence > 0) PT_TRY(build_kcoherence(t.get(), b_rgba.p, std::vector<int>()));
-    b_rgba.release();
+    PT_TRY(store_rows(t.get(), b_rgba));
     t->nslices = nslices;
     t->stride.assign(G, 1);
     t->ncells = 1;

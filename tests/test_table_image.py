@@ -69,3 +69,23 @@ def test_a_load_waits_for_no_other_stream(gpu, libc, tmp_path):
     side.synchronize()
     for t in tables:
         t.close()
+
+
+def test_a_build_fits_without_room_for_the_row_store(gpu, libc):
+    """The most that a build of many cells holds is those, their breadth-first lists and the image's
+    16-byte copy, not the row store of 64 nor the partition's scratch."""
+    h, w = 400, 500
+    _, b = synth.pair(h, w, 15)
+    p = ptb.PatchTableParams("-limit 5")
+    srand_all(libc, 1)
+    t = ptb.PatchTable(p, b)
+    cells, patches = t.table().size, (h - 7) * (w - 7)
+    t.close()
+    # cells and lists, the populate order, descriptors and k-coherence sets, bins, the copy, small buffers
+    bound = 22 * cells + (4 + 32 + 8 * p.kcoherence) * patches + p.ndims * 16384 * 4 + 16 * h * w + (1 << 20)
+    old = ptb.set_device_alloc_limit(ptb.device_bytes_in_use() + bound)
+    try:
+        srand_all(libc, 1)
+        ptb.PatchTable(p, b).close()
+    finally:
+        ptb.set_device_alloc_limit(old)
