@@ -629,13 +629,14 @@ pt_status query_dims(const pt_table *t, int h, int w, int &vh, int &vw) {
     return PT_OK;
 }
 
-pt_status ensure_query_buffers(pt_table *t, int h, int w) {
+/* desc: the call stores its descriptors (the fused table step keeps none: 32 or 64 bytes per patch). */
+pt_status ensure_query_buffers(pt_table *t, int h, int w, bool desc = false) {
     long long P = (long long) (h - 7) * (w - 7);
     int ih, iw;
     size_t in_floats;
     query_input_dims(t, h, w, ih, iw, in_floats);
     PT_CUDA(t->q_rgb.reserve(std::max((size_t) h * w * 3, in_floats)));
-    PT_CUDA(t->q_desc.reserve((size_t) P * t->ds));
+    if (desc) PT_CUDA(t->q_desc.reserve((size_t) P * t->ds));
     PT_CUDA(t->q_tcand.reserve(P));
     for (int k = 0; k < 2; k++) { PT_CUDA(t->q_pos[k].reserve(P)); PT_CUDA(t->q_d[k].reserve(P)); }
     PT_CUDA(t->q_chpos.reserve(P));
@@ -685,7 +686,9 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
     long long P = (long long) (h - 7) * (w - 7);
     if (P >= (1ll << 31)) return pt_fail(PT_BAD_ARG, "query image too large");
     int n = (int) P;
-    PT_TRY(ensure_query_buffers(t, h, w));
+    /* The plain single-table query needs its descriptors only for the table step: one fused pass. */
+    const bool fused = !t->desc_mode && !t->pca && !learned && t->subs.empty();
+    PT_TRY(ensure_query_buffers(t, h, w, !fused));
     /* the distance kernels read the query image itself: one that shares memory with the NNF is copied */
     const size_t rgb_bytes = sizeof(float) * (size_t) h * w * 3;
     if (!t->desc_mode && pt_overlap(a_rgb, rgb_bytes, d_ann, sizeof(double) * 3 * (size_t) P)) {
@@ -708,8 +711,6 @@ pt_status lookup_device(pt_table *t, const float *a_rgb, int h, int w, double *d
         PT_TRY(pt_launch_descriptor(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), nullptr, t->q_desc.p,
                                     t->ds, st));
     }
-    /* The plain single-table query needs its descriptors only for the table step: one fused pass. */
-    const bool fused = !t->desc_mode && !t->pca && !learned && t->subs.empty();
     if (fused)
         PT_TRY(pt_launch_descriptor_cells(p.ndims, p.nchroma, a_rgb, h, w, pt_color_mode(p), t->bins,
                                           t->to_bin.p, t->table.p, t->q_tcand.p, 0, (h - 7 + 7) / 8, st));
@@ -1509,7 +1510,7 @@ pt_status pt_table_proposal_samples(pt_table *t, const float *d_a, int h, int w,
     if (h < 8 || w < 8) return pt_fail(PT_BAD_ARG, "image %dx%d is smaller than one 8x8 patch", w, h);
     cudaStream_t st = (cudaStream_t) stream;
     long long P = (long long) (h - 7) * (w - 7);
-    PT_TRY(ensure_query_buffers(t, h, w));
+    PT_TRY(ensure_query_buffers(t, h, w, true));
     PtTableView v;
     PT_TRY(pt_table_view(t, &v));
     PT_TRY(pt_prop_check_table(v));
@@ -1524,7 +1525,7 @@ pt_status pt_table_proposal_infer(pt_table *t, pt_proposal *net, const float *d_
     if (h < 8 || w < 8) return pt_fail(PT_BAD_ARG, "image %dx%d is smaller than one 8x8 patch", w, h);
     cudaStream_t st = (cudaStream_t) stream;
     long long P = (long long) (h - 7) * (w - 7);
-    PT_TRY(ensure_query_buffers(t, h, w));
+    PT_TRY(ensure_query_buffers(t, h, w, true));
     PtTableView v;
     PT_TRY(pt_table_view(t, &v));
     PT_TRY(pt_launch_descriptor(t->p.ndims, t->p.nchroma, d_a, h, w, pt_color_mode(t->p), nullptr, t->q_desc.p, t->ds,

@@ -89,3 +89,24 @@ def test_a_build_fits_without_room_for_the_row_store(gpu, libc):
         ptb.PatchTable(p, b).close()
     finally:
         ptb.set_device_alloc_limit(old)
+
+
+def test_bytes_of_a_lookup(gpu, libc):
+    """12 bytes per pixel and 40 per patch: a lookup with the fused table step stores no descriptors, one
+    with learned proposals (tests/test_proposal.py) or several tables does."""
+    import torch
+    h, w = 300, 400
+    a, b = synth.pair(h, w, 16)
+    patches = (h - 7) * (w - 7)
+    d = torch.from_numpy(a).cuda()
+    ann = torch.empty((h - 7, w - 7, 3), dtype=torch.float64, device="cuda")
+    for ntables, each in ((1, 40), (2, 40 + 32 + 4)):
+        p = ptb.PatchTableParams("-limit 0.05 -coherence_spatial 4")
+        p.ntables = ntables
+        srand_all(libc, 1)
+        t = ptb.PatchTable(p, b)
+        before = ptb.device_bytes_in_use()
+        t.lookup_device(d.data_ptr(), h, w, ann.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert ptb.device_bytes_in_use() - before <= 12 * h * w + each * patches + 4096
+        t.close()
